@@ -29,11 +29,10 @@
 //
 // Result accuracy ~FP32 (relative error ~sqrt(K) 2^-24), at (BF16 rate) / 6 real-product
 // throughput: 48 BF16 flops per complex multiply-add.
-#include <cuda.h>
 #include <cuda_bf16.h>
-#include <mutex>
 #include "kernels.cuh"
 #include "prof.cuh"
+#include "tcgen05.cuh"
 
 namespace qr {
 
@@ -49,57 +48,12 @@ constexpr int TC_THREADS = 320;              // warp 0 TMA, warp 1 MMA + TMEM, w
 constexpr int TC_EPI_WARPS = 8;              // two per TMEM lane quarter, 64 columns each
 constexpr int TC_TMEM_COLS = 4 * TC_BN;      // two buffers x (corrections, leading term), FP32
 constexpr int TC_SMEM = TC_STAGES * TC_STAGE + 1024 /* alignment */ + 256 /* barriers */;
-constexpr unsigned TC_SPIN = 1u << 24;       // polls before a wait gives up (seconds)
-
-// a flag nobody sets: waits that must run to completion (the CTA's own copies and MMAs in flight)
-__device__ const uint32_t kNever = 0;
 
 // slice pairs (A slice, B slice) of the six products, small terms first
 __constant__ int kPairA[6] = {2, 0, 1, 1, 0, 0};
 __constant__ int kPairB[6] = {0, 2, 1, 0, 1, 0};
 
-// ---- PTX helpers ------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// true once the phase with the given parity has completed; false after TC_SPIN polls, or as soon
-// as another role of the CTA has given up (abort flag, checked every 256 polls)
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const volatile uint32_t* abort_flag) {
-  const uint32_t a = smem_u32(bar);
-  for (unsigned i = 0; i < TC_SPIN; i++) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((i & 255u) == 255u && *abort_flag) return false;
-  }
-  return false;
-}
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-          smem_u32(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
+// ---- MMA descriptors -------------------------------------------------------------------------
 // Shared-memory matrix descriptor of a K-major tile with 128-byte rows and the 128-byte swizzle:
 // start address >> 4 (bits 0-13), leading byte offset (unused for this layout: 1), stride byte
 // offset = 1024 B between 8-row groups (bits 32-45), descriptor version 1 (bit 46), layout type
@@ -126,25 +80,6 @@ __device__ __forceinline__ void tc_mma(uint32_t dtmem, uint64_t adesc, uint64_t 
       "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%"
-      "19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
-}
-
 // ---- pass 1: BF16 slices of the real-ified operands --------------------------------------------
 // x is rounded once to FP32 (the only FP64-pipe operation: this part's FP64 rate is 1/64 of FP32)
 // and split exactly in FP32: h = bf16(x), m = bf16(x - h), l = bf16(x - h - m); h + m + l carries
@@ -414,26 +349,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 }
 
 // ---- host side ----------------------------------------------------------------------------------
-using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-int encode_fn(EncodeTiled* out) {
-  static std::mutex mu;
-  static EncodeTiled fn = nullptr;
-  std::lock_guard<std::mutex> lk(mu);
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q);
-    if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || !p)
-      return fail(QR_ECUDA, "cuTensorMapEncodeTiled is not available from the CUDA driver");
-    fn = reinterpret_cast<EncodeTiled>(p);
-  }
-  *out = fn;
-  return QR_OK;
-}
-
 // bf16 planes [planes][rows][Kp] with a 64 x 128 box and the 128-byte swizzle
 int make_map(CUtensorMap* map, const void* base, long Kp, long rows, long planes) {
   EncodeTiled enc = nullptr;

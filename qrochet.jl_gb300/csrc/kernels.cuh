@@ -10,6 +10,16 @@ enum { OP_N = 0, OP_T = 1, OP_C = 2, OP_R = 3 };
 int zgemm(cudaStream_t s, int opA, int opB, int M, int N, int K, double2 alpha,
           const double2* A, long lda, long sA, const double2* B, long ldb, long sB,
           double2 beta, double2* C, long ldc, long sC, int batch, const double* dk);
+// the same product in FP64 on the CUDA cores, spread over all SMs; allocates nothing
+int zgemm_spread(cudaStream_t s, int opA, int opB, int M, int N, int K, double2 alpha, const double2* A, long lda,
+                 long sA, const double2* B, long ldb, long sB, double2 beta, double2* C, long ldc, long sC, int batch,
+                 const double* dk);
+
+// ---- gemm_oz.cu: C[b] = op(A[b]) diag(dk) op(B[b]) at FP64 accuracy on the tcgen05 tensor cores
+// (exact products of 8-bit slices); sB = 0 shares B.  Slices in a stream-ordered allocation.
+bool zgemm_oz_fits(int M, int N, int K);
+int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
+             const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk);
 
 // ---- gemm_tc.cu: C = op(A) op(B) on the tcgen05 tensor cores: operands rounded to FP32 and split
 // into three BF16 slices, six slice products, FP32 accumulation in TMEM, TMA-staged tiles.

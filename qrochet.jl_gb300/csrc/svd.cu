@@ -2794,7 +2794,7 @@ extern "C" int qr_svd_noalloc(int m, int n, const double* A, long lda, double* U
       gather_cols_k<double2><<<gs((long)k * k), TPB, 0, s>>>(V, k, k, k, perm, nullptr, Vhd, ldvh);
       QR_CHECK_LAUNCH("gather_cols_k");
       if (reorth) QR_TRY(reorthonormalize_noalloc(Bk, k, k, B));
-      QR_TRY(zgemm(s, OP_N, OP_N, rows, k, k, one, L, rows, 0, Vhd, ldvh, 0, zero, Ud, ldu, 0, 1, nullptr));
+      QR_TRY(zgemm_spread(s, OP_N, OP_N, rows, k, k, one, L, rows, 0, Vhd, ldvh, 0, zero, Ud, ldu, 0, 1, nullptr));
       QR_TRY(ztranspose(s, Bk, k, k, k, Vhd, ldvh, 1));
     } else {  // A = B0^H = Lw Sigma (Q Rf)^H: U = Lw (m x m), Vh = Rf^H Q^H (m x n)
       gather_cols_k<double2><<<gs((long)k * k), TPB, 0, s>>>(B, k, k, k, perm, sorted, Ud, ldu);
@@ -2802,7 +2802,7 @@ extern "C" int qr_svd_noalloc(int m, int n, const double* A, long lda, double* U
       gather_cols_k<double2><<<gs((long)k * k), TPB, 0, s>>>(V, k, k, k, perm, nullptr, Bk, k);
       QR_CHECK_LAUNCH("gather_cols_k");
       if (reorth) QR_TRY(reorthonormalize_noalloc(Ud, ldu, k, B));
-      QR_TRY(zgemm(s, OP_C, OP_C, k, rows, k, one, Bk, k, 0, L, rows, 0, zero, Vhd, ldvh, 0, 1, nullptr));
+      QR_TRY(zgemm_spread(s, OP_C, OP_C, k, rows, k, one, Bk, k, 0, L, rows, 0, zero, Vhd, ldvh, 0, 1, nullptr));
     }
   } else {
     // left factor Lf (rows x k) = B[:, perm] / sigma ; right factor (k x k) = V[:, perm]
