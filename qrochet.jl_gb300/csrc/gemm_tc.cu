@@ -50,8 +50,8 @@ constexpr int TC_TMEM_COLS = 4 * TC_BN;      // two buffers x (corrections, lead
 constexpr int TC_SMEM = TC_STAGES * TC_STAGE + 1024 /* alignment */ + 256 /* barriers */;
 
 // slice pairs (A slice, B slice) of the six products, small terms first
-__constant__ int kPairA[6] = {2, 0, 1, 1, 0, 0};
-__constant__ int kPairB[6] = {0, 2, 1, 0, 1, 0};
+__device__ constexpr int kPairA[6] = {2, 0, 1, 1, 0, 0};
+__device__ constexpr int kPairB[6] = {0, 2, 1, 0, 1, 0};
 
 // ---- MMA descriptors -------------------------------------------------------------------------
 // Shared-memory matrix descriptor of a K-major tile with 128-byte rows and the 128-byte swizzle:
@@ -72,14 +72,17 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TC_BN >> 3) << 17) |
                             ((uint32_t)(TC_BM >> 4) << 24);
 
-__device__ __forceinline__ void tc_mma(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+// The descriptors of a stage's tiles differ in their low words only, by compile-time offsets.
+__device__ __forceinline__ void tc_mma(uint32_t dtmem, uint32_t alo, uint32_t blo, uint32_t hi, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dtmem),
-      "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate)
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+      "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}" ::"r"(dtmem),
+      "r"(alo), "r"(blo), "r"(hi), "r"(kIdesc), "r"(accumulate)
       : "memory");
 }
+
 // ---- pass 1: BF16 slices of the real-ified operands --------------------------------------------
 // x is rounded once to FP32 (the only FP64-pipe operation: this part's FP64 rate is 1/64 of FP32)
 // and split exactly in FP32: h = bf16(x), m = bf16(x - h), l = bf16(x - h - m); h + m + l carries
@@ -222,7 +225,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- producer: TMA loads of the three slices of A and of B per k-block
       int issued[TC_STAGES] = {0, 0};
       unsigned g = 0;
@@ -253,7 +256,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         if (issued[s] > 0 && !mbar_wait(full + s, (uint32_t)(issued[s] - 1) & 1u, &kNever)) *abort_flag = 1;
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- MMA issuer
       bool ok = true;
       unsigned g = 0;
@@ -268,16 +271,18 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           const uint32_t ph = (g / TC_STAGES) & 1u;
           if (*abort_flag || !mbar_wait(full + s, ph, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t st = smem_u32(smem + s * TC_STAGE);
+          const uint64_t desc = smem_desc(smem_u32(smem + s * TC_STAGE));
+          const uint32_t st = (uint32_t)desc, dhi = (uint32_t)(desc >> 32);
 #pragma unroll
           for (int p = 0; p < 6; p++) {
-            const uint32_t a0 = st + kPairA[p] * TC_TILE, b0 = st + (3 + kPairB[p]) * TC_TILE;
+            const uint32_t a0 = st + (uint32_t)((kPairA[p] * TC_TILE) >> 4);
+            const uint32_t b0 = st + (uint32_t)(((3 + kPairB[p]) * TC_TILE) >> 4);
             const bool lead = p == 5;  // h h
             const uint32_t d = lead ? dt + TC_BN : dt;
 #pragma unroll
             for (int j = 0; j < TC_BK / 16; j++) {
               const uint32_t acc = ((!lead && p > 0) || j > 0) ? 1u : 0u;
-              tc_mma(d, smem_desc(a0 + 32 * j), smem_desc(b0 + 32 * j), acc);
+              tc_mma(d, a0 + 2 * j, b0 + 2 * j, dhi, acc);
             }
           }
           tc_commit(empty + s);   // the stage is free once these MMAs have read it
