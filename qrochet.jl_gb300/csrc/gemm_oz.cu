@@ -310,7 +310,8 @@ struct OzPlain {
 
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     zgemm_oz_k(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, double2* __restrict__ C,
-               long ldc, long sC, int M, int N, int nk, int bshared, int ntm, int ntn, int cs, const OzPlain plain) {
+               long ldc, long sC, int M, int N, int nk, int bshared, int ntm, int ntn, int cs, int herm,
+               int sub, const OzPlain plain) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OZ_STAGES * OZ_STAGE);
@@ -323,7 +324,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(afull + 6);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = blockIdx.x % cs;
-  const int t = blockIdx.x / cs, tn = t % ntn, tm = (t / ntn) % ntm, z = t / (ntn * ntm);
+  int t = blockIdx.x / cs, tn = t % ntn, tm = (t / ntn) % ntm, z = t / (ntn * ntm);
+  if (herm) {  // the tiles on and above the diagonal, by columns of tiles: t = tn (tn + 1) / 2 + tm
+    tn = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
+    while (tn * (tn + 1) / 2 > t) tn--;
+    while ((tn + 1) * (tn + 2) / 2 <= t) tn++;
+    tm = t - tn * (tn + 1) / 2;
+    z = 0;
+  }
   const int kb0 = (int)((long)nk * rank / cs), kb1 = (int)((long)nk * (rank + 1) / cs);
 
   if (threadIdx.x == 0) {
@@ -492,7 +500,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   for (int e = threadIdx.x; e < 64 * nc; e += OZ_THREADS) {
     const int i = e & 63, c = rank * nc + (e >> 6);
     const int gi = tm * 64 + i, gj = tn * OZ_BN + c;
-    if (gi >= M || gj >= N) continue;
+    if (gi >= M || gj >= N || (herm && gi > gj)) continue;
     double2 out;
     const int xa = ea[gi], xb = eb[gj];
     if (bad) {
@@ -527,7 +535,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       out.x = oz_double(re.x, re.y, sc);
       out.y = oz_double(im.x, im.y, sc);
     }
+    if (sub) out = csub(C[z * sC + gi + (long)gj * ldc], out);
     C[z * sC + gi + (long)gj * ldc] = out;
+    if (herm && gi != gj) C[gj + (long)gi * ldc] = cconj(out);
   }
   if (cs > 1) oz_cluster_sync();  // the sums stay readable until every CTA of the cluster has them
 }
@@ -581,8 +591,9 @@ size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 // Largest K of the integer sums (hi stays below 2^51) and the largest plane rows TMA addresses.
 bool zgemm_oz_fits(int M, int N, int K) { return K <= (1 << 20) && M <= (1 << 28) && N <= (1 << 28); }
 
-int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
-             const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk) {
+static int oz_run(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
+                  const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk,
+                  int herm, int eq_a, int sub) {
   const bool bshared = sB == 0 || batch == 1;
   const int bb = bshared ? 1 : batch;
   const int ntm = (M + 63) / 64, ntn = (N + OZ_BN - 1) / OZ_BN, Kh = (K + 15) / 16 * 16;
@@ -597,13 +608,13 @@ int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double
   OzPlain pl;
   pl.K = K;
   const bool an = opA == OP_N || opA == OP_R, bn = opB == OP_N || opB == OP_R;
-  pl.a = {A, an ? 1 : lda, an ? lda : 1, sA, M, opA == OP_C || opA == OP_R, 1, dk, (__nv_bfloat16*)ws,
+  pl.a = {A, an ? 1 : lda, an ? lda : 1, sA, M, opA == OP_C || opA == OP_R, eq_a ? -1 : 1, dk, (__nv_bfloat16*)ws,
           (int*)(ws + ab + bbt), apl};
-  pl.b = {B, bn ? ldb : 1, bn ? 1 : ldb, bshared ? 0 : sB, N, opB == OP_C || opB == OP_R, -1, nullptr,
+  pl.b = {B, bn ? ldb : 1, bn ? 1 : ldb, bshared ? 0 : sB, N, opB == OP_C || opB == OP_R, eq_a ? 1 : -1, nullptr,
           (__nv_bfloat16*)(ws + ab), (int*)(ws + ab + bbt + ea), bpl};
   int* g = (int*)(ws + ab + bbt + ea + eb);
   auto run = [&]() -> int {
-    oz_kmax_k<<<dim3(ceil_div(K, KMAX_K), 1, bb), 256, 0, s>>>(pl.b, K, g);
+    oz_kmax_k<<<dim3(ceil_div(K, KMAX_K), 1, bb), 256, 0, s>>>(eq_a ? pl.a : pl.b, K, g);
     QR_CHECK_LAUNCH("oz_kmax_k");
     // few rows: 4 per CTA so that the pass still covers the SMs; else 16
     const long rows = (long)M * batch + (long)N * bb;
@@ -619,7 +630,7 @@ int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double
     QR_TRY(oz_map_make(&mb, ws + ab, Kp, brows, (long)OZ_S * bb, OZ_BN));
     QR_TRY(set_func_attr_once((const void*)zgemm_oz_k, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
     const int nk = (int)(Kp / OZ_BK);
-    const long tiles = (long)ntm * ntn * batch;
+    const long tiles = herm ? (long)ntm * (ntm + 1) / 2 : (long)ntm * ntn * batch;
     // K split over a cluster: the split with the fewest (waves x stages per CTA), a CTA's fixed cost
     // counted as 5 stages and a split's as 2 more
     int cs = 1;
@@ -646,12 +657,58 @@ int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    QR_CUDA(cudaLaunchKernelEx(&cfg, zgemm_oz_k, ma, mb, C, ldc, sC, M, N, nk, bshared ? 1 : 0, ntm, ntn, cs, pl));
+    QR_CUDA(cudaLaunchKernelEx(&cfg, zgemm_oz_k, ma, mb, C, ldc, sC, M, N, nk, bshared ? 1 : 0, ntm, ntn, cs, herm, sub, pl));
     count_launch();
     return QR_OK;
   };
   const int rc = run();
   cudaFreeAsync(ws, s);
+  return rc;
+}
+
+int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
+             const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk) {
+  return oz_run(s, opA, opB, M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, dk, 0, 0, 0);
+}
+
+// C = A B (M x K, K x N) for an A whose columns spread over decades: the scaling along K equilibrates A's
+// columns instead of B's rows, so columns of C that combine small columns of A keep their relative accuracy
+int zgemm_graded(cudaStream_t s, int M, int N, int K, const double2* A, long lda, const double2* B, long ldb, double2* C,
+                 long ldc) {
+  const double work = (double)M * N * K;
+  if (work < OZ_MIN_WORK || !zgemm_oz_fits(M, N, K))
+    return zgemm(s, OP_N, OP_N, M, N, K, make_double2(1.0, 0.0), A, lda, 0, B, ldb, 0, make_double2(0.0, 0.0), C, ldc, 0,
+                 1, nullptr);
+  const int pr = prof_begin(s, PK_ZGEMM, 8.0 * work, 16.0 * ((double)M * K + (double)K * N + (double)M * N));
+  const int rc = oz_run(s, OP_N, OP_N, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, nullptr, 0, 1, 0);
+  prof_end(s, pr);
+  return rc;
+}
+
+// C -= A B (M x K, K x N)
+int zgemm_sub(cudaStream_t s, int M, int N, int K, const double2* A, long lda, const double2* B, long ldb, double2* C,
+              long ldc) {
+  if (M <= 0 || N <= 0 || K <= 0) return QR_OK;
+  const double work = (double)M * N * K;
+  const int pr = prof_begin(s, PK_ZGEMM, 8.0 * work, 16.0 * ((double)M * K + (double)K * N + 2.0 * M * N));
+  const int rc = work >= OZ_MIN_WORK && zgemm_oz_fits(M, N, K)
+                     ? oz_run(s, OP_N, OP_N, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, nullptr, 0, 0, 1)
+                     : zgemm_spread(s, OP_N, OP_N, M, N, K, make_double2(-1.0, 0.0), A, lda, 0, B, ldb, 0,
+                                    make_double2(1.0, 0.0), C, ldc, 0, 1, nullptr);
+  prof_end(s, pr);
+  return rc;
+}
+
+// C = A^H A (n x n, K rows): the entries on and above the diagonal, mirrored as they are stored (exactly
+// Hermitian, which the rotations formed from a Gram matrix rely on)
+int zherk(cudaStream_t s, int n, int K, const double2* A, long lda, double2* C, long ldc) {
+  if (n <= 0) return QR_OK;
+  const double work = (double)n * n * K;
+  const int pr = prof_begin(s, PK_ZGEMM, 4.0 * work, 16.0 * ((double)n * K + (double)n * n));
+  const int rc = work >= OZ_MIN_WORK && zgemm_oz_fits(n, n, K)
+                     ? oz_run(s, OP_C, OP_N, n, n, K, A, lda, 0, A, lda, 0, C, ldc, 0, 1, nullptr, 1, 0, 0)
+                     : zherk_spread(s, n, K, A, lda, C, ldc);
+  prof_end(s, pr);
   return rc;
 }
 

@@ -10,6 +10,11 @@ enum { OP_N = 0, OP_T = 1, OP_C = 2, OP_R = 3 };
 int zgemm(cudaStream_t s, int opA, int opB, int M, int N, int K, double2 alpha,
           const double2* A, long lda, long sA, const double2* B, long ldb, long sB,
           double2 beta, double2* C, long ldc, long sC, int batch, const double* dk);
+// From this many complex multiply-adds on, the three launches of the sliced product cost less than the
+// spread kernel's FP64 time (4 DFMA each at 2 per SM and cycle): 96 x 128 x 96 takes 25 us sliced and 19
+// spread, 128 x 128 x 128 25 and 31, 256 x 512 x 256 34 and 372.  (The 64 x 64-tile DMMA kernel that ran all
+// sizes before took 592 us at 128^3, 1176 at 256 x 512 x 256 and 64.9 ms at 2048^3; sliced: 2.07 ms.)
+constexpr double OZ_MIN_WORK = 1.5 * (1 << 20);
 // the same product in FP64 on the CUDA cores, spread over all SMs; allocates nothing
 int zgemm_spread(cudaStream_t s, int opA, int opB, int M, int N, int K, double2 alpha, const double2* A, long lda,
                  long sA, const double2* B, long ldb, long sB, double2 beta, double2* C, long ldc, long sC, int batch,
@@ -20,6 +25,16 @@ int zgemm_spread(cudaStream_t s, int opA, int opB, int M, int N, int K, double2 
 bool zgemm_oz_fits(int M, int N, int K);
 int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
              const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk);
+
+int zherk_spread(cudaStream_t s, int n, int K, const double2* A, long lda, double2* C, long ldc);
+// C = A B for an A whose columns spread over decades (see gemm_oz.cu)
+int zgemm_graded(cudaStream_t s, int M, int N, int K, const double2* A, long lda, const double2* B, long ldb, double2* C,
+                 long ldc);
+// C -= A B
+int zgemm_sub(cudaStream_t s, int M, int N, int K, const double2* A, long lda, const double2* B, long ldb, double2* C,
+              long ldc);
+// C = A^H A at FP64 accuracy, n x n from K rows (sliced or spread as zgemm)
+int zherk(cudaStream_t s, int n, int K, const double2* A, long lda, double2* C, long ldc);
 
 // ---- gemm_tc.cu: C = op(A) op(B) on the tcgen05 tensor cores: operands rounded to FP32 and split
 // into three BF16 slices, six slice products, FP32 accumulation in TMEM, TMA-staged tiles.
