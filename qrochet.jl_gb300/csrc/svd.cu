@@ -71,7 +71,7 @@ struct HBuf {
 };
 
 struct SvdWork {
-  DBuf B, V, B32, V32, X, Rm, E, T1, nrm, perm, cnt, tau, qtmp, host_sig, Bl, Qp, ml, pt, tcw;
+  DBuf B, V, B32, V32, X, Rm, E, T1, nrm, perm, cnt, tau, qtmp, host_sig, Bl, Qp, ml, pt, tcw, rfG, rfc;
   HBuf hl;
   cudaStream_t last = nullptr;
 };
@@ -82,7 +82,7 @@ SvdWork* svd_work_create() { return new SvdWork(); }
 void svd_work_free(SvdWork* w) {
   if (!w) return;
   DBuf* all[] = {&w->B, &w->V, &w->B32, &w->V32, &w->X, &w->Rm, &w->E, &w->T1,
-                 &w->nrm, &w->perm, &w->cnt, &w->tau, &w->qtmp, &w->host_sig, &w->Bl, &w->Qp, &w->ml, &w->pt, &w->tcw};
+                 &w->nrm, &w->perm, &w->cnt, &w->tau, &w->qtmp, &w->host_sig, &w->Bl, &w->Qp, &w->ml, &w->pt, &w->tcw, &w->rfG, &w->rfc};
   for (DBuf* b : all)
     if (b->p) cudaFree(b->p);
   if (w->hl.p) cudaFreeHost(w->hl.p);
@@ -1471,7 +1471,8 @@ __device__ __forceinline__ void db_block_pair(float2* __restrict__ Bh, float2* _
 __global__ void __launch_bounds__(DB_NT, 1)
     jacobi_block_df_k(float2* __restrict__ Bh, float2* __restrict__ Bl, long ldb, int m, int n, float2* __restrict__ Vh,
                       float2* __restrict__ Vl, long ldv, int nbp, double tol, const double* __restrict__ smax_p,
-                      unsigned* __restrict__ state, int sweep, unsigned* __restrict__ flags, int k0) {
+                      unsigned* __restrict__ state, int sweep, unsigned* __restrict__ flags, int k0,
+                      const unsigned* __restrict__ ml, unsigned* __restrict__ done) {
   __shared__ DbShared sh;
   extern __shared__ __align__(16) float2 db_sv[];
   if (((volatile unsigned*)state)[0]) return;
@@ -1479,6 +1480,22 @@ __global__ void __launch_bounds__(DB_NT, 1)
   unsigned* cnt = state + 8 + SW_STRIDE * sweep;
   const int nb = (n + 1) / 2;
   const int npairs = nbp / 2;
+  if (ml) {
+    // the listed block pairs (MaskedList over the nbp blocks), as in jacobi_block_reg_k
+    const MaskedList L = masked_list(ml, nbp);
+    const unsigned total = L.count[2];
+    for (unsigned i = blockIdx.x; i < total; i += gridDim.x) {
+      int bp, bq;
+      bool full;
+      list_item(L, i, bp, bq, full);
+      const unsigned op = L.ord[2 * (long)i], oq = L.ord[2 * (long)i + 1];
+      if (!wait_cols2(done, bp, bq, op, oq, state)) return;
+      db_block_pair(Bh, Bl, ldb, m, n, Vh, Vl, ldv, nb, bp, bq, full ? 0 : 1, (float)tol, smax, k0, cnt, sh, db_sv);
+      post_cols2(done, bp, bq, op + 1, oq + 1);
+    }
+    finish_sweep(state, cnt, sweep, 1e-7f);
+    return;
+  }
   const unsigned base = (unsigned)sweep * (unsigned)(nbp - 1);
   const bool dataflow = npairs > (int)gridDim.x;
   const long nit = dataflow ? ((long)(nbp - 1) * npairs - blockIdx.x + gridDim.x - 1) / gridDim.x : (long)(nbp - 1);
@@ -1549,19 +1566,6 @@ __global__ void __launch_bounds__(NT, 2) jacobi_sweep_df_k(float2* __restrict__ 
   // constant 0.05-0.3): the next sweep would only confirm convergence
   finish_sweep(state, cnt, sweep, 1e-7f);
 }
-
-// Xh[:, j] = src[:, perm[j]], Xl = 0 (an FP32 matrix as a double-float one, columns permuted)
-__global__ void gather_cols_f2_k(const float2* __restrict__ src, long lds, int rows, int cols,
-                                 const int* __restrict__ perm, float2* __restrict__ hi, float2* __restrict__ lo,
-                                 long ldd) {
-  const long total = (long)rows * cols;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
-    const long i = t % rows, j = t / rows;
-    hi[i + j * ldd] = src[i + (long)perm[j] * lds];
-    lo[i + j * ldd] = make_float2(0.f, 0.f);
-  }
-}
-
 
 // out[0] = max_j nrm[j] (one block)
 __global__ void max_reduce_k(const double* __restrict__ nrm, int k, double* __restrict__ out) {
@@ -2177,7 +2181,8 @@ int jacobi_df(cudaStream_t s, SvdWork* w, float2* Bh, float2* Bl, long ldb, int 
     void* args[] = {&a1, &a2, &l1, &mm, &kk, &a3, &a4, &l2, &npp, &tl, &sm, &st, &sw, &fl, &kz, &mk, &dn};
     if (blockdf && !mk) {
       int nbb = nbp;
-      void* bargs[] = {&a1, &a2, &l1, &mm, &kk, &a3, &a4, &l2, &nbb, &tl, &sm, &st, &sw, &fl, &kz};
+      unsigned* none = nullptr;
+      void* bargs[] = {&a1, &a2, &l1, &mm, &kk, &a3, &a4, &l2, &nbb, &tl, &sm, &st, &sw, &fl, &kz, &none, &none};
       QR_CUDA(cudaLaunchCooperativeKernel((const void*)jacobi_block_df_k, dim3(dbgrid), dim3(DB_NT), bargs, dbsm, s));
     } else {
       QR_CUDA(cudaLaunchCooperativeKernel((const void*)jacobi_sweep_df_k<NT, RPT>, dim3(grid), dim3(NT), args, vsm, s));
@@ -2340,6 +2345,8 @@ static int jacobi_f32_masked(cudaStream_t s, SvdWork* w, float2* B, int rows, in
   return rc;
 }
 
+#include "svd_refine.cuh"
+
 // Re-orthonormalise the m x k column block L in place (Householder QR, phase-preserving).
 static int reorthonormalize(cudaStream_t s, SvdWork* w, double2* L, long ldl, int m, int k) {
   svd_path(SP_REORTH);
@@ -2353,6 +2360,23 @@ static int reorthonormalize(cudaStream_t s, SvdWork* w, double2* L, long ldl, in
   QR_TRY(zqr_thin(s, Acopy, m, k, m, L, ldl, Rr, k, w->tau.as<double2>()));
   phase_fix_k<<<gs((long)m * k), TPB, 0, s>>>(L, ldl, m, k, Rr, k);
   QR_CHECK_LAUNCH("phase_fix_k");
+  return QR_OK;
+}
+
+// One Newton-Schulz step on nearly orthonormal columns, L <- L (3 I - L^H L) / 2 (m x k, ld ldl; columns of
+// singular values far below sigma_max are noise and must stay out of it).  The
+// columns B / sigma are orthogonal to ~eps sigma_max / sigma_j; the step brings that to rounding and moves
+// the represented matrix by eps sigma_max, for two products instead of a Householder QR.
+static int polish_columns(cudaStream_t s, SvdWork* w, double2* L, long ldl, int m, int k) {
+  QR_TRY(w->rfG.ensure(sizeof(double2) * (2 * (size_t)k * k + (size_t)m * k), s));
+  double2 *S = w->rfG.as<double2>(), *T = S + (size_t)k * k, *Y = T + (size_t)k * k;
+  QR_TRY(zherk(s, k, m, L, ldl, S, k));
+  QR_CUDA(cudaMemsetAsync(T, 0, sizeof(double2) * (size_t)k * k, s));
+  refine_m_k<<<gs((long)k * k), TPB, 0, s>>>(T, nullptr, S, k);  // (I - S) / 2
+  QR_CHECK_LAUNCH("refine_m_k");
+  QR_TRY(zgemm(s, OP_N, OP_N, m, k, k, make_double2(1.0, 0.0), L, ldl, 0, T, k, 0, make_double2(0.0, 0.0), Y, m, 0, 1, nullptr));
+  add_cols_k<<<gs((long)m * k), TPB, 0, s>>>(L, ldl, Y, m, k);
+  QR_CHECK_LAUNCH("add_cols_k");
   return QR_OK;
 }
 
@@ -2377,8 +2401,19 @@ constexpr int kMixedMinCols = 16;
 // there (the polish then takes 2-3 sweeps).
 constexpr int kPrecondMinCols = 32;
 constexpr int kMixedProbeSweeps = 11;
+// FP64: above this many columns one FP64 sweep closes the refinement, every pair tested in the sweep's
+// own arithmetic (the rounding of X and B = A X grows with the size, the tolerance only as its root).
+constexpr int kFp64CloseCols = 512;
 constexpr double kSmallCol = 1e-4;
 constexpr double kSmallColFrac = 0.1;
+// Above 128 columns the decision falls after kMixedFirstSweeps sweeps when the spectrum visibly decays:
+// more than kDecayFrac of those columns below kDecayCol sigma_max (a square Gaussian block has 1%).
+// A last probe sweep that still rotates more than kSlowFrac of the pairs (1% at 2048 Gaussian columns,
+// 44% over 4 decades) restarts as well.
+constexpr int kMixedFirstSweeps = 5;
+constexpr double kDecayCol = 1e-2;
+constexpr double kDecayFrac = 0.25;
+constexpr double kSlowFrac = 0.05;
 
 // B (rows x k, rows >= k) = Q R with Q in w->Qp (rows x k); B is replaced by W = R^H (k x k, ld k)
 static int qr_precondition(cudaStream_t s, SvdWork* w, double2* B, int rows, int k) {
@@ -2390,6 +2425,66 @@ static int qr_precondition(cudaStream_t s, SvdWork* w, double2* B, int rows, int
   return ztranspose(s, Rr, k, k, k, B, k, 1);
 }
 
+// B32 = fl32(2^-e B), 2^e the power of two above the largest column norm; B keeps its values
+static int scaled_f32(cudaStream_t s, SvdWork* w, double2* B, int rows, int k, float2* B32) {
+  double* nrm = w->nrm.as<double>();
+  double* smax_d = nrm + k;
+  col_norms_k<double2><<<ceil_div((long)k * 32, TPB), TPB, 0, s>>>(B, rows, rows, k, nrm);
+  QR_CHECK_LAUNCH("col_norms_k");
+  max_reduce_k<<<1, 256, 0, s>>>(nrm, k, smax_d);
+  QR_CHECK_LAUNCH("max_reduce_k");
+  pow2_scale_k<double2><<<gs((long)rows * k), TPB, 0, s>>>(B, rows, rows, k, smax_d, smax_d + 1, 0);
+  QR_CHECK_LAUNCH("pow2_scale_k");
+  QR_TRY(z2c(s, B, rows, B32, rows, rows, k));
+  pow2_scale_k<double2><<<gs((long)rows * k), TPB, 0, s>>>(B, rows, rows, k, smax_d, smax_d + 1, 1);
+  QR_CHECK_LAUNCH("pow2_scale_k");
+  return QR_OK;
+}
+
+// From the FP32 stage's rotations V32 (B32 = its rotated columns) to V and B <- B V at the accuracy of
+// `tol`: by refine(), and where that does not converge by sweeps, in double-float (df) or in FP64.
+// Columns at or beyond k0 need no rotation among themselves.
+static int finish_fp32(cudaStream_t s, SvdWork* w, double2* B, int rows, int k, const float2* B32, const float2* V32,
+                       double2* V, double tol, int k0, bool df) {
+  const size_t kk2 = (size_t)k * k, rk = (size_t)rows * k;
+  double* nrm = w->nrm.as<double>();
+  double* smax_d = nrm + k;  // two scratch doubles; the caller rewrites them
+  int* perm = w->perm.as<int>();
+  col_norms_k<float2><<<ceil_div((long)k * 32, TPB), TPB, 0, s>>>(B32, rows, rows, k, nrm);
+  QR_CHECK_LAUNCH("col_norms_k");
+  rank_sort_k<<<ceil_div(k, TPB), TPB, 0, s>>>(nrm, k, perm, nullptr);
+  QR_CHECK_LAUNCH("rank_sort_k");
+  gather_cols_k<float2><<<gs((long)k * k), TPB, 0, s>>>(V32, k, k, k, perm, nullptr, V, k);
+  QR_CHECK_LAUNCH("gather_cols_k");
+  // A scaled by a power of two so sigma_max ~ 1
+  QR_TRY(w->T1.ensure(sizeof(double2) * rk, s));
+  double2* AX = w->T1.as<double2>();
+  col_norms_k<double2><<<ceil_div((long)k * 32, TPB), TPB, 0, s>>>(B, rows, rows, k, nrm);
+  QR_CHECK_LAUNCH("col_norms_k");
+  max_reduce_k<<<1, 256, 0, s>>>(nrm, k, smax_d);
+  QR_CHECK_LAUNCH("max_reduce_k");
+  pow2_scale_k<double2><<<gs((long)rows * k), TPB, 0, s>>>(B, rows, rows, k, smax_d, smax_d + 1, 0);
+  QR_CHECK_LAUNCH("pow2_scale_k");
+  int done = 0;
+  QR_TRY(refine(s, w, B, rows, k, V, AX, tol, smax_d, k0, &done));
+  if (!done && df) {
+    QR_TRY(w->X.ensure(sizeof(float2) * 2 * kk2, s));
+    QR_TRY(w->Bl.ensure(sizeof(float2) * 2 * rk, s));
+    float2 *Xh = w->X.as<float2>(), *Xl = Xh + kk2, *Bh = w->Bl.as<float2>(), *Bl = Bh + rk;
+    QR_TRY(z2df(s, AX, rows, rows, k, nullptr, Bh, Bl, rows));
+    QR_TRY(z2df(s, V, k, k, k, nullptr, Xh, Xl, k));
+    // (the sweeps' own inner products carry ~sqrt(rows) 2^-48 noise)
+    QR_TRY(jacobi_df(s, w, Bh, Bl, rows, rows, k, Xh, Xl, k, 40, 32.0 * sqrt((double)rows) * Eps<double>::v, smax_d, k0));
+    QR_TRY(df2z(s, Bh, Bl, rows, rows, k, smax_d + 1, B, rows));
+    return df2z(s, Xh, Xl, k, k, k, nullptr, V, k);
+  }
+  QR_CUDA(cudaMemcpyAsync(B, AX, sizeof(double2) * rk, cudaMemcpyDeviceToDevice, s));
+  pow2_scale_k<double2><<<gs((long)rows * k), TPB, 0, s>>>(B, rows, rows, k, smax_d, smax_d + 1, 1);
+  QR_CHECK_LAUNCH("pow2_scale_k");
+  if (!done || (!df && k > kFp64CloseCols)) return jacobi<double>(s, w, B, rows, rows, k, V, k, 60, tol);
+  return QR_OK;
+}
+
 int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int n, long lda,
               double2* U, long ldu, double* S, double2* Vh, long ldvh, int keep) {
   if (m <= 0 || n <= 0) return QR_OK;
@@ -2398,6 +2493,7 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
   const int k = tall ? n : m;
   int rows = rows0;  // rows of the matrix the Jacobi runs on: rows0, or k after QR preconditioning
   bool pre = false;
+  bool refined = false;  // B and V come from the refinement, not from FP64 sweeps
   QR_TRY(w->B.ensure(sizeof(double2) * (size_t)rows0 * k, s));
   QR_TRY(w->V.ensure(sizeof(double2) * (size_t)k * k, s));
   QR_TRY(w->nrm.ensure(sizeof(double) * (size_t)k * 2, s));
@@ -2426,9 +2522,22 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
       rows = k;
       pre = true;
     }
-    QR_TRY(zset_identity(s, V, k, k, k));
     double tol = sqrt((double)rows) * Eps<double>::v;
-    QR_TRY(jacobi<double>(s, w, B, rows, rows, k, V, k, 60, tol));
+    if (pre) {
+      // R^H's columns keep full relative precision in FP32, so the FP32 stage (relative test) finds
+      // all right singular vectors to ~1e-5 and a few products finish them
+      QR_TRY(w->B32.ensure(sizeof(float2) * (size_t)rows * k, s));
+      QR_TRY(w->V32.ensure(sizeof(float2) * (size_t)k * k, s));
+      float2 *B32 = w->B32.as<float2>(), *V32 = w->V32.as<float2>();
+      float tol32 = fmaxf(4e-6f, 2.0f * sqrtf((float)rows) * Eps<float>::v);
+      QR_TRY(scaled_f32(s, w, B, rows, k, B32));
+      QR_TRY(cset_identity(s, V32, k, k, k));
+      QR_TRY(jacobi<float>(s, w, B32, rows, rows, k, V32, k, 20, -tol32, false, kPrecondTanStop));
+      QR_TRY(finish_fp32(s, w, B, rows, k, B32, V32, V, tol, k, false));
+    } else {
+      QR_TRY(zset_identity(s, V, k, k, k));
+      QR_TRY(jacobi<double>(s, w, B, rows, rows, k, V, k, 60, tol));
+    }
   } else {
     // ---- FP32 Jacobi preconditioner
     QR_TRY(w->B32.ensure(sizeof(float2) * (size_t)rows * k, s));
@@ -2440,14 +2549,10 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
     // a preconditioner: 1e-5 relative orthogonality is plenty for the FP64 refinement, and sits
     // above the FP32 rounding floor (~sqrt(m) eps32) so sweeps stop once rotations are noise
     float tol32 = fmaxf(4e-6f, 2.0f * sqrtf((float)rows) * Eps<float>::v);
-    int conv32 = 0;
-    double frac32 = 0.0;
-    QR_TRY(jacobi<float>(s, w, B32, rows, rows, k, V32, k, kMixedProbeSweeps, tol32, false, kPrecondTanStop,
-                         &conv32, &frac32));
     // columns the polish rotates: all, or the leading keep + margin (see below)
     const int k0 = keep > 0 && keep < k ? std::min(k, keep + std::max(32, keep / 8)) : k;
-    bool slow = false;
-    if (!conv32) {
+    // columns below `rel` of the largest, among the k0 leading ones by norm
+    auto small_cols = [&](double rel, int* count) -> int {
       col_norms_k<float2><<<ceil_div((long)k * 32, TPB), TPB, 0, s>>>(B32, rows, rows, k, nrm);
       QR_CHECK_LAUNCH("col_norms_k");
       double* hn = static_cast<double*>(host_scratch(sizeof(double) * k));
@@ -2456,14 +2561,35 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
       QR_CUDA(cudaStreamSynchronize(s));
       std::vector<double> sn(hn, hn + k);
       std::sort(sn.begin(), sn.end(), std::greater<double>());
-      int small = 0;
-      for (int j = 0; j < k0; j++) small += sn[j] < kSmallCol * sn[0];
-      slow = small > kSmallColFrac * k0;
-      if (debug_on())
-        fprintf(stderr, "[qr] mixed %dx%d: FP32 probe: last sweep rotated %.4f of the pairs; %d of the %d polished "
-                "columns below %.0e sigma_max -> %s\n", rows, k, frac32, small, k0, kSmallCol,
-                slow ? "QR preconditioning" : "continue");
+      *count = 0;
+      for (int j = 0; j < k0; j++) *count += sn[j] < rel * sn[0];
+      return QR_OK;
+    };
+    int conv32 = 0, small = 0;
+    double frac32 = 0.0;
+    bool slow = false;
+    int ran = 0;
+    if (k > 128) {
+      // a few sweeps already order the columns by size
+      QR_TRY(jacobi<float>(s, w, B32, rows, rows, k, V32, k, kMixedFirstSweeps, tol32, false, kPrecondTanStop, &conv32,
+                           &frac32));
+      ran = kMixedFirstSweeps;
+      if (!conv32) {
+        QR_TRY(small_cols(kDecayCol, &small));
+        slow = small > kDecayFrac * k0;
+      }
     }
+    if (!conv32 && !slow) {
+      QR_TRY(jacobi<float>(s, w, B32, rows, rows, k, V32, k, kMixedProbeSweeps - ran, tol32, false, kPrecondTanStop,
+                           &conv32, &frac32));
+      if (!conv32) {
+        QR_TRY(small_cols(kSmallCol, &small));
+        slow = small > kSmallColFrac * k0 || frac32 > kSlowFrac;
+      }
+    }
+    if (debug_on() && !conv32)
+      fprintf(stderr, "[qr] mixed %dx%d: FP32 probe: last sweep rotated %.4f of the pairs; %d small of the %d polished "
+              "columns -> %s\n", rows, k, frac32, small, k0, slow ? "QR preconditioning" : "continue");
     if (!conv32 && !slow) {
       if (rows <= JR_MAXROWS && k > 128) {
         QR_TRY(jacobi_f32_masked(s, w, B32, rows, k, V32, 20 - kMixedProbeSweeps, tol32, kPrecondTanStop));
@@ -2483,57 +2609,8 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
       // relative test: on R^H the small columns are exact to FP32 precision, not rounding noise
       QR_TRY(jacobi<float>(s, w, B32, rows, rows, k, V32, k, 20, -tol32, false, kPrecondTanStop));
     }
-    // X = V32 with columns sorted by the FP32 column norms (descending), as a double-float
-    // matrix (low parts zero); the Newton-Schulz steps and B = A X run in double-float on the
-    // FP32 pipes and B goes straight into the double-float polish
-    col_norms_k<float2><<<ceil_div((long)k * 32, TPB), TPB, 0, s>>>(B32, rows, rows, k, nrm);
-    QR_CHECK_LAUNCH("col_norms_k");
-    rank_sort_k<<<ceil_div(k, TPB), TPB, 0, s>>>(nrm, k, perm, nullptr);
-    QR_CHECK_LAUNCH("rank_sort_k");
-    const size_t kk2 = (size_t)k * k, rk = (size_t)rows * k;
-    QR_TRY(w->X.ensure(sizeof(float2) * 2 * kk2, s));   // X (hi, lo)
-    QR_TRY(w->Rm.ensure(sizeof(float2) * 2 * kk2, s));  // Newton-Schulz output (hi, lo)
-    QR_TRY(w->E.ensure(sizeof(float2) * kk2, s));       // R = I - X^H X (FP32)
-    QR_TRY(w->T1.ensure(sizeof(float2) * 2 * rk, s));   // A (hi, lo)
-    QR_TRY(w->Bl.ensure(sizeof(float2) * rk, s));       // B low parts (high parts reuse B32)
-    float2 *Xh = w->X.as<float2>(), *Xl = Xh + kk2;
-    float2 *Yh = w->Rm.as<float2>(), *Yl = Yh + kk2;
-    float2* R = w->E.as<float2>();
-    float2 *Ah = w->T1.as<float2>(), *Al = Ah + rk;
-    float2 *Bh = B32, *Bl = w->Bl.as<float2>();
-    gather_cols_f2_k<<<gs((long)k * k), TPB, 0, s>>>(V32, k, k, k, perm, Xh, Xl, k);
-    QR_CHECK_LAUNCH("gather_cols_f2_k");
-    // X must be unitary to double-float accuracy before it carries the polish rotations: two
-    // Newton-Schulz steps X <- X + X (I - X^H X) / 2 square the FP32-level error twice
-    // (1e-6 -> 1e-12 -> rounding).  I - X^H X needs the compensated products; X R has |R| << 1,
-    // so FP32 products are accurate enough for the correction term.
-    for (int it = 0; it < 2; it++) {
-      QR_TRY(zgemm_df(s, DF_GRAM, OP_C, k, k, k, Xh, Xl, k, Xh, Xl, k, R, nullptr, k));
-      QR_TRY(zgemm_df(s, DF_F32_AXPY, OP_N, k, k, k, Xh, nullptr, k, R, nullptr, k, Yh, Yl, k, Xh, Xl, k, 0.5f));
-      std::swap(Xh, Yh);
-      std::swap(Xl, Yl);
-    }
-    // A (B holds A or A^H in FP64) scaled by a power of two so sigma_max ~ 1, then B = A X
-    double* smax_d = sorted;  // two scratch doubles; `sorted` is rewritten below
-    col_norms_k<double2><<<ceil_div((long)k * 32, TPB), TPB, 0, s>>>(B, rows, rows, k, nrm);
-    QR_CHECK_LAUNCH("col_norms_k");
-    max_reduce_k<<<1, 256, 0, s>>>(nrm, k, smax_d);
-    QR_CHECK_LAUNCH("max_reduce_k");
-    pow2_scale_k<double2><<<gs((long)rows * k), TPB, 0, s>>>(B, rows, rows, k, smax_d, smax_d + 1, 0);
-    QR_CHECK_LAUNCH("pow2_scale_k");
-    QR_TRY(z2df(s, B, rows, rows, k, nullptr, Ah, Al, rows));
-    QR_TRY(zgemm_df(s, DF_STORE, OP_N, rows, k, k, Ah, Al, rows, Xh, Xl, k, Bh, Bl, rows));
-    // Hestenes sweeps on (B, X) in double-float finish the near-degenerate pairs the FP32 sweeps
-    // leave and bring the couplings down to the double-float tolerance (inner products carry
-    // ~sqrt(rows) 2^-48 relative noise; the tolerance sits 2x above that floor)
-    // When only the leading `keep` triplets are used (truncation to maxdim), pairs inside the
-    // trailing block need no rotation: the cross pairs still decouple that block from the leading
-    // columns, and every tail column's norm stays below the tail's largest sigma, so the final
-    // sort separates the two sets.  The margin covers FP32 misordering at the boundary.
-    QR_TRY(jacobi_df(s, w, Bh, Bl, rows, rows, k, Xh, Xl, k, 40, 32.0 * sqrt((double)rows) * Eps<double>::v,
-                     smax_d, k0));
-    QR_TRY(df2z(s, Bh, Bl, rows, rows, k, smax_d + 1, B, rows));
-    QR_TRY(df2z(s, Xh, Xl, k, k, k, nullptr, V, k));
+    QR_TRY(finish_fp32(s, w, B, rows, k, B32, V32, V, 4.0 * sqrt((double)rows) * Eps<double>::v, k0, true));
+    refined = true;
   }
 
   // ---- sigma, ordering, factors
@@ -2565,6 +2642,7 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
     gather_cols_k<double2><<<gs((long)k * k), TPB, 0, s>>>(B, k, k, k, perm, sorted, L, k);
     QR_CHECK_LAUNCH("gather_cols_k");
     if (reorth) QR_TRY(reorthonormalize(s, w, L, k, k, kk));
+    else QR_TRY(polish_columns(s, w, L, k, k, kk));
     gather_cols_k<double2><<<gs((long)k * k), TPB, 0, s>>>(V, k, k, k, perm, nullptr, Rf, k);
     QR_CHECK_LAUNCH("gather_cols_k");
     const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
@@ -2585,6 +2663,7 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
     gather_cols_k<double2><<<gs((long)rows * k), TPB, 0, s>>>(B, rows, rows, k, perm, sorted, U, ldu);
     QR_CHECK_LAUNCH("gather_cols_k");
     if (reorth) QR_TRY(reorthonormalize(s, w, U, ldu, m, kk));
+    else if (refined) QR_TRY(polish_columns(s, w, U, ldu, m, kk));
     gather_cols_k<double2><<<gs((long)k * k), TPB, 0, s>>>(V, k, k, k, perm, nullptr, Rf, k);
     QR_CHECK_LAUNCH("gather_cols_k");
     QR_TRY(ztranspose(s, Rf, k, k, k, Vh, ldvh, 1));  // Vh = Rf^H (k x n)
@@ -2595,6 +2674,7 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
     gather_cols_k<double2><<<gs((long)rows * k), TPB, 0, s>>>(B, rows, rows, k, perm, sorted, L, rows);
     QR_CHECK_LAUNCH("gather_cols_k");
     if (reorth) QR_TRY(reorthonormalize(s, w, L, rows, rows, kk));
+    else if (refined) QR_TRY(polish_columns(s, w, L, rows, rows, kk));
     gather_cols_k<double2><<<gs((long)k * k), TPB, 0, s>>>(V, k, k, k, perm, nullptr, U, ldu);
     QR_CHECK_LAUNCH("gather_cols_k");
     QR_TRY(ztranspose(s, L, rows, rows, k, Vh, ldvh, 1));
