@@ -1,18 +1,15 @@
 // Thin complex SVD for canonize_site!(...; method=:svd) and evolve_2site!'s bond compression.
 //
-// QR_FP64 (plain): one-sided (Hestenes) Jacobi in FP64.  Columns of B = A (or A^H when A is
-// wide) are rotated pairwise until mutually orthogonal: B V = U Sigma.  Pairs follow the
-// round-robin (circle) ordering, so each round is n/2 independent pair rotations, one warp per
-// pair.  Converged when no pair has |b_p^H b_q| > tol sqrt(|b_p|^2 |b_q|^2), tol = sqrt(m) eps.
+// One-sided (Hestenes) Jacobi: columns of B = A (or A^H when A is wide) are rotated pairwise until
+// mutually orthogonal, B V = U Sigma.  Pairs follow the round-robin (circle) ordering.
 //
-// QR_MIXED: the same Jacobi in FP32 (FFMA runs ~70x faster than DFMA on GB300) gives
-// approximate right singular vectors X.  FP64 then takes over: two Newton-Schulz steps make X
-// unitary to FP64 (DMMA GEMMs), B = A X is formed in FP64, and FP64 Hestenes sweeps polish
-// (B, X); they start from couplings ~1e-5 and converge quadratically, so a few sweeps replace
-// the ~15 of the plain path.  Sigma = column norms of B in FP64, so singular values and the
-// truncation cutoff are FP64.  (A first-order Ogita-Aishima update was tried as the polish and
-// rejected: FP32 couplings (~1e-5 lambda_max) are not small against the lambda gaps of dense
-// random spectra (~5e-4 lambda_max at n = 2048), and the update lost orthogonality.)
+// FP64 runs at 1/70 of the FP32 rate here, so above a few dozen columns FP32 sweeps find the right
+// singular vectors X to ~1e-5 (svd_gram.cuh) and products at FP64 accuracy on the tensor cores finish
+// them (svd_refine.cuh); singular values, vectors and the truncation cutoff are FP64.
+//   QR_FP64: QR first, the sweeps on R^H; the finish to the FP64 sweeps' tolerance, one FP64 sweep to
+//            close it above 512 columns.  Up to 32 columns the whole Jacobi runs in FP64.
+//   QR_MIXED: the sweeps on B itself (on R^H when the spectrum decays), the finish to a few times that
+//            tolerance and only for the leading triplets when the caller keeps no more.
 //
 // Left singular vectors are the normalised columns B/sigma.  When the spectrum spans many
 // decades (or has exact zeros) those columns lose orthogonality in proportion to
@@ -32,6 +29,8 @@
 #include "prof.cuh"
 #include "jacobi_rot.cuh"
 #include "grid_sync.cuh"
+#include <map>
+#include <tuple>
 
 namespace qr {
 
@@ -577,19 +576,16 @@ __device__ __forceinline__ bool rotation_params_f32(float a, float b, float gr, 
   return true;
 }
 
-// ---- block Jacobi sweep (FP32 preconditioner, rows <= 2048) ------------------------------------
-// The k columns form blocks of JR_W = 4; a work item is a pair of blocks.  Each of the 512 threads
+// ---- listed block Jacobi sweep (FP32 preconditioner's last sweeps, rows <= 2048) ----------------
+// The k columns form blocks of JR_W = 4; a work item is a listed pair of blocks.  Each of the 512 threads
 // holds 4 rows of the item's 8 columns in registers, so a local round moves no column data
 // through memory: the four pairs' inner products come from registers, one transposed butterfly
 // reduces the 16 sums per warp, lanes 0-3 of warp 0 form the four rotations in parallel, and
-// every thread rotates its rows in place.  Round 0 of a sweep (where every block appears once)
-// takes all 28 pairs of the 8 columns (7 local rounds); later rounds take the 16 cross pairs (4
-// local rounds), so every pair is met once per sweep.  The 8 x 8 product J of the rotations is
+// every thread rotates its rows in place.  A `full` item takes all 28 pairs of the 8 columns (7 local
+// rounds), the others the 16 cross pairs (4 local rounds).  The 8 x 8 product J of the rotations is
 // accumulated in shared memory and V's 8 columns are updated once as V[:, cols] <- V[:, cols] J.
-// Per sweep each column moves through L2 (nb - 1) times instead of (k - 1) times and (nb - 1)
-// rounds are synchronised instead of (k - 1), with the same two orderings as the scalar sweep
-// (per-block flags or the grid barrier).  Pair indices are compile-time constants (unrolled local
-// rounds), so the column arrays stay in registers.
+// Narrow blocks keep the lists short; the full sweeps use wide ones (svd_gram.cuh).  Pair indices are
+// compile-time constants (unrolled local rounds), so the column arrays stay in registers.
 constexpr int JR_NT = 512, JR_RPT = 4, JR_C = 8, JR_W = 4;
 constexpr int JR_MAXROWS = JR_NT * JR_RPT;  // 2048
 
@@ -705,9 +701,8 @@ __device__ __forceinline__ void jr_local_round(float2 (&x)[JR_C][RPT], JrShared<
   }
 }
 
-// One work item: block pair (bp, bq) of round `round`.  VPRE (n <= NT): V's rows of the 8
-// columns are loaded with B's, before the local rounds, so their L2 round trip overlaps them.
-template <int NT, int RPT, bool VPRE>
+// One work item: block pair (bp, bq); round 0 also meets the pairs inside the blocks.
+template <int NT, int RPT>
 __device__ __forceinline__ void jr_block_pair(float2* __restrict__ B, long ldb, int m, int n, float2* __restrict__ V,
                                               long ldv, int nb, int bp, int bq, int round, float tol, float smax,
                                               unsigned* cnt, JrShared<NT>& sh) {
@@ -727,14 +722,6 @@ __device__ __forceinline__ void jr_block_pair(float2* __restrict__ B, long ldb, 
     for (int j = 0; j < RPT; j++) {
       const int r = tid + NT * j;
       x[l][j] = (c >= 0 && r < m) ? __ldcg(B + (long)c * ldb + r) : make_float2(0.f, 0.f);
-    }
-  }
-  float2 vpre[VPRE ? JR_C : 1];
-  if constexpr (VPRE) {
-#pragma unroll
-    for (int l = 0; l < JR_C; l++) {
-      const int c = sh.col[l];
-      vpre[l] = (c >= 0 && tid < n) ? __ldcg(V + (long)c * ldv + tid) : make_float2(0.f, 0.f);
     }
   }
   if (round == 0) {
@@ -763,23 +750,7 @@ __device__ __forceinline__ void jr_block_pair(float2* __restrict__ B, long ldb, 
       if (r < m) __stcg(B + (long)c * ldb + r, x[l][j]);
     }
   }
-  if constexpr (VPRE) {
-    if (tid < n) {
-#pragma unroll
-      for (int l2 = 0; l2 < JR_C; l2++) {
-        const int c = sh.col[l2];
-        if (c < 0) continue;
-        float2 o = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int l = 0; l < JR_C; l++) {
-          const float2 jv = sh.J[l2][l];
-          o.x += vpre[l].x * jv.x - vpre[l].y * jv.y;
-          o.y += vpre[l].x * jv.y + vpre[l].y * jv.x;
-        }
-        __stcg(V + (long)c * ldv + tid, o);
-      }
-    }
-  } else {
+  {
     for (int r0 = tid; r0 < n; r0 += 2 * NT) {
       float2 vin[2][JR_C];
 #pragma unroll
@@ -854,51 +825,28 @@ __device__ __forceinline__ void list_item(const MaskedList& L, unsigned i, int& 
 __global__ void __launch_bounds__(JR_NT, 1)
     jacobi_block_reg_k(float2* __restrict__ B, long ldb, int m, int n, float2* __restrict__ V, long ldv, int nbp,
                        float tol, const double* __restrict__ smax_p, unsigned* __restrict__ state, int sweep,
-                       unsigned* __restrict__ flags, float tan_stop, const unsigned* __restrict__ ml,
-                       unsigned* __restrict__ done) {
+                       float tan_stop, const unsigned* __restrict__ ml, unsigned* __restrict__ done) {
   __shared__ JrShared<JR_NT> sh;
   if (((volatile unsigned*)state)[0]) return;
   const float smax = (float)(smax_p[0] / smax_p[1]);
   unsigned* cnt = state + 8 + SW_STRIDE * sweep;
   const int nb = (n + JR_W - 1) / JR_W;
-  const int npairs = nbp / 2;
-  if (ml) {
-    // masked sweep: the listed block pairs (MaskedList over the nbp blocks) dealt round-robin to
-    // the CTAs; a block pair waits until the listed block pairs before it on each of its blocks
-    // are done, and `full` pairs also meet the pairs inside their blocks (as in round 0)
-    const MaskedList L = masked_list(ml, nbp);
-    const unsigned total = L.count[2];
-    for (unsigned i = blockIdx.x; i < total; i += gridDim.x) {
-      int bp, bq;
-      bool full;
-      list_item(L, i, bp, bq, full);
-      const unsigned op = L.ord[2 * (long)i], oq = L.ord[2 * (long)i + 1];
-      if (!wait_cols2(done, bp, bq, op, oq, state)) return;
-      jr_block_pair<JR_NT, JR_RPT, false>(B, ldb, m, n, V, ldv, nb, bp, bq, full ? 0 : 1, tol, smax, cnt, sh);
-      post_cols2(done, bp, bq, op + 1, oq + 1);
-    }
-    finish_sweep(state, cnt, sweep, tan_stop);
-    return;
-  }
-  const unsigned base = (unsigned)sweep * (unsigned)(nbp - 1);
-  const bool dataflow = npairs > (int)gridDim.x;
-  const long nit = dataflow ? ((long)(nbp - 1) * npairs - blockIdx.x + gridDim.x - 1) / gridDim.x : (long)(nbp - 1);
-  for (long t = 0; t < nit; t++) {
-    const long it = dataflow ? blockIdx.x + t * (long)gridDim.x : t * npairs + blockIdx.x;
-    const int round = (int)(it / npairs), pair = (int)(it % npairs);
+  // masked sweep: the listed block pairs (MaskedList over the nbp blocks) dealt round-robin to
+  // the CTAs; a block pair waits until the listed block pairs before it on each of its blocks
+  // are done, and `full` pairs also meet the pairs inside their blocks (as in round 0)
+  const MaskedList L = masked_list(ml, nbp);
+  const unsigned total = L.count[2];
+  for (unsigned i = blockIdx.x; i < total; i += gridDim.x) {
     int bp, bq;
-    pair_cols(nbp, round, pair, bp, bq);
-    if (dataflow && !wait_cols(flags, bp, bq, nb, base + round, state)) return;
-    if (bp < nb) jr_block_pair<JR_NT, JR_RPT, false>(B, ldb, m, n, V, ldv, nb, bp, bq, round, tol, smax, cnt, sh);
-    if (dataflow) post_cols(flags, bp, bq, nb, base + round + 1);
-    else {
-      __syncthreads();
-      if (!grid_barrier(state + 2)) return;
-    }
+    bool full;
+    list_item(L, i, bp, bq, full);
+    const unsigned op = L.ord[2 * (long)i], oq = L.ord[2 * (long)i + 1];
+    if (!wait_cols2(done, bp, bq, op, oq, state)) return;
+    jr_block_pair<JR_NT, JR_RPT>(B, ldb, m, n, V, ldv, nb, bp, bq, full ? 0 : 1, tol, smax, cnt, sh);
+    post_cols2(done, bp, bq, op + 1, oq + 1);
   }
   finish_sweep(state, cnt, sweep, tan_stop);
 }
-
 
 // Barrier over all threads of a thread-block cluster; release/acquire orders the global-memory
 // writes of a round before the reads of the next one.
@@ -907,43 +855,8 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
-// FP32 block Jacobi for k <= 128 columns of at most 128 rows: the whole iteration in one
-// thread-block cluster with one 128-thread CTA per block pair of a round (one row per thread,
-// V's rows prefetched with B's), the hardware cluster barrier between block rounds and all sweeps
-// in one launch.  A sweep has nb - 1 block rounds (nb = k / 4 blocks) instead of the scalar
-// kernel's k - 1 rounds; the local rounds inside a block pair need only CTA barriers.  state as in
-// jacobi_cluster_k.
 constexpr int JC_NT = 128;
-__global__ void __launch_bounds__(JC_NT) jacobi_block_cluster_k(float2* __restrict__ B, long ldb, int m, int n,
-                                                                float2* __restrict__ V, long ldv, float tol,
-                                                                const double* __restrict__ smax_p, int max_sweeps,
-                                                                unsigned* __restrict__ state, float tan_stop) {
-  __shared__ JrShared<JC_NT> sh;
-  const float smax = (float)(smax_p[0] / smax_p[1]);
-  const int nb = (n + JR_W - 1) / JR_W, nbp = nb + (nb & 1), npairs = nbp / 2;
-  int sweep = 0;
-  bool conv = false;
-  for (; sweep < max_sweeps && !conv; sweep++) {
-    unsigned* cnt = state + 8 + SW_STRIDE * sweep;
-    for (int round = 0; round < nbp - 1; round++) {
-      for (int pair = blockIdx.x; pair < npairs; pair += gridDim.x) {
-        int bp, bq;
-        pair_cols(nbp, round, pair, bp, bq);
-        if (bp < nb) jr_block_pair<JC_NT, 1, true>(B, ldb, m, n, V, ldv, nb, bp, bq, round, tol, smax, cnt, sh);
-        __syncthreads();  // shared state is reused by the next item
-      }
-      cluster_sync_all();
-    }
-    const unsigned h = __ldcg(cnt);
-    const float tmax = __uint_as_float(__ldcg(cnt + 1));
-    conv = h == 0 || tmax < tan_stop;
-    cluster_sync_all();  // everyone has read this sweep's counters
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    state[0] = conv ? 1u : 0u;
-    state[1] = sweep;
-  }
-}
+#include "svd_gram.cuh"
 
 // Small problems (k <= 128 columns): the whole Jacobi iteration in one thread-block cluster of up
 // to 16 CTAs.  Each warp owns a pair of the round (1-4 warps per CTA, so a round's work spreads
@@ -1699,18 +1612,19 @@ int jacobi(cudaStream_t s, SvdWork* w, cplx_t<T>* B, long ldb, int rows, int k, 
     QR_CHECK_LAUNCH("pow2_scale_k");
   }
   int pr = prof_begin(s, kind, 0.0, 0.0);
-  const bool small = k <= 128;  // (at 256 columns the FP32 block kernel is 2x faster than the cluster)
+  const bool small = k <= 128;
   if (small) {
     // one cluster of up to 16 CTAs with one warp per pair of a round: as many CTAs as pairs (up
     // to 16), then 2-4 warps per CTA
     // FP32 with at most 128 rows: the block form (one CTA per block pair of 4-column blocks)
     const bool blk = sizeof(T) == 4 && rows <= JC_NT && k > 2 * JR_W;
-    const int nbk = (k + JR_W - 1) / JR_W;
+    constexpr int bw = 8;
+    const int nbk = (k + bw - 1) / bw;
     const int npairs = blk ? (nbk + (nbk & 1)) / 2 : (np / 2 > 0 ? np / 2 : 1);
     const int cl = npairs < 16 ? npairs : 16;
     const int wpc = blk ? JC_NT / 32 : std::min(4, (npairs + cl - 1) / cl);  // warps loop over pairs
     if (cl > 8) {
-      const void* f = blk ? (const void*)jacobi_block_cluster_k : (const void*)jacobi_cluster_k<T>;
+      const void* f = blk ? (const void*)jacobi_gram_cluster_k<bw> : (const void*)jacobi_cluster_k<T>;
       QR_TRY(set_func_attr_once(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     }
     cudaLaunchConfig_t cfg = {};
@@ -1727,36 +1641,30 @@ int jacobi(cudaStream_t s, SvdWork* w, cplx_t<T>* B, long ldb, int rows, int k, 
     cfg.numAttrs = 1;
     svd_path(blk ? SP_BLOCK_CLUSTER : SP_CLUSTER);
     if (blk) {
-      QR_CUDA(cudaLaunchKernelEx(&cfg, jacobi_block_cluster_k, (float2*)B, ldb, rows, k, (float2*)V, ldv, (float)tol,
+      cfg.dynamicSmemBytes = gr_smem<bw, JC_NT>();
+      QR_CUDA(cudaLaunchKernelEx(&cfg, jacobi_gram_cluster_k<bw>, (float2*)B, ldb, rows, k, (float2*)V, ldv, (float)tol,
                                  (const double*)smax_d, max_sweeps, state, tan_stop));
     } else {
       QR_CUDA(cudaLaunchKernelEx(&cfg, jacobi_cluster_k<T>, B, ldb, rows, k, V, ldv, tol, (const double*)smax_d,
                                  max_sweeps, state, tan_stop));
     }
     count_launch();
-  } else if (sizeof(T) == 4 && rows <= JR_MAXROWS) {
-    // FP32 with the rows in registers: block Jacobi (4-column blocks, pairs of blocks)
-    const int nb = (k + JR_W - 1) / JR_W, nbp = nb + (nb & 1);
-    int per_sm = 0, sms = 0;
-    QR_TRY(device_sm_count(&sms));
-    QR_TRY(blocks_per_sm((const void*)jacobi_block_reg_k, JR_NT, 0, &per_sm));
-    if (per_sm < 1) return fail(QR_ECUDA, "block Jacobi sweep kernel cannot be resident");
-    int grid = std::min(per_sm * sms, nbp / 2);
-    if (grid < 1) grid = 1;
-    svd_path(nbp / 2 > grid ? SP_BLOCK_DATAFLOW : SP_BLOCK_BARRIER);
+  } else if (sizeof(T) == 4 && std::max(rows, k) <= GR_MAXROWS) {
+    GramPlan g;
+    QR_TRY(gram_plan(rows, k, &g));
+    svd_path(SP_BLOCK_DATAFLOW);
     for (int sweep = 0; sweep < max_sweeps; sweep++) {
-      float2* Bp = reinterpret_cast<float2*>(B);
-      float2* Vp = reinterpret_cast<float2*>(V);
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[2];
+      gram_config(g, &cfg, attr, s);
+      float2 *Bp = reinterpret_cast<float2*>(B), *Vp = reinterpret_cast<float2*>(V);
       long ldbb = ldb, ldvv = ldv;
-      int mm = rows, kk2 = k, nbb = nbp, sw = sweep;
+      int mm = rows, kk2 = k, nbb = g.nbp, sw = sweep, cs = g.cs;
       float tl = (float)tol, ts = tan_stop;
       const double* sm = smax_d;
-      unsigned* st = state;
-      unsigned* fl = flags;
-      const unsigned* mlp = nullptr;
-      unsigned* dn = nullptr;
-      void* args[] = {&Bp, &ldbb, &mm, &kk2, &Vp, &ldvv, &nbb, &tl, &sm, &st, &sw, &fl, &ts, &mlp, &dn};
-      QR_CUDA(cudaLaunchCooperativeKernel((const void*)jacobi_block_reg_k, dim3(grid), dim3(JR_NT), args, 0, s));
+      unsigned *st = state, *fl = flags;
+      void* args[] = {&Bp, &ldbb, &mm, &kk2, &Vp, &ldvv, &nbb, &tl, &sm, &st, &sw, &fl, &ts, &cs};
+      QR_CUDA(cudaLaunchKernelExC(&cfg, g.kernel, args));
       count_launch();
     }
   } else {
@@ -2316,10 +2224,9 @@ static int jacobi_f32_masked(cudaStream_t s, SvdWork* w, float2* B, int rows, in
       float tl = tol, ts = tan_stop;
       const double* sm = smax_d;
       unsigned* st = state;
-      unsigned* fl = done;  // unused in list mode
       const unsigned* mlp = ml;
       unsigned* dn = done;
-      void* args[] = {&Bp, &ldbb, &mm, &kk2, &Vp, &ldvv, &nbb, &tl, &sm, &st, &sw, &fl, &ts, &mlp, &dn};
+      void* args[] = {&Bp, &ldbb, &mm, &kk2, &Vp, &ldvv, &nbb, &tl, &sm, &st, &sw, &ts, &mlp, &dn};
       QR_CUDA(cudaLaunchCooperativeKernel((const void*)jacobi_block_reg_k, dim3(grid), dim3(JR_NT), args, 0, s));
       count_launch();
     }

@@ -1,5 +1,5 @@
-"""The SVD's finish by matrix products: sizes around the cluster / listed-sweep limits, kept triplets, and
-spectra that steer it (degenerate and clustered values fall back to sweeps, graded ones restart on R^H).
+"""The SVD's FP32 sweeps on Gram matrices and its finish by matrix products: sizes around the limits of their
+launches, kept triplets, and spectra that steer it (degenerate and clustered values fall back to sweeps, graded ones restart on R^H).
 
 Both precisions must give LAPACK's values and factors orthonormal and exact to rounding: 1e-12 relative to
 sigma_max covers sqrt(512) eps with a factor 200; the clustered spectrum in mixed precision ends in
@@ -40,7 +40,10 @@ def check(mode, A, tol=1e-12):
 
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("m,n", [(17, 17), (33, 90), (128, 128), (129, 128), (129, 129), (130, 300), (191, 191),
-                                 (192, 192), (400, 193), (2049, 130), (513, 513)])
+                                 (192, 192), (400, 193), (2049, 130), (513, 513),
+                                 # FP32 sweeps: 8- and 16-column blocks, one CTA of 256 rows, clusters of 128-row
+                                 # and 256-row CTAs with a ragged last one, odd block counts, rows beyond a cluster
+                                 (256, 136), (257, 140), (385, 137), (897, 140), (1300, 161), (4096, 129), (4097, 129)])
 def test_sizes(mode, m, n):
     check(mode, R.complex_gaussian(R.rng(m * 7 + n), (m, n)))
 
