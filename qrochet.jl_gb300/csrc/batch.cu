@@ -16,7 +16,7 @@
 //     re-orthonormalisation of the kept vectors when their singular values fall below 1e-3
 //     sigma_max (classical Gram-Schmidt twice), and the write-back of U, Vh and Lambda.  A
 //     layer's gates sit on disjoint bonds, so the CTAs of one launch never touch the same site;
-//   - the expectation values are one more launch: one CTA per Pauli string sweeps the chain's
+//   - the expectation values are one more launch: one cluster per Pauli string sweeps the chain's
 //     environment (FP64).
 // The layer kernel's CTA size comes from a small autotuner (timed on synthetic gate steps of the
 // batch's largest bond class, cached per device and class, optionally in a file).
@@ -507,12 +507,23 @@ __global__ void __launch_bounds__(512, 1)
   }
 }
 
-// ---- expectation values of Pauli strings: one CTA per string, FP64 environment sweep ----------
+// ---- expectation values of Pauli strings: one cluster per string, FP64 environment sweep --------
 // E[a, a'] (ket a, bra a') from the left; per site X[a', o, r] = sum_a E[a, a'] A[a, o, r], then
 // E'[r, r'] = sum_{a', o'} conj(A[a', o', r']) sum_o P[o', o] X[a', o, r], times Lambda_r Lambda_r'
-// when the bond to the right holds a Lambda.  ws: 3 * 64 * 128 double2 per CTA.
+// when the bond to the right holds a Lambda.  A Pauli string's environment is Hermitian, so half of
+// E' is computed and E[a, a'] is read as conj(E[a', a]), which puts the lanes on consecutive values.
+//
+// Bound by the FP64 rate of the SMs that work on the longest chain: 6 chi^3 complex multiply-adds a
+// site at 0.5 DFMA per clock and scheduler.  So the columns r of a site are dealt to the CTAs of a
+// cluster: X for a CTA's own columns stays in its shared memory, E goes through L2, and one cluster
+// barrier ends the site.  The longest of 64 strings (40 sites, chi 64) took 47.7 ms on one CTA.
+// ws: 2 * 64 * 64 double2 per string.
+constexpr int BX_CL = 8;     // CTAs per string
+constexpr int BX_NT = 384;   // 9 warps' worth of E' at chi = 64: three per scheduler at most
+constexpr int BX_OWN = (BT_MAXCHI + BX_CL - 1) / BX_CL;
+
+// the part of pauli code's row op in (P x)[op] for x = (x0, x1)
 __device__ __forceinline__ double2 pauli_apply(int code, int op, const double2& x0, const double2& x1) {
-  // (P x)[op] for x = (x0, x1)
   switch (code) {
     case 1: return op == 0 ? x1 : x0;                                                    // X
     case 2: return op == 0 ? make_double2(x1.y, -x1.x) : make_double2(-x0.y, x0.x);      // Y
@@ -521,49 +532,68 @@ __device__ __forceinline__ double2 pauli_apply(int code, int op, const double2& 
   }
 }
 
-__global__ void batch_expect_k(const BObs* __restrict__ obs, int nobs, double2* __restrict__ ws) {
-  const BObs O = obs[blockIdx.x];
-  double2* E0 = ws + (size_t)blockIdx.x * 3 * BT_MAXCHI * BT_MAXK;
+__global__ void __launch_bounds__(BX_NT) batch_expect_k(const BObs* __restrict__ obs, double2* __restrict__ ws) {
+  __shared__ double2 X[(2 * BT_MAXCHI + 1) * BX_OWN];
+  const int str = blockIdx.x / BX_CL, rank = blockIdx.x % BX_CL;
+  const BObs O = obs[str];
+  double2* E0 = ws + (size_t)str * 2 * BT_MAXCHI * BT_MAXCHI;
   double2* E1 = E0 + BT_MAXCHI * BT_MAXCHI;
-  double2* X = E1 + BT_MAXCHI * BT_MAXCHI;
-  if (threadIdx.x == 0) E0[0] = make_double2(1.0, 0.0);
-  __syncthreads();
-  int ce = 1;  // current environment side
+  if (rank == 0 && threadIdx.x == 0) E0[0] = make_double2(1.0, 0.0);
+  __syncwarp();
+  cluster_sync_all();
   for (int i = 0; i < O.n; i++) {
     const double2* A = O.sites[i];
     const int cl = i > 0 ? O.bd[i - 1] : 1, cr = i + 1 < O.n ? O.bd[i] : 1;
     const int code = O.pauli[i];
-    // X[a', o, r] (a' fastest), 2 cl cr entries
-    for (int t = threadIdx.x; t < cl * 2 * cr; t += blockDim.x) {
-      const int ap = t % cl, orr = t / cl;  // orr = o + 2 r
+    const int r0 = cr * rank / BX_CL, own = cr * (rank + 1) / BX_CL - r0, ld = 2 * cl + 1;
+    // X[a', o, r] (a' fastest) of the own columns
+    for (int t = threadIdx.x; t < cl * 2 * own; t += BX_NT) {
+      const int ap = t % cl, orr = t / cl;  // orr = o + 2 (r - r0)
+      const double2* col = A + (long)cl * (2 * r0 + orr);
       double2 acc = make_double2(0.0, 0.0);
-      for (int a = 0; a < ce; a++) acc = cadd(acc, zmul(E0[a + ce * ap], A[a + (long)cl * orr]));
-      X[t] = acc;
+#pragma unroll 4
+      for (int a = 0; a < cl; a++) {
+        const double2 e = __ldcg(E0 + ap + cl * a), v = col[a];
+        acc.x = fma(e.x, v.x, fma(e.y, v.y, acc.x));
+        acc.y = fma(e.x, v.y, fma(-e.y, v.x, acc.y));
+      }
+      X[(orr >> 1) * ld + (orr & 1) * cl + ap] = acc;
     }
     __syncthreads();
     const bool lam_on = i + 1 < O.n && O.haslam[i];
     const double* lam = lam_on ? O.lams[i] : nullptr;
-    for (int t = threadIdx.x; t < cr * cr; t += blockDim.x) {
-      const int r = t % cr, rp = t / cr;
+    // row r of E' meets r' = r, r + 1, .. r + cr / 2 (mod cr): every CTA has the same share of the pairs
+    const int half = cr / 2 + 1;
+    for (int t = threadIdx.x; t < own * half; t += BX_NT) {
+      const int rl = t % own, j = t / own, r = r0 + rl;
+      int rp = r + j;
+      if (rp >= cr) rp -= cr;
+      if (2 * j == cr && rp < r) continue;  // the other end of this pair has it
+      const double2* x = X + rl * ld;
+      const double2* col = A + (long)cl * 2 * rp;
       double2 acc = make_double2(0.0, 0.0);
+#pragma unroll 2
       for (int ap = 0; ap < cl; ap++) {
-        const double2 x0 = X[ap + cl * (0 + 2 * r)], x1 = X[ap + cl * (1 + 2 * r)];
+        const double2 x0 = x[ap], x1 = x[cl + ap];
 #pragma unroll
         for (int op = 0; op < 2; op++) {
-          const double2 y = pauli_apply(code, op, x0, x1);
-          acc = cadd(acc, cmulc(A[ap + (long)cl * (op + 2 * rp)], y));
+          const double2 y = pauli_apply(code, op, x0, x1), v = col[ap + cl * op];
+          acc.x = fma(v.x, y.x, fma(v.y, y.y, acc.x));
+          acc.y = fma(v.x, y.y, fma(-v.y, y.x, acc.y));
         }
       }
       if (lam_on) acc = cscale(acc, lam[r] * lam[rp]);
-      E1[t] = acc;
+      if (j == 0) acc.y = 0.0;
+      __stcg(E1 + r + cr * rp, acc);
+      if (j) __stcg(E1 + rp + cr * r, cconj(acc));
     }
-    __syncthreads();
+    __syncwarp();
+    cluster_sync_all();
     double2* tmp = E0;
     E0 = E1;
     E1 = tmp;
-    ce = cr;
   }
-  if (threadIdx.x == 0) O.out[0] = E0[0];
+  if (rank == 0 && threadIdx.x == 0) O.out[0] = __ldcg(E0);
 }
 
 // state init: every site of every chain becomes |0> = (1, 0) in a (1, 2, 1) array
@@ -581,6 +611,23 @@ __global__ void batch_fill_k(double2* p, long count, double scale) {
     p[t] = make_double2(scale * ((double)(h1 & 0xffffff) / 16777216.0 - 0.5),
                         scale * ((double)(h2 & 0xffffff) / 16777216.0 - 0.5));
   }
+}
+
+// clusters x cl CTAs of nt threads
+template <typename... P, typename... A>
+cudaError_t launch_cluster(void (*kern)(P...), unsigned clusters, int cl, int nt, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(clusters * cl);
+  cfg.blockDim = dim3(nt);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cl;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
 
 int cap_of(int n, int b, int chi_max) {
@@ -887,7 +934,7 @@ int qr_batch_run(qr_batch* bt, double* ms) try {
   // workspace slots: enough CTAs to fill the GPU with the largest candidate CTA
   const int slots = sms * 4;
   const size_t o_ws = take(sizeof(double2) * BT_SLOT * slots);
-  const size_t o_ews = take(sizeof(double2) * 3 * BT_MAXCHI * BT_MAXK * std::max(1, nobs_total));
+  const size_t o_ews = take(sizeof(double2) * 2 * BT_MAXCHI * BT_MAXCHI * std::max(1, nobs_total));
   char* base = nullptr;
   {
     cudaError_t e = cudaMallocAsync((void**)&base, off, s);
@@ -993,8 +1040,8 @@ int qr_batch_run(qr_batch* bt, double* ms) try {
     launches++;
   }
   if (!obs.empty()) {
-    batch_expect_k<<<(unsigned)obs.size(), 256, 0, s>>>(reinterpret_cast<const BObs*>(base + o_obs), (int)obs.size(),
-                                                         reinterpret_cast<double2*>(base + o_ews));
+    QR_CUDA(launch_cluster(batch_expect_k, (unsigned)obs.size(), BX_CL, BX_NT, s,
+                           reinterpret_cast<const BObs*>(base + o_obs), reinterpret_cast<double2*>(base + o_ews)));
     launches++;
   }
   cudaError_t ce = cudaStreamEndCapture(s, &graph);

@@ -1,5 +1,5 @@
 // One-sided (Hestenes) Jacobi building blocks shared by the SVD kernels (svd.cu) and the batched
-// gate-step kernel (batch.cu): machine epsilons, a warp sum, the plane rotation of a column pair
+// gate-step kernel (batch.cu): machine epsilons, a warp sum, the cluster barrier, the plane rotation of a column pair
 // and its parameters.
 #pragma once
 #include "common.cuh"
@@ -15,6 +15,13 @@ template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
+}
+
+// Barrier over all threads of a thread-block cluster (its warps converged); release/acquire orders the
+// global-memory writes of a round before the reads of the next one.
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
 template <typename C, typename T>

@@ -848,13 +848,6 @@ __global__ void __launch_bounds__(JR_NT, 1)
   finish_sweep(state, cnt, sweep, tan_stop);
 }
 
-// Barrier over all threads of a thread-block cluster; release/acquire orders the global-memory
-// writes of a round before the reads of the next one.
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-
 constexpr int JC_NT = 128;
 #include "svd_gram.cuh"
 
