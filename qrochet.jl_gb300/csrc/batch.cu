@@ -31,6 +31,7 @@
 #include "kernels.cuh"
 #include "jacobi_rot.cuh"
 #include "jacobi_df.cuh"
+#include "gram_item.cuh"
 
 namespace qr {
 namespace {
@@ -38,8 +39,16 @@ namespace {
 constexpr int BT_MAXK = 128;         // largest theta side: chi_max <= 64
 constexpr int BT_MAXCHI = BT_MAXK / 2;
 constexpr int BT_MAX_SWEEPS = 60;
-constexpr size_t BT_SLOT = 4 * (size_t)BT_MAXK * BT_MAXK;  // B, V, W, Tm (double2) per CTA slot
-constexpr int BT_MIXED_MIN = 32;  // the mixed SVD precondition in FP32 above this many columns
+// per cluster: six squares, a column of coefficients, one of norms and the sweep counters (double2)
+constexpr size_t BT_SLOT = 6 * (size_t)BT_MAXK * BT_MAXK + 2 * BT_MAXK;
+constexpr int BT_PRE_MIN = 16;   // the SVD sweeps in FP32 first above this many columns
+constexpr int BT_MIXED_MIN = 32;  // with QR_MIXED, the finish is in double-float above this many columns
+constexpr int BT_MAXTEAM = 8;    // CTAs per gate step
+
+__device__ __forceinline__ void cfma(double2& acc, double2 a, double2 b) {
+  acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
+  acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
+}
 
 struct BTask {
   double2* sl;          // left site buffer
@@ -64,165 +73,275 @@ struct BObs {
 };
 
 // ---- the fused gate step ------------------------------------------------------------------------
-__device__ __forceinline__ double2 zmul(double2 a, double2 b) { return cmul(a, b); }
+// One cluster of 1 to 8 CTAs runs one gate step; every phase is dealt to the cluster's threads or
+// warps, and the data goes through L2.  `Team` is this thread's place in it.
+struct Team {
+  int size, rank;       // CTAs, this CTA
+  int tid, nt;          // thread of the cluster, its threads
+  int lane, warp, nw;   // warp of the cluster, its warps
+  __device__ __forceinline__ void sync() const {
+    if (size == 1) {
+      __syncthreads();
+    } else {
+      __syncwarp();
+      cluster_sync_all();
+    }
+  }
+};
 
-// Hestenes sweeps of one CTA on B (rows x k, ld rows) accumulating V (k x k, ld k) in precision
-// T: round-robin pairs, one warp per pair, a CTA barrier between rounds.  Stops after a sweep that
-// rotates nothing or whose largest rotation tangent is below tan_stop; returns that verdict.
-template <typename T>
-__device__ bool cta_sweeps(cplx_t<T>* __restrict__ B, cplx_t<T>* __restrict__ V, int rows, int k, T tol, T smax,
-                           int max_sweeps, float tan_stop, unsigned* rot_count, unsigned* tmax_bits) {
-  using Cx = cplx_t<T>;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// Rotations and largest tangent of a sweep, counted by the whole team: sweep s uses slot s % 3 and clears
+// the next one, which was last read two barriers ago.
+struct SweepCount {
+  unsigned* c;  // 3 x 2 words in global memory
+  __device__ __forceinline__ void start(const Team& T) const {
+    if (T.tid == 0) { __stcg(c, 0u); __stcg(c + 1, 0u); }
+  }
+  __device__ __forceinline__ unsigned* open(const Team& T, int sweep) const {
+    unsigned* nx = c + 2 * ((sweep + 1) % 3);
+    if (T.tid == 0) { __stcg(nx, 0u); __stcg(nx + 1, 0u); }
+    return c + 2 * (sweep % 3);
+  }
+  static __device__ __forceinline__ void add(unsigned* s, float tabs) {
+    atomicAdd(s, 1u);
+    atomicMax(s + 1, __float_as_uint(tabs));
+  }
+  static __device__ __forceinline__ bool done(const unsigned* s, float tan_stop) {
+    return __ldcg(s) == 0u || __uint_as_float(__ldcg(s + 1)) < tan_stop;
+  }
+};
+
+// pair `pair` of round `round` over np (even) columns, p < q
+__device__ __forceinline__ void round_pair(int np, int round, int pair, int& p, int& q) {
+  if (pair == 0) { p = round; q = np - 1; }
+  else { p = (round + pair) % (np - 1); q = (round - pair + np - 1) % (np - 1); }
+  if (p > q) { const int x = p; p = q; q = x; }
+}
+
+constexpr int BT_RPL = BT_MAXK / 32;  // rows a lane
+
+// FP64 Hestenes sweeps of the team on B (rows x k, ld rows) accumulating V (k x k, ld k): round-robin pairs,
+// one warp per pair with the columns' rows in registers, a team barrier between rounds.  Stops after a sweep
+// that rotates nothing or whose largest rotation tangent is below tan_stop; returns that verdict.
+__device__ bool team_sweeps(const Team& T, double2* B, double2* V, int rows, int k, double tol, double smax,
+                            int max_sweeps, float tan_stop, SweepCount cnt) {
   const int np = k + (k & 1), npairs = np / 2;
   bool converged = false;
+  cnt.start(T);
+  T.sync();
   for (int sweep = 0; sweep < max_sweeps && !converged; sweep++) {
-    if (threadIdx.x == 0) { *rot_count = 0u; *tmax_bits = 0u; }
-    __syncthreads();
+    unsigned* sc = cnt.open(T, sweep);
     for (int round = 0; round < np - 1; round++) {
-      for (int pair = warp; pair < npairs; pair += nw) {
+      for (int pair = T.warp; pair < npairs; pair += T.nw) {
         int p, q;
-        if (pair == 0) { p = round; q = np - 1; }
-        else { p = (round + pair) % (np - 1); q = (round - pair + np - 1) % (np - 1); }
-        if (p > q) { const int x = p; p = q; q = x; }
+        round_pair(np, round, pair, p, q);
         if (q >= k) continue;
-        Cx* bp = B + (long)rows * p;
-        Cx* bq = B + (long)rows * q;
-        T a = 0, bb = 0, gr = 0, gi = 0;
-        for (int r = lane; r < rows; r += 32) {
-          const Cx x = bp[r], y = bq[r];
-          a += x.x * x.x + x.y * x.y;
-          bb += y.x * y.x + y.y * y.y;
-          gr += x.x * y.x + x.y * y.y;
-          gi += x.x * y.y - x.y * y.x;
+        double2 *bp = B + (long)rows * p, *bq = B + (long)rows * q, *vp = V + (long)k * p, *vq = V + (long)k * q;
+        double2 x[BT_RPL], y[BT_RPL], u[BT_RPL], w[BT_RPL];
+        double a = 0, bb = 0, gr = 0, gi = 0;
+#pragma unroll
+        for (int j = 0; j < BT_RPL; j++) {
+          const int r = T.lane + 32 * j;
+          x[j] = y[j] = u[j] = w[j] = make_double2(0.0, 0.0);
+          if (r < rows) { x[j] = __ldcg(bp + r); y[j] = __ldcg(bq + r); }
+          if (r < k) { u[j] = __ldcg(vp + r); w[j] = __ldcg(vq + r); }
+        }
+#pragma unroll
+        for (int j = 0; j < BT_RPL; j++) {
+          if (32 * j >= rows) break;  // no arithmetic on rows that no lane has
+          a += x[j].x * x[j].x + x[j].y * x[j].y;
+          bb += y[j].x * y[j].x + y[j].y * y[j].y;
+          gr += x[j].x * y[j].x + x[j].y * y[j].y;
+          gi += x[j].x * y[j].y - x[j].y * y[j].x;
         }
         a = warp_sum(a); bb = warp_sum(bb); gr = warp_sum(gr); gi = warp_sum(gi);
-        T c, sr, si;
+        double c, sr, si;
         float tabs;
-        if (!rotation_params<T>(a, bb, gr, gi, tol, smax, c, sr, si, tabs)) continue;
-        for (int r = lane; r < rows; r += 32) {
-          Cx x = bp[r], y = bq[r];
-          rot(x, y, c, sr, si);
-          bp[r] = x;
-          bq[r] = y;
+        if (!rotation_params<double>(a, bb, gr, gi, tol, smax, c, sr, si, tabs)) continue;
+#pragma unroll
+        for (int j = 0; j < BT_RPL; j++) {
+          const int r = T.lane + 32 * j;
+          if (32 * j < rows) {
+            rot(x[j], y[j], c, sr, si);
+            if (r < rows) { __stcg(bp + r, x[j]); __stcg(bq + r, y[j]); }
+          }
+          if (32 * j < k) {
+            rot(u[j], w[j], c, sr, si);
+            if (r < k) { __stcg(vp + r, u[j]); __stcg(vq + r, w[j]); }
+          }
         }
-        Cx* vp = V + (long)k * p;
-        Cx* vq = V + (long)k * q;
-        for (int r = lane; r < k; r += 32) {
-          Cx x = vp[r], y = vq[r];
-          rot(x, y, c, sr, si);
-          vp[r] = x;
-          vq[r] = y;
-        }
-        if (lane == 0) {
-          atomicAdd(rot_count, 1u);
-          atomicMax(tmax_bits, __float_as_uint(tabs));
-        }
+        if (T.lane == 0) SweepCount::add(sc, tabs);
       }
-      __syncthreads();
+      T.sync();
     }
-    converged = *rot_count == 0u || __uint_as_float(*tmax_bits) < tan_stop;
-    __syncthreads();
+    converged = SweepCount::done(sc, tan_stop);
   }
   return converged;
 }
 
-// ---- the mixed finish in double-float (FP32 pairs, on the FP32 pipes) ----------------------------
-// One CTA's double-float Hestenes sweeps on B (Bh, Bl: rows x k, ld rows) accumulating V (Vh,
-// Vl: k x k, ld k): round-robin pairs, one warp per pair.  Every lane forms the pair's
-// compensated sums over its rows, the warp reduces them, and every lane derives the same rotation
-// from the broadcast sums (rotation_params_df), so a pair needs no shared memory; a CTA barrier
-// between rounds.  Stops after a sweep that rotates nothing or whose largest tangent is below
-// tan_stop; returns that verdict.
-__device__ bool cta_sweeps_df(float2* __restrict__ Bh, float2* __restrict__ Bl, float2* __restrict__ Vh,
-                              float2* __restrict__ Vl, int rows, int k, float tol, float smax, int max_sweeps,
-                              float tan_stop, unsigned* rot_count, unsigned* tmax_bits) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// The mixed finish: the same sweeps in double-float (FP32 pairs, on the FP32 pipes) on B (Bh, Bl: rows x k,
+// ld rows) accumulating V (Vh, Vl: k x k, ld k).  Every lane forms the pair's compensated sums over its rows,
+// the warp reduces them, and every lane derives the same rotation from the broadcast sums.
+__device__ bool team_sweeps_df(const Team& T, float2* Bh, float2* Bl, float2* Vh, float2* Vl, int rows, int k, float tol,
+                               float smax, int max_sweeps, float tan_stop, SweepCount cnt) {
   const int np = k + (k & 1), npairs = np / 2;
   bool converged = false;
+  cnt.start(T);
+  T.sync();
   for (int sweep = 0; sweep < max_sweeps && !converged; sweep++) {
-    if (threadIdx.x == 0) { *rot_count = 0u; *tmax_bits = 0u; }
-    __syncthreads();
+    unsigned* sc = cnt.open(T, sweep);
     for (int round = 0; round < np - 1; round++) {
-      for (int pair = warp; pair < npairs; pair += nw) {
+      for (int pair = T.warp; pair < npairs; pair += T.nw) {
         int p, q;
-        if (pair == 0) { p = round; q = np - 1; }
-        else { p = (round + pair) % (np - 1); q = (round - pair + np - 1) % (np - 1); }
-        if (p > q) { const int x = p; p = q; q = x; }
+        round_pair(np, round, pair, p, q);
         if (q >= k) continue;
-        float2 *bph = Bh + (long)rows * p, *bpl = Bl + (long)rows * p;
-        float2 *bqh = Bh + (long)rows * q, *bql = Bl + (long)rows * q;
+        const long cp = (long)rows * p, cq = (long)rows * q, dp = (long)k * p, dq = (long)k * q;
+        float2 xh[BT_RPL], xl[BT_RPL], yh[BT_RPL], yl[BT_RPL], uh[BT_RPL], ul[BT_RPL], wh[BT_RPL], wl[BT_RPL];
+#pragma unroll
+        for (int j = 0; j < BT_RPL; j++) {
+          const int r = T.lane + 32 * j;
+          xh[j] = xl[j] = yh[j] = yl[j] = uh[j] = ul[j] = wh[j] = wl[j] = make_float2(0.f, 0.f);
+          if (r < rows) {
+            xh[j] = __ldcg(Bh + cp + r); xl[j] = __ldcg(Bl + cp + r);
+            yh[j] = __ldcg(Bh + cq + r); yl[j] = __ldcg(Bl + cq + r);
+          }
+          if (r < k) {
+            uh[j] = __ldcg(Vh + dp + r); ul[j] = __ldcg(Vl + dp + r);
+            wh[j] = __ldcg(Vh + dq + r); wl[j] = __ldcg(Vl + dq + r);
+          }
+        }
         DotAcc a{0.f, 0.f}, b{0.f, 0.f}, gr{0.f, 0.f}, gi{0.f, 0.f};
-        for (int r = lane; r < rows; r += 32) df_dot_acc(bph[r], bpl[r], bqh[r], bql[r], a, b, gr, gi);
+#pragma unroll
+        for (int j = 0; j < BT_RPL; j++) {
+          if (32 * j >= rows) break;
+          df_dot_acc(xh[j], xl[j], yh[j], yl[j], a, b, gr, gi);
+        }
         const dfl k4 = df_warp_sum4_t(dot_final(a), dot_final(b), dot_final(gr), dot_final(gi));
         DfParams P;
         if (!rotation_params_df(df_shfl(k4, 0), df_shfl(k4, 8), df_shfl(k4, 16), df_shfl(k4, 24), tol, smax, P))
           continue;
-        for (int r = lane; r < rows; r += 32) {
-          float2 xh = bph[r], xl = bpl[r], yh = bqh[r], yl = bql[r];
-          df_rot_any(xh, xl, yh, yl, P);
-          bph[r] = xh; bpl[r] = xl; bqh[r] = yh; bql[r] = yl;
+#pragma unroll
+        for (int j = 0; j < BT_RPL; j++) {
+          const int r = T.lane + 32 * j;
+          if (r < rows) {
+            df_rot_any(xh[j], xl[j], yh[j], yl[j], P);
+            __stcg(Bh + cp + r, xh[j]); __stcg(Bl + cp + r, xl[j]);
+            __stcg(Bh + cq + r, yh[j]); __stcg(Bl + cq + r, yl[j]);
+          }
+          if (r < k) {
+            df_rot_any(uh[j], ul[j], wh[j], wl[j], P);
+            __stcg(Vh + dp + r, uh[j]); __stcg(Vl + dp + r, ul[j]);
+            __stcg(Vh + dq + r, wh[j]); __stcg(Vl + dq + r, wl[j]);
+          }
         }
-        float2 *vph = Vh + (long)k * p, *vpl = Vl + (long)k * p;
-        float2 *vqh = Vh + (long)k * q, *vql = Vl + (long)k * q;
-        for (int r = lane; r < k; r += 32) {
-          float2 xh = vph[r], xl = vpl[r], yh = vqh[r], yl = vql[r];
-          df_rot_any(xh, xl, yh, yl, P);
-          vph[r] = xh; vpl[r] = xl; vqh[r] = yh; vql[r] = yl;
-        }
-        if (lane == 0) {
-          atomicAdd(rot_count, 1u);
-          atomicMax(tmax_bits, __float_as_uint(P.tabs));
-        }
+        if (T.lane == 0) SweepCount::add(sc, P.tabs);
       }
-      __syncthreads();
+      T.sync();
     }
-    converged = *rot_count == 0u || __uint_as_float(*tmax_bits) < tan_stop;
-    __syncthreads();
+    converged = SweepCount::done(sc, tan_stop);
   }
   return converged;
 }
 
-// R = I - X^H X (FP32 values of compensated double-float sums), X = (Xh, Xl) k x k, ld k.
-__device__ void cta_gram_df(const float2* __restrict__ Xh, const float2* __restrict__ Xl, int k, float2* __restrict__ R) {
-  for (int t = threadIdx.x; t < k * k; t += blockDim.x) {
-    const int i = t % k, j = t / k;
+// FP32 sweeps on Gram matrices of block pairs (gram_item.cuh), an item a CTA; up to BT_MAXK rows.
+constexpr int BT_W = 8;
+constexpr size_t BT_TILE = gr_smem<BT_W, BT_MAXK>() / sizeof(float2);
+__device__ void team_sweeps_f32(const Team& T, float2* B, float2* V, int rows, int k, float tol, float smax,
+                                int max_sweeps, float tan_stop, SweepCount cnt, GrShared<BT_W>& sh, float2* tile) {
+  const int nb = (k + BT_W - 1) / BT_W, nbp = nb + (nb & 1), npairs = nbp / 2;
+  bool converged = false;
+  cnt.start(T);
+  T.sync();
+  for (int sweep = 0; sweep < max_sweeps && !converged; sweep++) {
+    unsigned* sc = cnt.open(T, sweep);
+    for (int round = 0; round < nbp - 1; round++) {
+      for (int pair = T.rank; pair < npairs; pair += T.size) {
+        int bp, bq;
+        round_pair(nbp, round, pair, bp, bq);
+        if (bq < nb || round == 0) {
+          if (blockDim.x == BT_MAXK)
+            gr_item<BT_W, BT_MAXK>(B, rows, rows, k, V, k, nb, bp, bq, round == 0, tol, smax, sc, sh, tile, 0, 0, 1);
+          else if (threadIdx.x < 2 * BT_MAXK)
+            gr_item<BT_W, 2 * BT_MAXK, true>(B, rows, rows, k, V, k, nb, bp, bq, round == 0, tol, smax, sc, sh, tile, 0,
+                                             0, 1);
+        }
+        __syncthreads();  // shared state is reused by the next item
+      }
+      T.sync();
+    }
+    converged = SweepCount::done(sc, tan_stop);
+  }
+}
+
+// R = I - X^H X from X's transpose Xt (k x k, ld k), half of it computed: lanes on consecutive columns of X,
+// column i with column i - d.  FP32 values of compensated double-float sums.
+__device__ void team_gram_df(const Team& T, const float2* Th, const float2* Tl, int k, float2* R) {
+  for (int t = T.tid; t < k * (k / 2 + 1); t += T.nt) {
+    const int i = t % k, d = t / k, j = i >= d ? i - d : i - d + k;
+    if (2 * d == k && i < j) continue;  // the pair's other end has it
     DotAcc re{0.f, 0.f}, im{0.f, 0.f};
     for (int x = 0; x < k; x++) {
-      const float2 ah = Xh[x + (long)k * i], al = Xl[x + (long)k * i];
-      const float2 bh = Xh[x + (long)k * j], bl = Xl[x + (long)k * j];
+      const float2 ah = Th[i + k * x], al = Tl[i + k * x], bh = Th[j + k * x], bl = Tl[j + k * x];
       dot2_step(re, ah.x, al.x, bh.x, bl.x);  // conj(a) b
       dot2_step(re, ah.y, al.y, bh.y, bl.y);
       dot2_step(im, ah.x, al.x, bh.y, bl.y);
       dot2_step(im, -ah.y, -al.y, bh.x, bl.x);
     }
-    const dfl r = df_add({i == j ? 1.f : 0.f, 0.f}, df_neg(dot_final(re))), m = df_neg(dot_final(im));
-    R[t] = make_float2(r.h + r.l, m.h + m.l);
+    const dfl r = df_add({d == 0 ? 1.f : 0.f, 0.f}, df_neg(dot_final(re))), m = df_neg(dot_final(im));
+    const float2 v = make_float2(r.h + r.l, d == 0 ? 0.f : m.h + m.l);
+    R[i + k * j] = v;
+    if (d) R[j + k * i] = make_float2(v.x, -v.y);
+  }
+}
+// the same with FP64 sums of FP64 values
+__device__ void team_gram(const Team& T, const double2* Xt, int k, float2* R) {
+  for (int t = T.tid; t < k * (k / 2 + 1); t += T.nt) {
+    const int i = t % k, d = t / k, j = i >= d ? i - d : i - d + k;
+    if (2 * d == k && i < j) continue;  // the pair's other end has it
+    double re = d == 0 ? -1.0 : 0.0, im = 0.0;
+#pragma unroll 4
+    for (int x = 0; x < k; x++) {
+      const double2 a = Xt[i + k * x], b = Xt[j + k * x];
+      re = fma(a.x, b.x, fma(a.y, b.y, re));
+      im = fma(a.x, b.y, fma(-a.y, b.x, im));
+    }
+    const float2 v = make_float2((float)-re, d == 0 ? 0.f : (float)-im);
+    R[i + k * j] = v;
+    if (d) R[j + k * i] = make_float2(v.x, -v.y);
   }
 }
 
-// Y = X + X_hi R / 2: FP32 products (|R| << 1), double-float sum; k x k, ld k.
-__device__ void cta_ns_update(const float2* __restrict__ Xh, const float2* __restrict__ Xl, const float2* __restrict__ R,
-                              int k, float2* __restrict__ Yh, float2* __restrict__ Yl) {
-  for (int t = threadIdx.x; t < k * k; t += blockDim.x) {
-    const int i = t % k, j = t / k;
-    float ar = 0.f, ai = 0.f;
-    for (int x = 0; x < k; x++) {
-      const float2 a = Xh[i + (long)k * x], r = R[x + (long)k * j];
-      ar = fmaf(a.x, r.x, fmaf(-a.y, r.y, ar));
-      ai = fmaf(a.x, r.y, fmaf(a.y, r.x, ai));
-    }
-    const dfl yr = df_add_f({Xh[t].x, Xl[t].x}, 0.5f * ar), yi = df_add_f({Xh[t].y, Xl[t].y}, 0.5f * ai);
+// X_hi R / 2 at element t: FP32 products (|R| << 1)
+__device__ __forceinline__ float2 half_product(const float2* Xh, const float2* R, int k, int t) {
+  const int i = t % k, j = t / k;
+  float ar = 0.f, ai = 0.f;
+  for (int x = 0; x < k; x++) {
+    const float2 a = Xh[i + (long)k * x], r = R[x + (long)k * j];
+    ar = fmaf(a.x, r.x, fmaf(-a.y, r.y, ar));
+    ai = fmaf(a.x, r.y, fmaf(a.y, r.x, ai));
+  }
+  return make_float2(0.5f * ar, 0.5f * ai);
+}
+
+// Y = X + X_hi R / 2 in double-float and its transpose; k x k, ld k.
+__device__ void team_ns_df(const Team& T, const float2* Xh, const float2* Xl, const float2* R, int k, float2* Yh, float2* Yl,
+                           float2* Th, float2* Tl) {
+  for (int t = T.tid; t < k * k; t += T.nt) {
+    const float2 a = half_product(Xh, R, k, t);
+    const dfl yr = df_add_f({Xh[t].x, Xl[t].x}, a.x), yi = df_add_f({Xh[t].y, Xl[t].y}, a.y);
     Yh[t] = make_float2(yr.h, yi.h);
     Yl[t] = make_float2(yr.l, yi.l);
+    if (Th) {
+      const int tt = t / k + k * (t % k);
+      Th[tt] = Yh[t];
+      Tl[tt] = Yl[t];
+    }
   }
 }
 
 // C = A X in double-float: A (Ah, Al) rows x k (ld rows), X (Xh, Xl) k x k, C rows x k (ld rows).
-__device__ void cta_gemm_df(const float2* __restrict__ Ah, const float2* __restrict__ Al, int rows,
-                            const float2* __restrict__ Xh, const float2* __restrict__ Xl, int k, float2* __restrict__ Ch,
-                            float2* __restrict__ Cl) {
-  for (int t = threadIdx.x; t < rows * k; t += blockDim.x) {
+__device__ void team_gemm_df(const Team& T, const float2* Ah, const float2* Al, int rows, const float2* Xh,
+                             const float2* Xl, int k, float2* Ch, float2* Cl) {
+  for (int t = T.tid; t < rows * k; t += T.nt) {
     const int i = t % rows, j = t / rows;
     DotAcc re{0.f, 0.f}, im{0.f, 0.f};
     for (int x = 0; x < k; x++) {
@@ -238,33 +357,121 @@ __device__ void cta_gemm_df(const float2* __restrict__ Ah, const float2* __restr
     Cl[t] = make_float2(r.l, m.l);
   }
 }
+__device__ void team_gemm(const Team& T, const double2* A, int rows, const double2* X, int k, double2* C) {
+  for (int t = T.tid; t < rows * k; t += T.nt) {
+    const int i = t % rows, j = t / rows;
+    double2 c = make_double2(0.0, 0.0);
+#pragma unroll 4
+    for (int x = 0; x < k; x++) {
+      const double2 a = A[i + (long)rows * x], b = X[x + (long)k * j];
+      c.x = fma(a.x, b.x, fma(-a.y, b.y, c.x));
+      c.y = fma(a.x, b.y, fma(a.y, b.x, c.y));
+    }
+    C[t] = c;
+  }
+}
 
-// One CTA per task (strided over the layer's tasks).  ws: BT_SLOT double2 per CTA.  dry = 1 runs
-// the arithmetic without writing the chain (the autotuner's timing runs).  MIXED: above
-// BT_MIXED_MIN columns the SVD first runs FP32 sweeps on a copy of theta (64x the FP64 rate on
-// this part), then finishes in double-float on the FP32 pipes: two Newton-Schulz steps
-// X <- X + X (I - X^H X) / 2 make the rotations unitary to rounding, B = theta X is formed with
-// compensated products, and double-float sweeps (cta_sweeps_df) finish from couplings of ~1e-6
-// in two or three sweeps.  The FP64 finish this replaces kept the FP64 pipe 76 % busy.
+// column norms of B (rows x k, ld rows) into nrm (global), and into every CTA's sig after the barrier
+__device__ void team_norms(const Team& T, const double2* B, int rows, int k, double* nrm, double* sig) {
+  for (int j = T.warp; j < k; j += T.nw) {
+    double s = 0.0;
+    for (int r = T.lane; r < rows; r += 32) {
+      const double2 v = B[r + (long)rows * j];
+      s += v.x * v.x + v.y * v.y;
+    }
+    s = warp_sum(s);
+    if (T.lane == 0) __stcg(nrm + j, sqrt(s));
+  }
+  T.sync();
+  for (int j = threadIdx.x; j < k; j += blockDim.x) sig[j] = __ldcg(nrm + j);
+  __syncthreads();
+}
+
+// W's first `keep` columns (rows x keep, ld rows, nearly unit) made orthonormal, each column's direction and
+// phase kept: classical Gram-Schmidt twice.  A column's updates are dealt out by row, 8 lanes to a row.
+__device__ void team_orthonormalise(const Team& T, double2* W, int rows, int keep, double2* coef) {
+  for (int j = 0; j < keep; j++) {
+    double2* wj = W + (long)rows * j;
+    for (int pass = 0; pass < 2 && j > 0; pass++) {
+      for (int i = T.warp; i < j; i += T.nw) {
+        const double2* wi = W + (long)rows * i;
+        double re = 0.0, im = 0.0;
+        for (int r = T.lane; r < rows; r += 32) {
+          const double2 x = wi[r], y = wj[r];
+          re += x.x * y.x + x.y * y.y;
+          im += x.x * y.y - x.y * y.x;
+        }
+        re = warp_sum(re);
+        im = warp_sum(im);
+        if (T.lane == 0) coef[i] = make_double2(re, im);
+      }
+      T.sync();
+      for (int r0 = 4 * T.warp; r0 < rows; r0 += 4 * T.nw) {
+        const int r = r0 + (T.lane >> 3);
+        double2 v = make_double2(0.0, 0.0);
+        if (r < rows)
+          for (int i = T.lane & 7; i < j; i += 8) v = cadd(v, cmul(W[r + (long)rows * i], coef[i]));
+        for (int o = 4; o > 0; o >>= 1) {
+          v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+          v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+        }
+        if (r < rows && (T.lane & 7) == 0) wj[r] = csub(wj[r], v);
+      }
+      T.sync();
+    }
+    if (j == 0) continue;
+    // every warp forms the norm of the column, then scales its share of the rows
+    double s = 0.0;
+    for (int r = T.lane; r < rows; r += 32) s += wj[r].x * wj[r].x + wj[r].y * wj[r].y;
+    s = warp_sum(s);
+    const double inv = s > 0.0 ? 1.0 / sqrt(s) : 0.0;
+    T.sync();
+    for (int r = T.tid; r < rows; r += T.nt) wj[r] = cscale(wj[r], inv);
+    T.sync();
+  }
+}
+
+// One cluster per task (strided over the layer's tasks).  ws: BT_SLOT double2 per cluster.  dry = 1 runs
+// the arithmetic without writing the chain (the autotuner's timing runs).
+//
+// Above BT_PRE_MIN columns the SVD first runs FP32 sweeps on a copy of theta (64x the FP64 rate on
+// this part): two Newton-Schulz steps X <- X + X (I - X^H X) / 2 make their rotations unitary to rounding,
+// B = theta X is formed, and full-precision sweeps finish from couplings of ~1e-6 in two or three sweeps:
+// in FP64, or with MIXED in double-float on the FP32 pipes.
+//
+// What bounds a step is its chain of rounds: 127 of them in a sweep of 128 columns.  On one CTA a
+// double-float sweep of theta 128 x 128 needs 1.4 ms of its SM's FP32 rate and an FP64 sweep ~10, so a layer of
+// saturated bonds took 20 ms while most SMs idled.  A cluster deals the rounds' pairs out to up to 8 SMs, and
+// the FP32 sweeps run 15 rounds a sweep on Gram matrices.
 template <bool MIXED>
 __global__ void __launch_bounds__(512, 1)
-    batch_gate_k(const BTask* __restrict__ tasks, int ntasks, double2* __restrict__ ws, int dry) {
+    batch_gate_k(const BTask* __restrict__ tasks, int ntasks, double2* __restrict__ ws, int dry, int team) {
   __shared__ BTask T;
   __shared__ double2 G[16];
   __shared__ double sig[BT_MAXK], srt[BT_MAXK];
   __shared__ int perm[BT_MAXK];
-  __shared__ unsigned rot_count, tmax_bits;
-  __shared__ double red[32];
-  __shared__ double2 coef[BT_MAXK];
   __shared__ double scale_f, smax_s;
   __shared__ int keep_s, reorth_s;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  double2* B = ws + (size_t)blockIdx.x * BT_SLOT;
-  double2* V = B + (size_t)BT_MAXK * BT_MAXK;
-  double2* W = V + (size_t)BT_MAXK * BT_MAXK;
-  double2* Tm = W + (size_t)BT_MAXK * BT_MAXK;
+  __shared__ GrShared<BT_W> gsh;
+  __shared__ __align__(16) float2 tile[BT_TILE];
+  Team M;
+  M.size = team;
+  M.rank = blockIdx.x % team;
+  M.tid = M.rank * blockDim.x + threadIdx.x;
+  M.nt = team * blockDim.x;
+  M.lane = threadIdx.x & 31;
+  M.warp = M.tid >> 5;
+  M.nw = M.nt >> 5;
+  const int tid = threadIdx.x;
+  constexpr size_t K2 = (size_t)BT_MAXK * BT_MAXK;
+  // the slot: theta | V | W | three work squares | norms, coefficients, counters
+  double2* TH = ws + (size_t)(blockIdx.x / team) * BT_SLOT;
+  double2 *Vv = TH + K2, *W = Vv + K2, *S0 = W + K2, *S1 = S0 + K2, *S2 = S1 + K2;
+  double2* coef = S2 + K2;
+  double* nrm = reinterpret_cast<double*>(coef + BT_MAXK);
+  const SweepCount cnt{reinterpret_cast<unsigned*>(nrm + BT_MAXK)};
 
-  for (int ti = blockIdx.x; ti < ntasks; ti += gridDim.x) {
+  for (int ti = blockIdx.x / team; ti < ntasks; ti += gridDim.x / team) {
     if (tid == 0) T = tasks[ti];
     __syncthreads();
     if (tid < 16) G[tid] = T.gate[tid];
@@ -274,21 +481,24 @@ __global__ void __launch_bounds__(512, 1)
     const bool tall = m >= nn;
     const int rows = tall ? m : nn, k = tall ? nn : m;
     const bool lam_on = T.haslam[b] != 0;
+    const bool pre = k > BT_PRE_MIN, df = MIXED && k > BT_MIXED_MIN;
+    double2 *B = TH, *V = Vv;  // the sweeps' columns and rotations
     __syncthreads();
 
-    // ---- theta' = G (A_l diag(Lambda) A_r), into B (tall) or B = theta'^H (wide)
-    for (int t = tid; t < cl * cr; t += blockDim.x) {
+    // ---- theta' = G (A_l diag(Lambda) A_r), into TH (tall) or TH = theta'^H (wide)
+    for (int t = M.tid; t < cl * cr; t += M.nt) {
       const int l = t % cl, r = t / cl;
       double2 acc[2][2];
       acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = make_double2(0.0, 0.0);
+#pragma unroll 2
       for (int x = 0; x < cc; x++) {
         const double w = lam_on ? T.lam[x] : 1.0;
         const double2 a0 = cscale(T.sl[l + (long)cl * (2 * x)], w), a1 = cscale(T.sl[l + (long)cl * (1 + 2 * x)], w);
         const double2 b0 = T.sr[x + (long)cc * (2 * r)], b1 = T.sr[x + (long)cc * (1 + 2 * r)];
-        acc[0][0] = cadd(acc[0][0], zmul(a0, b0));
-        acc[0][1] = cadd(acc[0][1], zmul(a0, b1));
-        acc[1][0] = cadd(acc[1][0], zmul(a1, b0));
-        acc[1][1] = cadd(acc[1][1], zmul(a1, b1));
+        cfma(acc[0][0], a0, b0);
+        cfma(acc[0][1], a0, b1);
+        cfma(acc[1][0], a1, b0);
+        cfma(acc[1][1], a1, b1);
       }
 #pragma unroll
       for (int p1 = 0; p1 < 2; p1++)
@@ -298,115 +508,128 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll
           for (int o1 = 0; o1 < 2; o1++)
 #pragma unroll
-            for (int o2 = 0; o2 < 2; o2++) v = cadd(v, zmul(G[(2 * p1 + p2) * 4 + 2 * o1 + o2], acc[o1][o2]));
+            for (int o2 = 0; o2 < 2; o2++) cfma(v, G[(2 * p1 + p2) * 4 + 2 * o1 + o2], acc[o1][o2]);
           const int rt = l + cl * p1, ct = p2 + 2 * r;
-          if (tall) B[rt + (long)rows * ct] = v;
-          else B[ct + (long)rows * rt] = cconj(v);
+          if (tall) TH[rt + (long)rows * ct] = v;
+          else TH[ct + (long)rows * rt] = cconj(v);
         }
     }
-    for (int t = tid; t < k * k; t += blockDim.x) V[t] = make_double2((t % k) == (t / k) ? 1.0 : 0.0, 0.0);
-    __syncthreads();
+    M.sync();
 
     // ---- column norms, power-of-two prescale (sigma_max of the scaled columns in [1/2, 1))
-    for (int j = warp; j < k; j += nw) {
-      double s = 0.0;
-      for (int r = lane; r < rows; r += 32) {
-        const double2 v = B[r + (long)rows * j];
-        s += v.x * v.x + v.y * v.y;
-      }
-      s = warp_sum(s);
-      if (lane == 0) sig[j] = sqrt(s);
-    }
-    __syncthreads();
-    if (tid == 0) {
+    team_norms(M, TH, rows, k, nrm, sig);
+    if (tid < 32) {
       double mx = 0.0;
-      for (int j = 0; j < k; j++) mx = fmax(mx, sig[j]);
-      int e = 0;
-      if (mx > 0.0) frexp(mx, &e);
-      scale_f = ldexp(1.0, e);
-      smax_s = mx > 0.0 ? ldexp(mx, -e) : 0.0;
+      for (int j = tid; j < k; j += 32) mx = fmax(mx, sig[j]);
+      for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      if (tid == 0) {
+        int e = 0;
+        if (mx > 0.0) frexp(mx, &e);
+        scale_f = ldexp(1.0, e);
+        smax_s = mx > 0.0 ? ldexp(mx, -e) : 0.0;
+      }
     }
     __syncthreads();
-    {
-      const double inv = 1.0 / scale_f;
-      for (int t = tid; t < rows * k; t += blockDim.x) B[t] = cscale(B[t], inv);
-    }
-    __syncthreads();
-
-    // ---- Hestenes sweeps (optionally preconditioned in FP32)
-    const double tol = sqrt((double)rows) * Eps<double>::v;
     const double smax = smax_s;
-    if (MIXED && k > BT_MIXED_MIN) {
-      float2* B32 = reinterpret_cast<float2*>(W);
-      float2* V32 = B32 + (size_t)rows * k;
-      for (int t = tid; t < rows * k; t += blockDim.x) B32[t] = make_float2((float)B[t].x, (float)B[t].y);
-      for (int t = tid; t < k * k; t += blockDim.x) V32[t] = make_float2((t % k) == (t / k) ? 1.f : 0.f, 0.f);
-      __syncthreads();
-      const float tol32 = fmaxf(4e-6f, 2.f * sqrtf((float)rows) * Eps<float>::v);
-      cta_sweeps<float>(B32, V32, rows, k, tol32, (float)smax, 20, 0.15f, &rot_count, &tmax_bits);
-      // the finish in double-float on the FP32 pipes.  The CTA's four slot regions (B, V, W, Tm;
-      // 2 BT_MAXK^2 float2 each) hold, phase by phase:
-      //   W: B32 | V32 -> theta (hi | lo) -> X (hi | lo) before the conversion back
-      //   Tm: X0 (hi | lo) -> R2 | X2 hi
-      //   V: R1 | X1 hi -> B' (hi | lo) -> V (FP64)
-      //   B: theta (FP64) -> X1 lo | X2 lo -> B (FP64)
-      constexpr size_t H = (size_t)BT_MAXK * BT_MAXK;  // float2 per half region
-      float2 *rW = reinterpret_cast<float2*>(W), *rT = reinterpret_cast<float2*>(Tm);
-      float2 *rV = reinterpret_cast<float2*>(V), *rB = reinterpret_cast<float2*>(B);
-      for (int t = tid; t < k * k; t += blockDim.x) { rT[t] = V32[t]; rT[H + t] = make_float2(0.f, 0.f); }
-      __syncthreads();
-      for (int t = tid; t < rows * k; t += blockDim.x) {
-        const dfl re = df_from(B[t].x), im = df_from(B[t].y);
-        rW[t] = make_float2(re.h, im.h);
-        rW[H + t] = make_float2(re.l, im.l);
+    {
+      // (the FP32 sweeps' copies in S0: B32 | V32)
+      const double inv = 1.0 / scale_f;
+      float2* B32 = reinterpret_cast<float2*>(S0);
+      for (int t = M.tid; t < rows * k; t += M.nt) {
+        const double2 v = cscale(TH[t], inv);
+        TH[t] = v;
+        if (pre) B32[t] = make_float2((float)v.x, (float)v.y);
       }
-      __syncthreads();
-      // two Newton-Schulz steps X <- X + X (I - X^H X) / 2 (1e-6 -> 1e-12 -> rounding)
-      cta_gram_df(rT, rT + H, k, rV);
-      __syncthreads();
-      cta_ns_update(rT, rT + H, rV, k, rV + H, rB);
-      __syncthreads();
-      cta_gram_df(rV + H, rB, k, rT);
-      __syncthreads();
-      cta_ns_update(rV + H, rB, rT, k, rT + H, rB + H);
-      __syncthreads();
-      float2 *Xh = rT + H, *Xl = rB + H;
-      // B' = theta X into V's region, then the double-float sweeps on (B', X)
-      cta_gemm_df(rW, rW + H, rows, Xh, Xl, k, rV, rV + H);
-      __syncthreads();
-      const float toldf = (float)(32.0 * sqrt((double)rows) * Eps<double>::v);
-      const bool conv_df = cta_sweeps_df(rV, rV + H, Xh, Xl, rows, k, toldf, (float)smax, BT_MAX_SWEEPS, 1e-7f,
-                                         &rot_count, &tmax_bits);
-      if (!conv_df && tid == 0) atomicExch(T.status, (int)QR_ENOCONV);
-      // back to FP64: X into W first (its lo part sits in B's region), then B, then V
-      for (int t = tid; t < k * k; t += blockDim.x) { rW[t] = Xh[t]; rW[H + t] = Xl[t]; }
-      __syncthreads();
-      for (int t = tid; t < rows * k; t += blockDim.x) {
-        const float2 h = rV[t], l = rV[H + t];
-        B[t] = make_double2((double)h.x + l.x, (double)h.y + l.y);
+      for (int t = M.tid; t < k * k; t += M.nt) {
+        const bool d = (t % k) == (t / k);
+        if (pre) B32[K2 + t] = make_float2(d ? 1.f : 0.f, 0.f);
+        else V[t] = make_double2(d ? 1.0 : 0.0, 0.0);
       }
-      __syncthreads();
-      for (int t = tid; t < k * k; t += blockDim.x) {
-        const float2 h = rW[t], l = rW[H + t];
-        V[t] = make_double2((double)h.x + l.x, (double)h.y + l.y);
-      }
-      __syncthreads();
     }
-    const bool converged = (MIXED && k > BT_MIXED_MIN) ||
-                           cta_sweeps<double>(B, V, rows, k, tol, smax, BT_MAX_SWEEPS, 1e-8f, &rot_count, &tmax_bits);
-    if (!converged && tid == 0) atomicExch(T.status, (int)QR_ENOCONV);
+    M.sync();
+
+    // ---- Hestenes sweeps, preconditioned in FP32
+    const double tol = sqrt((double)rows) * Eps<double>::v;
+    bool converged = false;
+    if (pre) {
+      float2 *B32 = reinterpret_cast<float2*>(S0), *V32 = B32 + K2;
+      const float tol32 = fmaxf(4e-6f, 2.f * sqrtf((float)rows) * Eps<float>::v);
+      team_sweeps_f32(M, B32, V32, rows, k, tol32, (float)smax, 20, 0.15f, cnt, gsh, tile);
+      if (df) {
+        // halves of the squares: S0 B32 | X0 -> B' (hi | lo), S1 theta (hi | lo), S2 X0's transpose -> X1's
+        // (hi | lo) -> X2 (hi | lo), W X1 (hi | lo), V R | zeros
+        float2 *h0 = reinterpret_cast<float2*>(S0), *h1 = reinterpret_cast<float2*>(S1), *h2 = reinterpret_cast<float2*>(S2);
+        float2 *hV = reinterpret_cast<float2*>(V), *hW = reinterpret_cast<float2*>(W);
+        float2 *X0 = V32, *zero = hV + K2;
+        for (int t = M.tid; t < k * k; t += M.nt) {
+          h2[t / k + k * (t % k)] = X0[t];
+          zero[t] = make_float2(0.f, 0.f);
+        }
+        for (int t = M.tid; t < rows * k; t += M.nt) {
+          const dfl re = df_from(TH[t].x), im = df_from(TH[t].y);
+          h1[t] = make_float2(re.h, im.h);
+          h1[K2 + t] = make_float2(re.l, im.l);
+        }
+        M.sync();
+        team_gram_df(M, h2, zero, k, hV);  // 1e-6 -> 1e-12 -> rounding
+        M.sync();
+        team_ns_df(M, X0, zero, hV, k, hW, hW + K2, h2, h2 + K2);
+        M.sync();
+        team_gram_df(M, h2, h2 + K2, k, hV);
+        M.sync();
+        float2 *Xh = h2, *Xl = h2 + K2;  // (the transposes have been read)
+        team_ns_df(M, hW, hW + K2, hV, k, Xh, Xl, nullptr, nullptr);
+        M.sync();
+        team_gemm_df(M, h1, h1 + K2, rows, Xh, Xl, k, h0, h0 + K2);
+        const float toldf = (float)(32.0 * sqrt((double)rows) * Eps<double>::v);
+        converged = team_sweeps_df(M, h0, h0 + K2, Xh, Xl, rows, k, toldf, (float)smax, BT_MAX_SWEEPS, 1e-7f, cnt);
+        for (int t = M.tid; t < rows * k; t += M.nt) {
+          const float2 h = h0[t], l = h0[K2 + t];
+          B[t] = make_double2((double)h.x + l.x, (double)h.y + l.y);
+        }
+        for (int t = M.tid; t < k * k; t += M.nt) {
+          const float2 h = Xh[t], l = Xl[t];
+          V[t] = make_double2((double)h.x + l.x, (double)h.y + l.y);
+        }
+        M.sync();
+      } else {
+        // the same in FP64 (the steps' corrections X R / 2 in FP32, |R| ~ 1e-6 and 1e-12; the first step's
+        // R needs no more than double-float sums): S1 X0's transpose | zeros -> X2, S2 X1's transpose, W X1,
+        // V R | X1 hi
+        double2 *Xt = S2, *X1 = W;
+        float2 *R = reinterpret_cast<float2*>(V), *Xf = R + K2, *Tf = reinterpret_cast<float2*>(S1);
+        for (int t = M.tid; t < k * k; t += M.nt) {
+          Tf[t / k + k * (t % k)] = V32[t];
+          Tf[K2 + t] = make_float2(0.f, 0.f);
+        }
+        M.sync();
+        team_gram_df(M, Tf, Tf + K2, k, R);
+        M.sync();
+        for (int t = M.tid; t < k * k; t += M.nt) {
+          const float2 a = half_product(V32, R, k, t);
+          const double2 v = make_double2((double)V32[t].x + a.x, (double)V32[t].y + a.y);
+          X1[t] = v;
+          Xt[t / k + k * (t % k)] = v;
+          Xf[t] = make_float2((float)v.x, (float)v.y);
+        }
+        M.sync();
+        team_gram(M, Xt, k, R);
+        M.sync();
+        for (int t = M.tid; t < k * k; t += M.nt) {
+          const float2 a = half_product(Xf, R, k, t);
+          S1[t] = make_double2(X1[t].x + a.x, X1[t].y + a.y);
+        }
+        M.sync();
+        team_gemm(M, TH, rows, S1, k, S0);
+        B = S0;
+        V = S1;
+      }
+    }
+    if (!df) converged = team_sweeps(M, B, V, rows, k, tol, smax, BT_MAX_SWEEPS, 1e-8f, cnt);
+    if (!converged && M.tid == 0) atomicExch(T.status, (int)QR_ENOCONV);
 
     // ---- sigma, descending order (ties by index), truncation on the device
-    for (int j = warp; j < k; j += nw) {
-      double s = 0.0;
-      for (int r = lane; r < rows; r += 32) {
-        const double2 v = B[r + (long)rows * j];
-        s += v.x * v.x + v.y * v.y;
-      }
-      s = warp_sum(s);
-      if (lane == 0) sig[j] = sqrt(s);
-    }
-    __syncthreads();
+    team_norms(M, B, rows, k, nrm, sig);
     for (int j = tid; j < k; j += blockDim.x) {
       int rank = 0;
       const double v = sig[j];
@@ -421,7 +644,7 @@ __global__ void __launch_bounds__(512, 1)
       int kp = 0;
       while (kp < upto && fabs(srt[kp] * scale_f) > thr) kp++;
       if (kp == 0) {  // the chain would be left with an empty bond: keep one vector, flag the request
-        atomicExch(T.status, (int)QR_EINVAL);
+        if (M.rank == 0) atomicExch(T.status, (int)QR_EINVAL);
         kp = 1;
       }
       keep_s = kp;
@@ -431,79 +654,39 @@ __global__ void __launch_bounds__(512, 1)
     const int keep = keep_s;
 
     // ---- the kept left vectors of B (columns perm[j] / sigma) into W
-    for (int t = tid; t < rows * keep; t += blockDim.x) {
+    for (int t = M.tid; t < rows * keep; t += M.nt) {
       const int r = t % rows, j = t / rows;
       const double s = srt[j];
       W[r + (long)rows * j] = s > 0.0 ? cscale(B[r + (long)rows * perm[j]], 1.0 / s) : make_double2(0.0, 0.0);
     }
-    __syncthreads();
-    if (reorth_s) {
-      // classical Gram-Schmidt twice: keeps each column's direction and phase, orthonormal to ~eps
-      for (int j = 1; j < keep; j++) {
-        double2* wj = W + (long)rows * j;
-        for (int pass = 0; pass < 2; pass++) {
-          for (int i = warp; i < j; i += nw) {
-            const double2* wi = W + (long)rows * i;
-            double cr_ = 0.0, ci_ = 0.0;
-            for (int r = lane; r < rows; r += 32) {
-              const double2 x = wi[r], y = wj[r];
-              cr_ += x.x * y.x + x.y * y.y;
-              ci_ += x.x * y.y - x.y * y.x;
-            }
-            cr_ = warp_sum(cr_);
-            ci_ = warp_sum(ci_);
-            if (lane == 0) coef[i] = make_double2(cr_, ci_);
-          }
-          __syncthreads();
-          for (int r = tid; r < rows; r += blockDim.x) {
-            double2 v = wj[r];
-            for (int i = 0; i < j; i++) v = csub(v, zmul(W[r + (long)rows * i], coef[i]));
-            wj[r] = v;
-          }
-          __syncthreads();
-        }
-        double s = 0.0;
-        for (int r = tid; r < rows; r += blockDim.x) s += wj[r].x * wj[r].x + wj[r].y * wj[r].y;
-        s = warp_sum(s);
-        if (lane == 0) red[warp] = s;
-        __syncthreads();
-        if (tid == 0) {
-          double tot = 0.0;
-          for (int w = 0; w < nw; w++) tot += red[w];
-          red[0] = tot > 0.0 ? 1.0 / sqrt(tot) : 0.0;
-        }
-        __syncthreads();
-        const double inv = red[0];
-        for (int r = tid; r < rows; r += blockDim.x) wj[r] = cscale(wj[r], inv);
-        __syncthreads();
-      }
-    }
+    M.sync();
+    if (reorth_s) team_orthonormalise(M, W, rows, keep, coef);
 
     // ---- write-back: A_l (cl, 2, keep), A_r (keep, 2, cr), Lambda, bond dimension
     if (!dry) {
       if (tall) {  // theta = W S (V[:, perm])^H
-        for (int t = tid; t < m * keep; t += blockDim.x) T.sl[t] = W[t % m + (long)rows * (t / m)];
-        for (int t = tid; t < keep * nn; t += blockDim.x) {
+        for (int t = M.tid; t < m * keep; t += M.nt) T.sl[t] = W[t % m + (long)rows * (t / m)];
+        for (int t = M.tid; t < keep * nn; t += M.nt) {
           const int j = t % keep, col = t / keep;
           T.sr[t] = cconj(V[col + (long)k * perm[j]]);
         }
       } else {  // theta^H = W S V^H  =>  theta = V[:, perm] S W^H
-        for (int t = tid; t < m * keep; t += blockDim.x) {
+        for (int t = M.tid; t < m * keep; t += M.nt) {
           const int row = t % m, j = t / m;
           T.sl[t] = V[row + (long)k * perm[j]];
         }
-        for (int t = tid; t < keep * nn; t += blockDim.x) {
+        for (int t = M.tid; t < keep * nn; t += M.nt) {
           const int j = t % keep, col = t / keep;
           T.sr[t] = cconj(W[col + (long)rows * j]);
         }
       }
-      for (int j = tid; j < keep; j += blockDim.x) T.lam[j] = srt[j] * scale_f;
-      if (tid == 0) {
+      for (int j = M.tid; j < keep; j += M.nt) T.lam[j] = srt[j] * scale_f;
+      if (M.tid == 0) {
         T.bd[b] = keep;
         T.haslam[b] = 1;
       }
     }
-    __syncthreads();
+    M.sync();
   }
 }
 
@@ -650,9 +833,30 @@ struct BReq {
   std::vector<int> layer_of_gate;
 };
 
+// CTAs per gate step of theta with k columns: as many as have work in a round.  A round of the sweeps has
+// k / 2 pairs (a warp each, at least 4 warps a CTA) and one of the FP32 sweeps k / 16 items.
+int team_size(int k) { return k > 64 ? BT_MAXTEAM : k > 16 ? 4 : 1; }
+
 // Autotuner cache: (device name, chi class) -> warps per CTA of the layer kernel
 std::mutex g_tune_mu;
 std::map<std::string, int> g_tune;
+
+// CTAs per gate step of each layer, from the largest theta that its bonds can have reached
+std::vector<int> layer_teams(const std::vector<BReq>& reqs, int nlayers) {
+  std::vector<int> k(nlayers, 1);
+  for (const BReq& r : reqs) {
+    std::vector<int> ub(r.n - 1, 1);  // bounds of the bond dimensions after the gates so far
+    for (size_t g = 0; g < r.gsite.size(); g++) {
+      const int b = r.gsite[g], m = 2 * (b > 0 ? ub[b - 1] : 1), n = 2 * (b + 1 < r.n - 1 ? ub[b + 1] : 1);
+      int& kl = k[r.layer_of_gate[g]];
+      kl = std::max(kl, std::min(m, n));
+      ub[b] = std::min(std::min(m, n), cap_of(r.n, b, r.chi_max));
+    }
+  }
+  std::vector<int> team(nlayers);
+  for (int L = 0; L < nlayers; L++) team[L] = team_size(k[L]);
+  return team;
+}
 
 std::string tune_file() {
   const char* p = getenv("QROCHET_TUNE_FILE");
@@ -722,7 +926,7 @@ int autotune(qr_batch* bt, cudaStream_t s, int chi, int slots, double2* ws) {
     }
   }
   // synthetic chain of 3 bonds at chi on both sides of the middle one
-  const int ntask = std::max(1, std::min(slots, 2 * 152));
+  const int team = team_size(2 * chi), ntask = std::max(1, std::min(slots, 2 * 152 / team));
   const size_t site = (size_t)chi * 2 * chi;
   double2* sites = nullptr;
   double* lam = nullptr;
@@ -761,10 +965,10 @@ int autotune(qr_batch* bt, cudaStream_t s, int chi, int slots, double2* ws) {
   bt->tune_candidates_ms.clear();
   for (int w : cand) {
     auto kern = mixed ? batch_gate_k<true> : batch_gate_k<false>;
-    kern<<<ntask, 32 * w, 0, s>>>(dt, ntask, ws, 1);  // warm-up
+    QR_CUDA(launch_cluster(kern, ntask, team, 32 * w, s, dt, ntask, ws, 1, team));  // warm-up
     count_launch();
     QR_CUDA(cudaEventRecord(e0, s));
-    kern<<<ntask, 32 * w, 0, s>>>(dt, ntask, ws, 1);
+    QR_CUDA(launch_cluster(kern, ntask, team, 32 * w, s, dt, ntask, ws, 1, team));
     count_launch();
     QR_CUDA(cudaEventRecord(e1, s));
     QR_CUDA(cudaEventSynchronize(e1));
@@ -929,10 +1133,10 @@ int qr_batch_run(qr_batch* bt, double* ms) try {
   const size_t o_tasks = take(sizeof(BTask) * std::max<size_t>(1, ntask_total));
   const size_t o_obs = take(sizeof(BObs) * std::max(1, nobs_total));
   const size_t o_sites_tab = take(sizeof(double2*) * nsites_total);
-  int sms = 0, per_sm = 0;
+  int sms = 0;
   QR_TRY(device_sm_count(&sms));
-  // workspace slots: enough CTAs to fill the GPU with the largest candidate CTA
-  const int slots = sms * 4;
+  // workspace slots, one per CTA or cluster: enough to fill the GPU
+  const int slots = sms * 2;
   const size_t o_ws = take(sizeof(double2) * BT_SLOT * slots);
   const size_t o_ews = take(sizeof(double2) * 2 * BT_MAXCHI * BT_MAXCHI * std::max(1, nobs_total));
   char* base = nullptr;
@@ -1021,8 +1225,7 @@ int qr_batch_run(qr_batch* bt, double* ms) try {
   double2* ws = reinterpret_cast<double2*>(base + o_ws);
   QR_TRY(autotune(bt, s, std::min(maxchi, BT_MAXCHI), slots, ws));
   auto gate_kernel = (bt->precision & QR_MIXED) ? batch_gate_k<true> : batch_gate_k<false>;
-  QR_TRY(blocks_per_sm((const void*)gate_kernel, 32 * bt->warps, 0, &per_sm));
-  const int grid_cap = std::min(slots, std::max(1, per_sm) * sms);
+  const std::vector<int> team = layer_teams(bt->reqs, nlayers);
 
   // ---- one CUDA graph: init, every layer, the expectation sweep
   const BTask* dtasks = reinterpret_cast<const BTask*>(base + o_tasks);
@@ -1036,7 +1239,8 @@ int qr_batch_run(qr_batch* bt, double* ms) try {
   for (int L = 0; L < nlayers; L++) {
     const int nt = (int)(layer_start[L + 1] - layer_start[L]);
     if (nt == 0) continue;
-    gate_kernel<<<std::min(nt, grid_cap), 32 * bt->warps, 0, s>>>(dtasks + layer_start[L], nt, ws, 0);
+    QR_CUDA(launch_cluster(gate_kernel, std::min(nt, slots), team[L], 32 * bt->warps, s, dtasks + layer_start[L], nt, ws,
+                           0, team[L]));
     launches++;
   }
   if (!obs.empty()) {

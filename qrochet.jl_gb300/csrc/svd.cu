@@ -28,6 +28,7 @@
 #include "jacobi_df.cuh"
 #include "prof.cuh"
 #include "jacobi_rot.cuh"
+#include "gram_item.cuh"
 #include "grid_sync.cuh"
 #include <map>
 #include <tuple>
@@ -1615,7 +1616,7 @@ int jacobi(cudaStream_t s, SvdWork* w, cplx_t<T>* B, long ldb, int rows, int k, 
     const int nbk = (k + bw - 1) / bw;
     const int npairs = blk ? (nbk + (nbk & 1)) / 2 : (np / 2 > 0 ? np / 2 : 1);
     const int cl = npairs < 16 ? npairs : 16;
-    const int wpc = blk ? JC_NT / 32 : std::min(4, (npairs + cl - 1) / cl);  // warps loop over pairs
+    const int wpc = blk ? GC_NT / 32 : std::min(4, (npairs + cl - 1) / cl);  // warps loop over pairs
     if (cl > 8) {
       const void* f = blk ? (const void*)jacobi_gram_cluster_k<bw> : (const void*)jacobi_cluster_k<T>;
       QR_TRY(set_func_attr_once(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -1634,7 +1635,7 @@ int jacobi(cudaStream_t s, SvdWork* w, cplx_t<T>* B, long ldb, int rows, int k, 
     cfg.numAttrs = 1;
     svd_path(blk ? SP_BLOCK_CLUSTER : SP_CLUSTER);
     if (blk) {
-      cfg.dynamicSmemBytes = gr_smem<bw, JC_NT>();
+      cfg.dynamicSmemBytes = gr_smem<bw, GC_NT, true>();
       QR_CUDA(cudaLaunchKernelEx(&cfg, jacobi_gram_cluster_k<bw>, (float2*)B, ldb, rows, k, (float2*)V, ldv, (float)tol,
                                  (const double*)smax_d, max_sweeps, state, tan_stop));
     } else {
