@@ -27,6 +27,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cmath>
+#include <cstring>
 #include <algorithm>
 #include "kernels.cuh"
 #include "jacobi_rot.cuh"
@@ -39,8 +40,9 @@ namespace {
 constexpr int BT_MAXK = 128;         // largest theta side: chi_max <= 64
 constexpr int BT_MAXCHI = BT_MAXK / 2;
 constexpr int BT_MAX_SWEEPS = 60;
-// per cluster: six squares, a column of coefficients, one of norms and the sweep counters (double2)
-constexpr size_t BT_SLOT = 6 * (size_t)BT_MAXK * BT_MAXK + 2 * BT_MAXK;
+// workspace of a gate step of theta up to side x side: six squares, a column of coefficients, one of norms and
+// the sweep counters (double2)
+constexpr size_t slot_size(int side) { return 6 * (size_t)side * side + 2 * BT_MAXK; }
 constexpr int BT_PRE_MIN = 16;   // the SVD sweeps in FP32 first above this many columns
 constexpr int BT_MIXED_MIN = 32;  // with QR_MIXED, the finish is in double-float above this many columns
 constexpr int BT_MAXTEAM = 8;    // CTAs per gate step
@@ -431,7 +433,7 @@ __device__ void team_orthonormalise(const Team& T, double2* W, int rows, int kee
   }
 }
 
-// One cluster per task (strided over the layer's tasks).  ws: BT_SLOT double2 per cluster.  dry = 1 runs
+// One cluster per task (strided over the layer's tasks).  ws: slot_size(side) double2 per cluster.  dry = 1 runs
 // the arithmetic without writing the chain (the autotuner's timing runs).
 //
 // Above BT_PRE_MIN columns the SVD first runs FP32 sweeps on a copy of theta (64x the FP64 rate on
@@ -445,7 +447,7 @@ __device__ void team_orthonormalise(const Team& T, double2* W, int rows, int kee
 // the FP32 sweeps run 15 rounds a sweep on Gram matrices.
 template <bool MIXED>
 __global__ void __launch_bounds__(512, 1)
-    batch_gate_k(const BTask* __restrict__ tasks, int ntasks, double2* __restrict__ ws, int dry, int team) {
+    batch_gate_k(const BTask* __restrict__ tasks, int ntasks, double2* __restrict__ ws, int side, int dry, int team) {
   __shared__ BTask T;
   __shared__ double2 G[16];
   __shared__ double sig[BT_MAXK], srt[BT_MAXK];
@@ -463,9 +465,9 @@ __global__ void __launch_bounds__(512, 1)
   M.warp = M.tid >> 5;
   M.nw = M.nt >> 5;
   const int tid = threadIdx.x;
-  constexpr size_t K2 = (size_t)BT_MAXK * BT_MAXK;
+  const size_t K2 = (size_t)side * side;
   // the slot: theta | V | W | three work squares | norms, coefficients, counters
-  double2* TH = ws + (size_t)(blockIdx.x / team) * BT_SLOT;
+  double2* TH = ws + (size_t)(blockIdx.x / team) * (6 * K2 + 2 * BT_MAXK);
   double2 *Vv = TH + K2, *W = Vv + K2, *S0 = W + K2, *S1 = S0 + K2, *S2 = S1 + K2;
   double2* coef = S2 + K2;
   double* nrm = reinterpret_cast<double*>(coef + BT_MAXK);
@@ -833,7 +835,7 @@ struct BReq {
   std::vector<int> layer_of_gate;
 };
 
-// CTAs per gate step of theta with k columns: as many as have work in a round.  A round of the sweeps has
+// CTAs per gate step of theta up to k x k: as many as have work in a round.  A round of the sweeps has
 // k / 2 pairs (a warp each, at least 4 warps a CTA) and one of the FP32 sweeps k / 16 items.
 int team_size(int k) { return k > 64 ? BT_MAXTEAM : k > 16 ? 4 : 1; }
 
@@ -841,21 +843,31 @@ int team_size(int k) { return k > 64 ? BT_MAXTEAM : k > 16 ? 4 : 1; }
 std::mutex g_tune_mu;
 std::map<std::string, int> g_tune;
 
-// CTAs per gate step of each layer, from the largest theta that its bonds can have reached
-std::vector<int> layer_teams(const std::vector<BReq>& reqs, int nlayers) {
-  std::vector<int> k(nlayers, 1);
+// The launch of a layer: the largest theta that its bonds can have reached, CTAs per gate step and clusters.  Four
+// CTAs of 128 threads a SM fill the GPU; more clusters would only want more workspace.
+struct Layer {
+  int side = 2, team = 1, clusters = 1;
+  size_t ws() const { return slot_size(side) * clusters; }
+};
+void size_layer(Layer& l, int ntasks, int sms) {
+  l.team = team_size(l.side);
+  l.clusters = std::max(1, std::min(ntasks, 4 * sms / l.team));
+}
+std::vector<Layer> plan_layers(const std::vector<BReq>& reqs, int nlayers, int sms) {
+  std::vector<Layer> out(nlayers);
+  std::vector<int> ntasks(nlayers, 0);
   for (const BReq& r : reqs) {
     std::vector<int> ub(r.n - 1, 1);  // bounds of the bond dimensions after the gates so far
     for (size_t g = 0; g < r.gsite.size(); g++) {
       const int b = r.gsite[g], m = 2 * (b > 0 ? ub[b - 1] : 1), n = 2 * (b + 1 < r.n - 1 ? ub[b + 1] : 1);
-      int& kl = k[r.layer_of_gate[g]];
-      kl = std::max(kl, std::min(m, n));
+      Layer& l = out[r.layer_of_gate[g]];
+      l.side = std::max(l.side, std::max(m, n));
+      ntasks[r.layer_of_gate[g]]++;
       ub[b] = std::min(std::min(m, n), cap_of(r.n, b, r.chi_max));
     }
   }
-  std::vector<int> team(nlayers);
-  for (int L = 0; L < nlayers; L++) team[L] = team_size(k[L]);
-  return team;
+  for (int L = 0; L < nlayers; L++) size_layer(out[L], ntasks[L], sms);
+  return out;
 }
 
 std::string tune_file() {
@@ -906,27 +918,30 @@ struct qr_batch {
 };
 
 namespace {
-// warps per CTA for the layer kernel at bond class `chi` (the batch's largest), measured on
-// synthetic gate steps of that class in dry mode (no chain is written)
-int autotune(qr_batch* bt, cudaStream_t s, int chi, int slots, double2* ws) {
+// the tuning cache's key of the batch's largest bond class, and the choice that it holds (0: none yet)
+int tune_key(const qr_batch* bt, int chi, std::string* out) {
   cudaDeviceProp prop;
   QR_CUDA(cudaGetDeviceProperties(&prop, bt->device));
   const bool mixed = (bt->precision & QR_MIXED) != 0;
   std::string key = std::string(prop.name).substr(0, 40) + "/chi" + std::to_string(chi) + (mixed ? "/mixed" : "/fp64");
   for (char& ch : key)
     if (ch == ' ') ch = '_';
-  {
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    tune_load();
-    auto it = g_tune.find(key);
-    if (it != g_tune.end()) {
-      bt->warps = it->second;
-      bt->tuned_from_cache = 1;
-      return QR_OK;
-    }
-  }
+  *out = key;
+  return QR_OK;
+}
+int tuned_warps(const std::string& key) {
+  std::lock_guard<std::mutex> lk(g_tune_mu);
+  tune_load();
+  auto it = g_tune.find(key);
+  return it != g_tune.end() ? it->second : 0;
+}
+
+// warps per CTA for the layer kernel at bond class `chi` (the batch's largest), measured on
+// synthetic gate steps of that class in dry mode (no chain is written)
+int autotune(qr_batch* bt, cudaStream_t s, const std::string& key, int chi, const Layer& l, double2* ws) {
+  const bool mixed = (bt->precision & QR_MIXED) != 0;
   // synthetic chain of 3 bonds at chi on both sides of the middle one
-  const int team = team_size(2 * chi), ntask = std::max(1, std::min(slots, 2 * 152 / team));
+  const int ntask = l.clusters;
   const size_t site = (size_t)chi * 2 * chi;
   double2* sites = nullptr;
   double* lam = nullptr;
@@ -965,10 +980,10 @@ int autotune(qr_batch* bt, cudaStream_t s, int chi, int slots, double2* ws) {
   bt->tune_candidates_ms.clear();
   for (int w : cand) {
     auto kern = mixed ? batch_gate_k<true> : batch_gate_k<false>;
-    QR_CUDA(launch_cluster(kern, ntask, team, 32 * w, s, dt, ntask, ws, 1, team));  // warm-up
+    QR_CUDA(launch_cluster(kern, ntask, l.team, 32 * w, s, dt, ntask, ws, l.side, 1, l.team));  // warm-up
     count_launch();
     QR_CUDA(cudaEventRecord(e0, s));
-    QR_CUDA(launch_cluster(kern, ntask, team, 32 * w, s, dt, ntask, ws, 1, team));
+    QR_CUDA(launch_cluster(kern, ntask, l.team, 32 * w, s, dt, ntask, ws, l.side, 1, l.team));
     count_launch();
     QR_CUDA(cudaEventRecord(e1, s));
     QR_CUDA(cudaEventSynchronize(e1));
@@ -1104,18 +1119,33 @@ int qr_batch_run(qr_batch* bt, double* ms) try {
       o.site[i] = take(sizeof(double2) * (size_t)cl * 2 * cr);
       maxchi = std::max(maxchi, std::max(cl, cr));
     }
-    for (int b = 0; b < r.n - 1; b++) o.lam[b] = take(sizeof(double) * cap_of(r.n, b, r.chi_max));
-    o.bd = take(sizeof(int) * (r.n - 1));
-    o.hl = take(sizeof(int) * (r.n - 1));
-    o.sp = take(sizeof(double2*) * r.n);
-    o.lp = take(sizeof(double*) * (r.n - 1));
-    o.gates = take(sizeof(double2) * std::max<size_t>(1, r.gmat.size()));
-    o.paulis = take(sizeof(int) * (size_t)r.n * std::max<size_t>(1, r.ow.size()));
-    o.out = take(sizeof(double2) * std::max<size_t>(1, r.ow.size()));
-    o.status = take(sizeof(int));
     nsites_total += r.n;
     nobs_total += (int)r.ow.size();
     for (int L : r.layer_of_gate) nlayers = std::max(nlayers, L + 1);
+  }
+  // The tables are one block, [Lambda | values | bonds, flags, status | pointers, gates, strings, tasks]: the
+  // start of its third part is uploaded with one copy, and its first three parts come back with one.  (A copy
+  // per array took 9 ms of host time at 32 requests.)
+  const size_t o_results = off;
+  for (int q = 0; q < R; q++) {
+    const BReq& r = bt->reqs[q];
+    for (int b = 0; b < r.n - 1; b++) ro[q].lam[b] = take(sizeof(double) * cap_of(r.n, b, r.chi_max));
+    ro[q].out = take(sizeof(double2) * std::max<size_t>(1, r.ow.size()));
+  }
+  const size_t o_image = off;
+  for (int q = 0; q < R; q++) {
+    const BReq& r = bt->reqs[q];
+    ro[q].bd = take(sizeof(int) * (r.n - 1));
+    ro[q].hl = take(sizeof(int) * (r.n - 1));
+    ro[q].status = take(sizeof(int));
+  }
+  const size_t o_results_end = off;
+  for (int q = 0; q < R; q++) {
+    const BReq& r = bt->reqs[q];
+    ro[q].sp = take(sizeof(double2*) * r.n);
+    ro[q].lp = take(sizeof(double*) * (r.n - 1));
+    ro[q].gates = take(sizeof(double2) * std::max<size_t>(1, r.gmat.size()));
+    ro[q].paulis = take(sizeof(int) * (size_t)r.n * std::max<size_t>(1, r.ow.size()));
   }
   // per-layer task tables, larger bond classes first inside a layer
   std::vector<std::vector<std::pair<int, int>>> layer_tasks(nlayers);  // (request, gate)
@@ -1135,10 +1165,21 @@ int qr_batch_run(qr_batch* bt, double* ms) try {
   const size_t o_sites_tab = take(sizeof(double2*) * nsites_total);
   int sms = 0;
   QR_TRY(device_sm_count(&sms));
-  // workspace slots, one per CTA or cluster: enough to fill the GPU
-  const int slots = sms * 2;
-  const size_t o_ws = take(sizeof(double2) * BT_SLOT * slots);
+  const size_t o_image_end = off;
+  const std::vector<Layer> layers = plan_layers(bt->reqs, nlayers, sms);
+  const int tune_chi = std::min(maxchi, BT_MAXCHI);
+  std::string key;
+  QR_TRY(tune_key(bt, tune_chi, &key));
+  bt->warps = tuned_warps(key);
+  bt->tuned_from_cache = bt->warps != 0;
+  Layer tune_layer;
+  tune_layer.side = 2 * tune_chi;
+  size_layer(tune_layer, 4 * sms, sms);
+  size_t ws_words = bt->warps ? 0 : tune_layer.ws();
+  for (const Layer& l : layers) ws_words = std::max(ws_words, l.ws());
+  const size_t o_ws = take(sizeof(double2) * ws_words);
   const size_t o_ews = take(sizeof(double2) * 2 * BT_MAXCHI * BT_MAXCHI * std::max(1, nobs_total));
+  std::vector<char> image(o_image_end - o_image, 0), results(o_results_end - o_results);  // (outlive the copies)
   char* base = nullptr;
   {
     cudaError_t e = cudaMallocAsync((void**)&base, off, s);
@@ -1150,7 +1191,8 @@ int qr_batch_run(qr_batch* bt, double* ms) try {
     ~MemGuard() { cudaFreeAsync(p, s); cudaStreamSynchronize(s); }
   } mg{base, s};
 
-  // ---- host images of the tables
+  // ---- host image of the tables
+  auto put = [&](size_t at, const void* src, size_t bytes) { memcpy(image.data() + (at - o_image), src, bytes); };
   std::vector<BTask> tasks;
   tasks.reserve(ntask_total);
   std::vector<size_t> layer_start(nlayers + 1, 0);
@@ -1186,13 +1228,13 @@ int qr_batch_run(qr_batch* bt, double* ms) try {
     std::vector<double*> lp(r.n - 1);
     for (int i = 0; i < r.n; i++) sp[i] = reinterpret_cast<double2*>(base + o.site[i]), sites_tab.push_back(sp[i]);
     for (int b = 0; b < r.n - 1; b++) lp[b] = reinterpret_cast<double*>(base + o.lam[b]);
-    std::vector<int> zeros(r.n - 1, 0), ones(r.n - 1, 1);
-    QR_CUDA(cudaMemcpyAsync(base + o.bd, ones.data(), sizeof(int) * (r.n - 1), cudaMemcpyHostToDevice, s));
-    QR_CUDA(cudaMemcpyAsync(base + o.hl, zeros.data(), sizeof(int) * (r.n - 1), cudaMemcpyHostToDevice, s));
-    QR_CUDA(cudaMemcpyAsync(base + o.sp, sp.data(), sizeof(double2*) * r.n, cudaMemcpyHostToDevice, s));
-    QR_CUDA(cudaMemcpyAsync(base + o.lp, lp.data(), sizeof(double*) * (r.n - 1), cudaMemcpyHostToDevice, s));
-    if (!r.gmat.empty())
-      QR_CUDA(cudaMemcpyAsync(base + o.gates, r.gmat.data(), sizeof(double2) * r.gmat.size(), cudaMemcpyHostToDevice, s));
+    const std::vector<int> ones(r.n - 1, 1);
+    const int ok = QR_OK;
+    put(o.bd, ones.data(), sizeof(int) * (r.n - 1));  // (Lambda flags: zero)
+    put(o.status, &ok, sizeof(int));
+    put(o.sp, sp.data(), sizeof(double2*) * r.n);
+    put(o.lp, lp.data(), sizeof(double*) * (r.n - 1));
+    if (!r.gmat.empty()) put(o.gates, r.gmat.data(), sizeof(double2) * r.gmat.size());
     std::vector<int> pc((size_t)r.n * std::max<size_t>(1, r.ow.size()), 0);
     int pos = 0;
     for (size_t j = 0; j < r.ow.size(); j++) {
@@ -1211,21 +1253,16 @@ int qr_batch_run(qr_batch* bt, double* ms) try {
       b.pad = 0;
       obs.push_back(b);
     }
-    QR_CUDA(cudaMemcpyAsync(base + o.paulis, pc.data(), sizeof(int) * pc.size(), cudaMemcpyHostToDevice, s));
-    const int ok = QR_OK;
-    QR_CUDA(cudaMemcpyAsync(base + o.status, &ok, sizeof(int), cudaMemcpyHostToDevice, s));
+    put(o.paulis, pc.data(), sizeof(int) * pc.size());
   }
-  if (!tasks.empty())
-    QR_CUDA(cudaMemcpyAsync(base + o_tasks, tasks.data(), sizeof(BTask) * tasks.size(), cudaMemcpyHostToDevice, s));
-  if (!obs.empty()) QR_CUDA(cudaMemcpyAsync(base + o_obs, obs.data(), sizeof(BObs) * obs.size(), cudaMemcpyHostToDevice, s));
-  QR_CUDA(cudaMemcpyAsync(base + o_sites_tab, sites_tab.data(), sizeof(double2*) * sites_tab.size(),
-                          cudaMemcpyHostToDevice, s));
-  QR_CUDA(cudaStreamSynchronize(s));  // the pageable host images above must be consumed
+  if (!tasks.empty()) put(o_tasks, tasks.data(), sizeof(BTask) * tasks.size());
+  if (!obs.empty()) put(o_obs, obs.data(), sizeof(BObs) * obs.size());
+  put(o_sites_tab, sites_tab.data(), sizeof(double2*) * sites_tab.size());
+  QR_CUDA(cudaMemcpyAsync(base + o_image, image.data(), image.size(), cudaMemcpyHostToDevice, s));
 
   double2* ws = reinterpret_cast<double2*>(base + o_ws);
-  QR_TRY(autotune(bt, s, std::min(maxchi, BT_MAXCHI), slots, ws));
+  if (!bt->warps) QR_TRY(autotune(bt, s, key, tune_chi, tune_layer, ws));
   auto gate_kernel = (bt->precision & QR_MIXED) ? batch_gate_k<true> : batch_gate_k<false>;
-  const std::vector<int> team = layer_teams(bt->reqs, nlayers);
 
   // ---- one CUDA graph: init, every layer, the expectation sweep
   const BTask* dtasks = reinterpret_cast<const BTask*>(base + o_tasks);
@@ -1239,8 +1276,9 @@ int qr_batch_run(qr_batch* bt, double* ms) try {
   for (int L = 0; L < nlayers; L++) {
     const int nt = (int)(layer_start[L + 1] - layer_start[L]);
     if (nt == 0) continue;
-    QR_CUDA(launch_cluster(gate_kernel, std::min(nt, slots), team[L], 32 * bt->warps, s, dtasks + layer_start[L], nt, ws,
-                           0, team[L]));
+    const Layer& l = layers[L];
+    QR_CUDA(launch_cluster(gate_kernel, l.clusters, l.team, 32 * bt->warps, s, dtasks + layer_start[L], nt, ws, l.side, 0,
+                           l.team));
     launches++;
   }
   if (!obs.empty()) {
@@ -1281,22 +1319,24 @@ int qr_batch_run(qr_batch* bt, double* ms) try {
   if (ms) *ms = gms;
 
   // ---- results
+  QR_CUDA(cudaMemcpyAsync(results.data(), base + o_results, results.size(), cudaMemcpyDeviceToHost, s));
+  QR_CUDA(cudaStreamSynchronize(s));
+  auto get = [&](size_t at, void* dst, size_t bytes) { memcpy(dst, results.data() + (at - o_results), bytes); };
   for (int q = 0; q < R; q++) {
     BReq& r = bt->reqs[q];
     const ROff& o = ro[q];
-    QR_CUDA(cudaMemcpy(&r.status, base + o.status, sizeof(int), cudaMemcpyDeviceToHost));
+    get(o.status, &r.status, sizeof(int));
     r.values.resize(r.ow.size());
-    if (!r.ow.empty())
-      QR_CUDA(cudaMemcpy(r.values.data(), base + o.out, sizeof(double2) * r.ow.size(), cudaMemcpyDeviceToHost));
+    if (!r.ow.empty()) get(o.out, r.values.data(), sizeof(double2) * r.ow.size());
     r.bd.resize(r.n - 1);
-    QR_CUDA(cudaMemcpy(r.bd.data(), base + o.bd, sizeof(int) * (r.n - 1), cudaMemcpyDeviceToHost));
+    get(o.bd, r.bd.data(), sizeof(int) * (r.n - 1));
     std::vector<int> hl(r.n - 1);
-    QR_CUDA(cudaMemcpy(hl.data(), base + o.hl, sizeof(int) * (r.n - 1), cudaMemcpyDeviceToHost));
+    get(o.hl, hl.data(), sizeof(int) * (r.n - 1));
     r.lam.assign(r.n - 1, {});
     for (int b = 0; b < r.n - 1; b++) {
       if (!hl[b]) continue;
       r.lam[b].resize(r.bd[b]);
-      QR_CUDA(cudaMemcpy(r.lam[b].data(), base + o.lam[b], sizeof(double) * r.bd[b], cudaMemcpyDeviceToHost));
+      get(o.lam[b], r.lam[b].data(), sizeof(double) * r.bd[b]);
     }
   }
   bt->ran = true;
