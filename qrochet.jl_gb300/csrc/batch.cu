@@ -30,9 +30,8 @@
 #include <cstring>
 #include <algorithm>
 #include "kernels.cuh"
-#include "jacobi_rot.cuh"
 #include "jacobi_df.cuh"
-#include "gram_item.cuh"
+#include "team_svd.cuh"
 
 namespace qr {
 namespace {
@@ -40,11 +39,11 @@ namespace {
 constexpr int BT_MAXK = 128;         // largest theta side: chi_max <= 64
 constexpr int BT_MAXCHI = BT_MAXK / 2;
 constexpr int BT_MAX_SWEEPS = 60;
-// workspace of a gate step of theta up to side x side: six squares, a column of coefficients, one of norms and
-// the sweep counters (double2)
-constexpr size_t slot_size(int side) { return 6 * (size_t)side * side + 2 * BT_MAXK; }
+// workspace of a gate step of theta up to side x side (double2): theta, B, V and the kept vectors, the SVD's
+// own, a column of coefficients and one of norms
+constexpr size_t slot_size(int side) { return 4 * (size_t)side * side + team_ws(side) + 2 * BT_MAXK; }
 constexpr int BT_PRE_MIN = 16;   // the SVD sweeps in FP32 first above this many columns
-constexpr int BT_MIXED_MIN = 32;  // with QR_MIXED, the finish is in double-float above this many columns
+constexpr int BT_TEAM_MAX = 32;  // and its FP64 refinement by products pays up to this many
 constexpr int BT_MAXTEAM = 8;    // CTAs per gate step
 
 __device__ __forceinline__ void cfma(double2& acc, double2 a, double2 b) {
@@ -75,111 +74,6 @@ struct BObs {
 };
 
 // ---- the fused gate step ------------------------------------------------------------------------
-// One cluster of 1 to 8 CTAs runs one gate step; every phase is dealt to the cluster's threads or
-// warps, and the data goes through L2.  `Team` is this thread's place in it.
-struct Team {
-  int size, rank;       // CTAs, this CTA
-  int tid, nt;          // thread of the cluster, its threads
-  int lane, warp, nw;   // warp of the cluster, its warps
-  __device__ __forceinline__ void sync() const {
-    if (size == 1) {
-      __syncthreads();
-    } else {
-      __syncwarp();
-      cluster_sync_all();
-    }
-  }
-};
-
-// Rotations and largest tangent of a sweep, counted by the whole team: sweep s uses slot s % 3 and clears
-// the next one, which was last read two barriers ago.
-struct SweepCount {
-  unsigned* c;  // 3 x 2 words in global memory
-  __device__ __forceinline__ void start(const Team& T) const {
-    if (T.tid == 0) { __stcg(c, 0u); __stcg(c + 1, 0u); }
-  }
-  __device__ __forceinline__ unsigned* open(const Team& T, int sweep) const {
-    unsigned* nx = c + 2 * ((sweep + 1) % 3);
-    if (T.tid == 0) { __stcg(nx, 0u); __stcg(nx + 1, 0u); }
-    return c + 2 * (sweep % 3);
-  }
-  static __device__ __forceinline__ void add(unsigned* s, float tabs) {
-    atomicAdd(s, 1u);
-    atomicMax(s + 1, __float_as_uint(tabs));
-  }
-  static __device__ __forceinline__ bool done(const unsigned* s, float tan_stop) {
-    return __ldcg(s) == 0u || __uint_as_float(__ldcg(s + 1)) < tan_stop;
-  }
-};
-
-// pair `pair` of round `round` over np (even) columns, p < q
-__device__ __forceinline__ void round_pair(int np, int round, int pair, int& p, int& q) {
-  if (pair == 0) { p = round; q = np - 1; }
-  else { p = (round + pair) % (np - 1); q = (round - pair + np - 1) % (np - 1); }
-  if (p > q) { const int x = p; p = q; q = x; }
-}
-
-constexpr int BT_RPL = BT_MAXK / 32;  // rows a lane
-
-// FP64 Hestenes sweeps of the team on B (rows x k, ld rows) accumulating V (k x k, ld k): round-robin pairs,
-// one warp per pair with the columns' rows in registers, a team barrier between rounds.  Stops after a sweep
-// that rotates nothing or whose largest rotation tangent is below tan_stop; returns that verdict.
-__device__ bool team_sweeps(const Team& T, double2* B, double2* V, int rows, int k, double tol, double smax,
-                            int max_sweeps, float tan_stop, SweepCount cnt) {
-  const int np = k + (k & 1), npairs = np / 2;
-  bool converged = false;
-  cnt.start(T);
-  T.sync();
-  for (int sweep = 0; sweep < max_sweeps && !converged; sweep++) {
-    unsigned* sc = cnt.open(T, sweep);
-    for (int round = 0; round < np - 1; round++) {
-      for (int pair = T.warp; pair < npairs; pair += T.nw) {
-        int p, q;
-        round_pair(np, round, pair, p, q);
-        if (q >= k) continue;
-        double2 *bp = B + (long)rows * p, *bq = B + (long)rows * q, *vp = V + (long)k * p, *vq = V + (long)k * q;
-        double2 x[BT_RPL], y[BT_RPL], u[BT_RPL], w[BT_RPL];
-        double a = 0, bb = 0, gr = 0, gi = 0;
-#pragma unroll
-        for (int j = 0; j < BT_RPL; j++) {
-          const int r = T.lane + 32 * j;
-          x[j] = y[j] = u[j] = w[j] = make_double2(0.0, 0.0);
-          if (r < rows) { x[j] = __ldcg(bp + r); y[j] = __ldcg(bq + r); }
-          if (r < k) { u[j] = __ldcg(vp + r); w[j] = __ldcg(vq + r); }
-        }
-#pragma unroll
-        for (int j = 0; j < BT_RPL; j++) {
-          if (32 * j >= rows) break;  // no arithmetic on rows that no lane has
-          a += x[j].x * x[j].x + x[j].y * x[j].y;
-          bb += y[j].x * y[j].x + y[j].y * y[j].y;
-          gr += x[j].x * y[j].x + x[j].y * y[j].y;
-          gi += x[j].x * y[j].y - x[j].y * y[j].x;
-        }
-        a = warp_sum(a); bb = warp_sum(bb); gr = warp_sum(gr); gi = warp_sum(gi);
-        double c, sr, si;
-        float tabs;
-        if (!rotation_params<double>(a, bb, gr, gi, tol, smax, c, sr, si, tabs)) continue;
-#pragma unroll
-        for (int j = 0; j < BT_RPL; j++) {
-          const int r = T.lane + 32 * j;
-          if (32 * j < rows) {
-            rot(x[j], y[j], c, sr, si);
-            if (r < rows) { __stcg(bp + r, x[j]); __stcg(bq + r, y[j]); }
-          }
-          if (32 * j < k) {
-            rot(u[j], w[j], c, sr, si);
-            if (r < k) { __stcg(vp + r, u[j]); __stcg(vq + r, w[j]); }
-          }
-        }
-        if (T.lane == 0) SweepCount::add(sc, tabs);
-      }
-      T.sync();
-    }
-    converged = SweepCount::done(sc, tan_stop);
-  }
-  return converged;
-}
-
 // The mixed finish: the same sweeps in double-float (FP32 pairs, on the FP32 pipes) on B (Bh, Bl: rows x k,
 // ld rows) accumulating V (Vh, Vl: k x k, ld k).  Every lane forms the pair's compensated sums over its rows,
 // the warp reduces them, and every lane derives the same rotation from the broadcast sums.
@@ -197,9 +91,9 @@ __device__ bool team_sweeps_df(const Team& T, float2* Bh, float2* Bl, float2* Vh
         round_pair(np, round, pair, p, q);
         if (q >= k) continue;
         const long cp = (long)rows * p, cq = (long)rows * q, dp = (long)k * p, dq = (long)k * q;
-        float2 xh[BT_RPL], xl[BT_RPL], yh[BT_RPL], yl[BT_RPL], uh[BT_RPL], ul[BT_RPL], wh[BT_RPL], wl[BT_RPL];
+        float2 xh[TM_RPL], xl[TM_RPL], yh[TM_RPL], yl[TM_RPL], uh[TM_RPL], ul[TM_RPL], wh[TM_RPL], wl[TM_RPL];
 #pragma unroll
-        for (int j = 0; j < BT_RPL; j++) {
+        for (int j = 0; j < TM_RPL; j++) {
           const int r = T.lane + 32 * j;
           xh[j] = xl[j] = yh[j] = yl[j] = uh[j] = ul[j] = wh[j] = wl[j] = make_float2(0.f, 0.f);
           if (r < rows) {
@@ -213,7 +107,7 @@ __device__ bool team_sweeps_df(const Team& T, float2* Bh, float2* Bl, float2* Vh
         }
         DotAcc a{0.f, 0.f}, b{0.f, 0.f}, gr{0.f, 0.f}, gi{0.f, 0.f};
 #pragma unroll
-        for (int j = 0; j < BT_RPL; j++) {
+        for (int j = 0; j < TM_RPL; j++) {
           if (32 * j >= rows) break;
           df_dot_acc(xh[j], xl[j], yh[j], yl[j], a, b, gr, gi);
         }
@@ -222,7 +116,7 @@ __device__ bool team_sweeps_df(const Team& T, float2* Bh, float2* Bl, float2* Vh
         if (!rotation_params_df(df_shfl(k4, 0), df_shfl(k4, 8), df_shfl(k4, 16), df_shfl(k4, 24), tol, smax, P))
           continue;
 #pragma unroll
-        for (int j = 0; j < BT_RPL; j++) {
+        for (int j = 0; j < TM_RPL; j++) {
           const int r = T.lane + 32 * j;
           if (r < rows) {
             df_rot_any(xh[j], xl[j], yh[j], yl[j], P);
@@ -241,37 +135,8 @@ __device__ bool team_sweeps_df(const Team& T, float2* Bh, float2* Bl, float2* Vh
     }
     converged = SweepCount::done(sc, tan_stop);
   }
+  T.sync();  // the counters have been read
   return converged;
-}
-
-// FP32 sweeps on Gram matrices of block pairs (gram_item.cuh), an item a CTA; up to BT_MAXK rows.
-constexpr int BT_W = 8;
-constexpr size_t BT_TILE = gr_smem<BT_W, BT_MAXK>() / sizeof(float2);
-__device__ void team_sweeps_f32(const Team& T, float2* B, float2* V, int rows, int k, float tol, float smax,
-                                int max_sweeps, float tan_stop, SweepCount cnt, GrShared<BT_W>& sh, float2* tile) {
-  const int nb = (k + BT_W - 1) / BT_W, nbp = nb + (nb & 1), npairs = nbp / 2;
-  bool converged = false;
-  cnt.start(T);
-  T.sync();
-  for (int sweep = 0; sweep < max_sweeps && !converged; sweep++) {
-    unsigned* sc = cnt.open(T, sweep);
-    for (int round = 0; round < nbp - 1; round++) {
-      for (int pair = T.rank; pair < npairs; pair += T.size) {
-        int bp, bq;
-        round_pair(nbp, round, pair, bp, bq);
-        if (bq < nb || round == 0) {
-          if (blockDim.x == BT_MAXK)
-            gr_item<BT_W, BT_MAXK>(B, rows, rows, k, V, k, nb, bp, bq, round == 0, tol, smax, sc, sh, tile, 0, 0, 1);
-          else if (threadIdx.x < 2 * BT_MAXK)
-            gr_item<BT_W, 2 * BT_MAXK, true>(B, rows, rows, k, V, k, nb, bp, bq, round == 0, tol, smax, sc, sh, tile, 0,
-                                             0, 1);
-        }
-        __syncthreads();  // shared state is reused by the next item
-      }
-      T.sync();
-    }
-    converged = SweepCount::done(sc, tan_stop);
-  }
 }
 
 // R = I - X^H X from X's transpose Xt (k x k, ld k), half of it computed: lanes on consecutive columns of X,
@@ -373,22 +238,6 @@ __device__ void team_gemm(const Team& T, const double2* A, int rows, const doubl
   }
 }
 
-// column norms of B (rows x k, ld rows) into nrm (global), and into every CTA's sig after the barrier
-__device__ void team_norms(const Team& T, const double2* B, int rows, int k, double* nrm, double* sig) {
-  for (int j = T.warp; j < k; j += T.nw) {
-    double s = 0.0;
-    for (int r = T.lane; r < rows; r += 32) {
-      const double2 v = B[r + (long)rows * j];
-      s += v.x * v.x + v.y * v.y;
-    }
-    s = warp_sum(s);
-    if (T.lane == 0) __stcg(nrm + j, sqrt(s));
-  }
-  T.sync();
-  for (int j = threadIdx.x; j < k; j += blockDim.x) sig[j] = __ldcg(nrm + j);
-  __syncthreads();
-}
-
 // W's first `keep` columns (rows x keep, ld rows, nearly unit) made orthonormal, each column's direction and
 // phase kept: classical Gram-Schmidt twice.  A column's updates are dealt out by row, 8 lanes to a row.
 __device__ void team_orthonormalise(const Team& T, double2* W, int rows, int keep, double2* coef) {
@@ -454,8 +303,8 @@ __global__ void __launch_bounds__(512, 1)
   __shared__ int perm[BT_MAXK];
   __shared__ double scale_f, smax_s;
   __shared__ int keep_s, reorth_s;
-  __shared__ GrShared<BT_W> gsh;
-  __shared__ __align__(16) float2 tile[BT_TILE];
+  __shared__ GrShared<TM_W> gsh;
+  __shared__ __align__(16) float2 tile[TM_TILE];
   Team M;
   M.size = team;
   M.rank = blockIdx.x % team;
@@ -466,10 +315,8 @@ __global__ void __launch_bounds__(512, 1)
   M.nw = M.nt >> 5;
   const int tid = threadIdx.x;
   const size_t K2 = (size_t)side * side;
-  // the slot: theta | V | W | three work squares | norms, coefficients, counters
-  double2* TH = ws + (size_t)(blockIdx.x / team) * (6 * K2 + 2 * BT_MAXK);
-  double2 *Vv = TH + K2, *W = Vv + K2, *S0 = W + K2, *S1 = S0 + K2, *S2 = S1 + K2;
-  double2* coef = S2 + K2;
+  double2* TH = ws + (size_t)(blockIdx.x / team) * (4 * K2 + TM_SQUARES * K2 + TM_MAXK + 2 * BT_MAXK);
+  double2 *B = TH + K2, *V = B + K2, *W = V + K2, *coef = W + K2, *S0 = coef + 2 * BT_MAXK, *S1 = S0 + K2, *S2 = S1 + K2;
   double* nrm = reinterpret_cast<double*>(coef + BT_MAXK);
   const SweepCount cnt{reinterpret_cast<unsigned*>(nrm + BT_MAXK)};
 
@@ -483,8 +330,7 @@ __global__ void __launch_bounds__(512, 1)
     const bool tall = m >= nn;
     const int rows = tall ? m : nn, k = tall ? nn : m;
     const bool lam_on = T.haslam[b] != 0;
-    const bool pre = k > BT_PRE_MIN, df = MIXED && k > BT_MIXED_MIN;
-    double2 *B = TH, *V = Vv;  // the sweeps' columns and rotations
+    const bool sweep = k <= BT_PRE_MIN, wide = k > BT_TEAM_MAX;
     __syncthreads();
 
     // ---- theta' = G (A_l diag(Lambda) A_r), into TH (tall) or TH = theta'^H (wide)
@@ -534,30 +380,34 @@ __global__ void __launch_bounds__(512, 1)
     __syncthreads();
     const double smax = smax_s;
     {
-      // (the FP32 sweeps' copies in S0: B32 | V32)
+      // (copies for the FP32 sweeps: B32 | V32)
       const double inv = 1.0 / scale_f;
       float2* B32 = reinterpret_cast<float2*>(S0);
       for (int t = M.tid; t < rows * k; t += M.nt) {
         const double2 v = cscale(TH[t], inv);
-        TH[t] = v;
-        if (pre) B32[t] = make_float2((float)v.x, (float)v.y);
+        (sweep ? B : TH)[t] = v;
+        if (wide) B32[t] = make_float2((float)v.x, (float)v.y);
       }
       for (int t = M.tid; t < k * k; t += M.nt) {
         const bool d = (t % k) == (t / k);
-        if (pre) B32[K2 + t] = make_float2(d ? 1.f : 0.f, 0.f);
-        else V[t] = make_double2(d ? 1.0 : 0.0, 0.0);
+        if (wide) B32[K2 + t] = make_float2(d ? 1.f : 0.f, 0.f);
+        if (sweep) V[t] = make_double2(d ? 1.0 : 0.0, 0.0);
       }
     }
     M.sync();
 
-    // ---- Hestenes sweeps, preconditioned in FP32
+    // ---- B = theta V with orthogonal columns: FP64 sweeps, a refinement, or sweeps preconditioned in FP32
     const double tol = sqrt((double)rows) * Eps<double>::v;
     bool converged = false;
-    if (pre) {
+    if (sweep) {
+      converged = team_sweeps(M, B, V, rows, k, tol, smax, BT_MAX_SWEEPS, 1e-8f, cnt);
+    } else if (!wide) {
+      converged = team_svd(M, TH, B, V, rows, k, tol, smax, S0, side, gsh, tile);
+    } else {
       float2 *B32 = reinterpret_cast<float2*>(S0), *V32 = B32 + K2;
       const float tol32 = fmaxf(4e-6f, 2.f * sqrtf((float)rows) * Eps<float>::v);
       team_sweeps_f32(M, B32, V32, rows, k, tol32, (float)smax, 20, 0.15f, cnt, gsh, tile);
-      if (df) {
+      if (MIXED) {
         // halves of the squares: S0 B32 | X0 -> B' (hi | lo), S1 theta (hi | lo), S2 X0's transpose -> X1's
         // (hi | lo) -> X2 (hi | lo), W X1 (hi | lo), V R | zeros
         float2 *h0 = reinterpret_cast<float2*>(S0), *h1 = reinterpret_cast<float2*>(S1), *h2 = reinterpret_cast<float2*>(S2);
@@ -623,11 +473,12 @@ __global__ void __launch_bounds__(512, 1)
         }
         M.sync();
         team_gemm(M, TH, rows, S1, k, S0);
-        B = S0;
-        V = S1;
+        M.sync();
+        for (int t = M.tid; t < rows * k; t += M.nt) B[t] = S0[t];
+        for (int t = M.tid; t < k * k; t += M.nt) V[t] = S1[t];
+        converged = team_sweeps(M, B, V, rows, k, tol, smax, BT_MAX_SWEEPS, 1e-8f, cnt);
       }
     }
-    if (!df) converged = team_sweeps(M, B, V, rows, k, tol, smax, BT_MAX_SWEEPS, 1e-8f, cnt);
     if (!converged && M.tid == 0) atomicExch(T.status, (int)QR_ENOCONV);
 
     // ---- sigma, descending order (ties by index), truncation on the device

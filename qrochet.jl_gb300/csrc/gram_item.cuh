@@ -41,9 +41,8 @@ struct GrShared {
   float2 part[(W / 2) * (W / 2 + 1) / 2 * 16];       // this CTA's partial Gram matrix, 4 x 4 tiles
   unsigned count, tmax;
 };
-// the tile of B's rows; with SPLIT half of the threads hold rows of V
-template <int W, int NT, bool SPLIT = false>
-constexpr size_t gr_smem() { return sizeof(float2) * (SPLIT ? NT / 2 : NT) * (2 * W + 2); }
+template <int W, int NT>
+constexpr size_t gr_smem() { return sizeof(float2) * NT * (2 * W + 2); }
 
 // Rotation of the pair with squared norms a, b and product g (the test of rotation_params_f32), from the
 // normalised product g / (|x| |y|) so that small columns do not underflow; c and s by fast approximations
@@ -117,16 +116,14 @@ __device__ __forceinline__ void gr_round(float2 (&x)[2 * W], const float4* rot_r
 }
 
 // One work item: blocks bp < bq of nb; this CTA's first NT threads hold rows row0 + tid of B (m rows) and V (n
-// rows).  SPLIT (one CTA per item): the first half of the threads holds rows of B and the other rows of V.
-template <int W, int NT, bool SPLIT = false>
+// rows).
+template <int W, int NT>
 __device__ __forceinline__ void gr_item(float2* __restrict__ B, long ldb, int m, int n, float2* __restrict__ V, long ldv,
                                         int nb, int bp, int bq, bool full, float tol, float smax, unsigned* cnt,
                                         GrShared<W>& sh, float2* rows, int row0, int rank, int cs) {
-  constexpr int C = 2 * W, LD = C + 2, TC = C / 4, NTL = TC * (TC + 1) / 2, RT = SPLIT ? NT / 2 : NT;
-  constexpr int NG = NT / NTL * NTL * 16 <= RT * LD ? NT / NTL : RT * LD / (NTL * 16);
-  static_assert(NG >= 1, "the group sums reuse the row tile");
-  const int tid = threadIdx.x, r = row0 + tid % RT;
-  const bool vrow = SPLIT && tid >= RT;
+  constexpr int C = 2 * W, LD = C + 2, TC = C / 4, NTL = TC * (TC + 1) / 2, NG = NT / NTL;
+  static_assert(NG >= 1 && NG * NTL * 16 <= NT * LD, "the group sums reuse the row tile");
+  const int tid = threadIdx.x, r = row0 + tid;
   const int nq = min(W, n - bq * W);  // bq may be the padding block (bq >= nb: no columns)
   const int np = min(W, n - bp * W);
   auto colp = [&](int c) { return c < W ? (c < np ? bp * W + c : -1) : (bq < nb && c - W < nq ? bq * W + c - W : -1); };
@@ -135,18 +132,11 @@ __device__ __forceinline__ void gr_item(float2* __restrict__ B, long ldb, int m,
 #pragma unroll
   for (int c = 0; c < C; c++) {
     const int col = colp(c);
-    x[c] = make_float2(0.f, 0.f);
-    if (vrow) {
-      if (col >= 0 && r < n) x[c] = __ldcg(V + (long)col * ldv + r);
-    } else {
-      if (col >= 0 && r < m) x[c] = __ldcg(B + (long)col * ldb + r);
-    }
+    x[c] = (col >= 0 && r < m) ? __ldcg(B + (long)col * ldb + r) : make_float2(0.f, 0.f);
   }
-  if (!vrow) {
 #pragma unroll
-    for (int c = 0; c < C; c += 2)
-      *reinterpret_cast<float4*>(rows + tid * LD + c) = make_float4(x[c].x, x[c].y, x[c + 1].x, x[c + 1].y);
-  }
+  for (int c = 0; c < C; c += 2)
+    *reinterpret_cast<float4*>(rows + tid * LD + c) = make_float4(x[c].x, x[c].y, x[c + 1].x, x[c + 1].y);
   gr_item_sync<NT>();
   // partial Gram matrix: a thread owns a 4 x 4 tile on or above the diagonal for every NG-th row
   float2 acc[4][4];
@@ -158,7 +148,7 @@ __device__ __forceinline__ void gr_item(float2* __restrict__ B, long ldb, int m,
   int tj = 0;
   while ((tj + 1) * (tj + 2) / 2 <= tl) tj++;
   const int ti = tl - tj * (tj + 1) / 2;
-  const int live = min(RT, max(0, m - row0));
+  const int live = min(NT, max(0, m - row0));
   if (g < NG) {
 #pragma unroll 2
     for (int q = g; q < live; q += NG) {
@@ -305,13 +295,9 @@ __device__ __forceinline__ void gr_item(float2* __restrict__ B, long ldb, int m,
 #pragma unroll
   for (int c = 0; c < C; c++) {
     const int col = colp(c);
-    if (vrow) {
-      if (col >= 0 && r < n) __stcg(V + (long)col * ldv + r, x[c]);
-    } else {
-      if (col >= 0 && r < m) __stcg(B + (long)col * ldb + r, x[c]);
-    }
+    if (col >= 0 && r < m) __stcg(B + (long)col * ldb + r, x[c]);
   }
-  if (!SPLIT && r < n) {
+  if (r < n) {
 #pragma unroll
     for (int c = 0; c < C; c++) {
       const int col = colp(c);

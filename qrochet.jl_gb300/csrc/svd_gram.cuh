@@ -37,9 +37,8 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 4 : 2)
 
 // Up to 128 columns and 128 rows: all sweeps in one cluster, a CTA per item of a round, the cluster barrier
 // between rounds.  state as in jacobi_cluster_k.
-constexpr int GC_NT = 2 * JC_NT;  // a thread per row of B and one per row of V
 template <int W>
-__global__ void __launch_bounds__(GC_NT) jacobi_gram_cluster_k(float2* __restrict__ B, long ldb, int m, int n,
+__global__ void __launch_bounds__(JC_NT) jacobi_gram_cluster_k(float2* __restrict__ B, long ldb, int m, int n,
                                                                float2* __restrict__ V, long ldv, float tol,
                                                                const double* __restrict__ smax_p, int max_sweeps,
                                                                unsigned* __restrict__ state, float tan_stop) {
@@ -56,7 +55,7 @@ __global__ void __launch_bounds__(GC_NT) jacobi_gram_cluster_k(float2* __restric
         int bp, bq;
         pair_cols(nbp, round, pair, bp, bq);
         if (bq < nb || round == 0) 
-          gr_item<W, GC_NT, true>(B, ldb, m, n, V, ldv, nb, bp, bq, round == 0, tol, smax, cnt, sh, gr_rows, 0, 0, 1);
+          gr_item<W, JC_NT>(B, ldb, m, n, V, ldv, nb, bp, bq, round == 0, tol, smax, cnt, sh, gr_rows, 0, 0, 1);
         __syncthreads();  // shared state is reused by the next item
       }
       cluster_sync_all();
