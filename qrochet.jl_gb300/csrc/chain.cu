@@ -541,11 +541,12 @@ __global__ void mix_k(const double2* __restrict__ X, double2* __restrict__ Y, co
 // The nonzero entries of one site's W, grouped by output (o, w'): MPOs of local Hamiltonians and
 // products of few-site observables are sparse (the XXZ MPO has 12 nonzeros among its 100 entries),
 // so the mixing step does only their multiply-adds.  Passed to the kernel by value.
-constexpr int MIX_MAX_TERMS = 96, MIX_MAX_OUT = 16;
+constexpr int MIX_MAX_TERMS = 96, MIX_MAX_OUT = 16, MIX_REAL = 4;
 struct MixTable {
   int nout;
   int start[MIX_MAX_OUT + 1];
   short w[MIX_MAX_TERMS], i[MIX_MAX_TERMS];
+  char kind[MIX_MAX_TERMS];       // n < MIX_REAL: i^n; MIX_REAL: real; larger: complex
   double2 v[MIX_MAX_TERMS];
 };
 
@@ -566,6 +567,8 @@ bool build_mix_table(const double2* W, int wl, int d, int wr, MixTable* t) {
           t->w[nt] = (short)w;
           t->i[nt] = (short)i;
           t->v[nt] = v;
+          t->kind[nt] = v.y == 0.0 ? (v.x == 1.0 ? 0 : v.x == -1.0 ? 2 : MIX_REAL)
+                                   : v.x == 0.0 && v.y == 1.0 ? 1 : v.x == 0.0 && v.y == -1.0 ? 3 : MIX_REAL + 1;
           nt++;
         }
     }
@@ -573,20 +576,73 @@ bool build_mix_table(const double2* W, int wl, int d, int wr, MixTable* t) {
   return true;
 }
 
-// mix_k over the nonzeros only: Y[b,o,w',a'] = sum over the table's (w, i) of W X[w,b,i,a']
-__global__ void mix_sparse_k(const double2* __restrict__ X, double2* __restrict__ Y, const MixTable tab, int wl,
-                             int d, int cb, int ca2) {
-  const long pairs = (long)cb * ca2;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < pairs; t += (long)gridDim.x * blockDim.x) {
-    const long b = t % cb, a2 = t / cb;
-    for (int out = 0; out < tab.nout; out++) {
-      double2 acc = make_double2(0, 0);
-      for (int e = tab.start[out]; e < tab.start[out + 1]; e++)
-        acc = cadd(acc, cmul(tab.v[e], X[tab.w[e] + wl * (b + (long)cb * (tab.i[e] + (long)d * a2))]));
-      const int o = out % d, w2 = out / d;
-      Y[b + (long)cb * (o + (long)d * (w2 + (long)(tab.nout / d) * a2))] = acc;
-    }
+// mix_k over the nonzeros only: Y[b,o,w',a'] = sum over the table's (w, i) of W X[w,b,i,a'].
+//
+// A block takes nb values of b at one a'; with STAGED it copies their X (contiguous for every i) to shared
+// memory first, from which the terms' strided reads are conflict-free for odd wl.  Bound by memory: the
+// coefficients of Pauli sums are mostly 1, -1, i and -i, which cost no multiplication, and real ones half of a
+// complex one.  (Reading global memory once per term, with complex multiply-adds throughout, was bound by both
+// FP64 and latency: 91 us for 704 x 704 pairs and 5 channels, 53 now.)  A sum that is not finite
+// is formed again with all operations, as 0 * inf belongs to it.
+__device__ __forceinline__ double flip(double x) {  // -x without the FP64 pipe
+  return __hiloint2double(__double2hiint(x) ^ 0x80000000, __double2loint(x));
+}
+template <bool STAGED>
+__global__ void __launch_bounds__(256) mix_sparse_k(const double2* __restrict__ X, double2* __restrict__ Y,
+                                                    const MixTable tab, int wl, int d, int cb, int nb, int nchunk) {
+  extern __shared__ __align__(16) double2 mix_sm[];
+  const long a2 = blockIdx.x / nchunk;
+  const int b0 = (blockIdx.x % nchunk) * nb, live = min(nb, cb - b0);
+  const double2* src = X + wl * (b0 + (long)cb * d * a2);
+  long istride = (long)wl * cb;
+  if (STAGED) {
+    for (int i = 0; i < d; i++)
+      for (int e = threadIdx.x; e < wl * live; e += 256) mix_sm[i * wl * nb + e] = src[i * istride + e];
+    __syncthreads();
+    src = mix_sm;
+    istride = wl * nb;
   }
+  const int bl = threadIdx.x % nb;
+  if (bl >= live) return;
+  src += wl * bl;
+  for (int out = threadIdx.x / nb; out < tab.nout; out += 256 / nb) {
+    double2 acc = make_double2(0.0, 0.0);
+    const int e0 = tab.start[out], e1 = tab.start[out + 1];
+    for (int e = e0; e < e1; e++) {
+      double2 x = src[tab.w[e] + tab.i[e] * istride];
+      const int kind = tab.kind[e];
+      if (kind < MIX_REAL) {  // a power of i: 1, i, -1, -i
+        if (kind & 1) x = make_double2(flip(x.y), x.x);
+        if (kind & 2) x = make_double2(flip(x.x), flip(x.y));
+        acc = e == e0 ? x : cadd(acc, x);
+      } else {
+        const double2 v = tab.v[e];
+        acc.x = fma(v.x, x.x, acc.x);
+        acc.y = fma(v.x, x.y, acc.y);
+        if (kind != MIX_REAL) {
+          acc.x = fma(-v.y, x.y, acc.x);
+          acc.y = fma(v.y, x.x, acc.y);
+        }
+      }
+    }
+    if (!isfinite(acc.x) || !isfinite(acc.y)) {
+      acc = make_double2(0.0, 0.0);
+      for (int e = e0; e < e1; e++) acc = cadd(acc, cmul(tab.v[e], src[tab.w[e] + tab.i[e] * istride]));
+    }
+    const int o = out % d, w2 = out / d;
+    Y[b0 + bl + (long)cb * (o + (long)d * (w2 + (long)(tab.nout / d) * a2))] = acc;
+  }
+}
+int mix_sparse(cudaStream_t s, const double2* X, double2* Y, const MixTable& tab, int wl, int d, int cb, int ca2) {
+  int nb = 256;
+  while (nb > 32 && (nb >= 2 * cb || sizeof(double2) * wl * d * nb > 48 * 1024)) nb /= 2;
+  const size_t smem = sizeof(double2) * wl * d * nb;
+  const bool staged = smem <= 48 * 1024;
+  const int nchunk = (cb + nb - 1) / nb;
+  if (staged) mix_sparse_k<true><<<(unsigned)nchunk * ca2, 256, smem, s>>>(X, Y, tab, wl, d, cb, nb, nchunk);
+  else mix_sparse_k<false><<<(unsigned)nchunk * ca2, 256, 0, s>>>(X, Y, tab, wl, d, cb, nb, nchunk);
+  QR_CHECK_LAUNCH("mix_sparse_k");
+  return QR_OK;
 }
 
 struct EnvOps {
@@ -795,13 +851,15 @@ int env_sweep(const qr_chain* a, const qr_chain* b, const EnvOps* ops, cudaStrea
     if (rc) break;
     const double2* Yp = X;
     if (W) {
-      long pairs = (long)cb * ca2;
-      unsigned g = (unsigned)((pairs + 255) / 256);
-      if (!ops->has_tab.empty() && ops->has_tab[i])
-        mix_sparse_k<<<g > 4864 ? 4864 : g, 256, 0, s>>>(X, Y, ops->tab[i], wl, d, cb, ca2);
-      else
+      if (!ops->has_tab.empty() && ops->has_tab[i]) {
+        rc = mix_sparse(s, X, Y, ops->tab[i], wl, d, cb, ca2);
+        if (rc) break;
+      } else {
+        const long pairs = (long)cb * ca2;
+        const unsigned g = (unsigned)((pairs + 255) / 256);
         mix_k<<<g > 4864 ? 4864 : g, 256, sizeof(double2) * wl * d * d * wr, s>>>(X, Y, W, wl, wr, d, cb, ca2);
-      count_launch();
+        count_launch();
+      }
       Yp = Y;
     }
     // E'_w' = Y_w'^T conj(B)
