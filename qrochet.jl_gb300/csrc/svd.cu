@@ -1555,6 +1555,13 @@ __global__ void gather_cols_k(const CS* __restrict__ src, long lds, int rows, in
 
 
 // Q[:, j] *= phase(R_jj) (R_jj == 0 -> 1): keeps Q as close to the input columns as possible
+// row i of src to row perm[i] of dst
+__global__ void scatter_rows_k(const double2* __restrict__ src, int k, const int* __restrict__ perm, double2* __restrict__ dst,
+                               long ldd) {
+  const long total = (long)k * k;
+  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x)
+    dst[perm[t % k] + t / k * ldd] = src[t];
+}
 __global__ void phase_fix_k(double2* Q, long ldq, int m, int k, const double2* R, long ldr) {
   long total = (long)m * k;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
@@ -2371,21 +2378,35 @@ constexpr int kFp64CloseCols = 512;
 constexpr double kSmallCol = 1e-4;
 constexpr double kSmallColFrac = 0.1;
 // Above 128 columns the decision falls after kMixedFirstSweeps sweeps when the spectrum visibly decays:
-// more than kDecayFrac of those columns below kDecayCol sigma_max (a square Gaussian block has 1%).
+// more than kDecayFrac of all columns below kDecayCol of the largest.  In a CPU model of theta of 180 to 192
+// columns that part is 0 - 4% over 0.5 to 2 decades of Schmidt values (10 - 12 sweeps, 7 on R^H: not worth a QR at
+// large sizes) and 22 - 69% over 3 to 7 decades (11 - 19 sweeps).  768 columns over 7 decades: 45.2 ms when
+// deciding after 5 sweeps, without the order of qr_precondition, 32.3 now; 154 columns over 4 decades 5.8 and 4.7.
 // A last probe sweep that still rotates more than kSlowFrac of the pairs (1% at 2048 Gaussian columns,
 // 44% over 4 decades) restarts as well.
-constexpr int kMixedFirstSweeps = 5;
-constexpr double kDecayCol = 1e-2;
-constexpr double kDecayFrac = 0.25;
+constexpr int kMixedFirstSweeps = 2;
+constexpr double kDecayCol = 3e-2;
+constexpr double kDecayFrac = 0.1;
 constexpr double kSlowFrac = 0.05;
 
-// B (rows x k, rows >= k) = Q R with Q in w->Qp (rows x k); B is replaced by W = R^H (k x k, ld k)
-static int qr_precondition(cudaStream_t s, SvdWork* w, double2* B, int rows, int k) {
+// B P = Q R (B rows x k, rows >= k) with Q in w->Qp (rows x k) and P, columns by falling norm, in `order`; B is
+// replaced by W = R^H (k x k, ld k).  The order gathers what the columns know of the spectrum, much like column
+// pivoting would: W is closer to diagonal, and its FP32 sweeps fall from 15 to 7 at 7 decades (CPU model, 192
+// columns; 11 to 8 at 4 decades).
+static int qr_precondition(cudaStream_t s, SvdWork* w, double2* B, int rows, int k, int* order) {
   QR_TRY(w->Qp.ensure(sizeof(double2) * (size_t)rows * k, s));
   QR_TRY(w->qtmp.ensure(sizeof(double2) * (size_t)k * k, s));
   QR_TRY(w->tau.ensure(sizeof(double2) * (size_t)k, s));
   double2* Rr = w->qtmp.as<double2>();
-  QR_TRY(zqr_thin(s, B, rows, k, rows, w->Qp.as<double2>(), rows, Rr, k, w->tau.as<double2>()));
+  QR_TRY(w->T1.ensure(sizeof(double2) * (size_t)rows * k, s));
+  double2* S = w->T1.as<double2>();
+  col_norms_k<double2><<<ceil_div((long)k * 32, TPB), TPB, 0, s>>>(B, rows, rows, k, w->nrm.as<double>());
+  QR_CHECK_LAUNCH("col_norms_k");
+  rank_sort_k<<<ceil_div(k, TPB), TPB, 0, s>>>(w->nrm.as<double>(), k, order, nullptr);
+  QR_CHECK_LAUNCH("rank_sort_k");
+  gather_cols_k<double2><<<gs((long)rows * k), TPB, 0, s>>>(B, rows, rows, k, order, nullptr, S, rows);
+  QR_CHECK_LAUNCH("gather_cols_k");
+  QR_TRY(zqr_thin(s, S, rows, k, rows, w->Qp.as<double2>(), rows, Rr, k, w->tau.as<double2>()));
   return ztranspose(s, Rr, k, k, k, B, k, 1);
 }
 
@@ -2461,13 +2482,13 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
   QR_TRY(w->B.ensure(sizeof(double2) * (size_t)rows0 * k, s));
   QR_TRY(w->V.ensure(sizeof(double2) * (size_t)k * k, s));
   QR_TRY(w->nrm.ensure(sizeof(double) * (size_t)k * 2, s));
-  QR_TRY(w->perm.ensure(sizeof(int) * (size_t)k, s));
+  QR_TRY(w->perm.ensure(sizeof(int) * 2 * (size_t)k, s));
   QR_TRY(w->cnt.ensure(sizeof(unsigned) * 8, s));
   double2* B = w->B.as<double2>();
   double2* V = w->V.as<double2>();
   double* nrm = w->nrm.as<double>();
   double* sorted = nrm + k;
-  int* perm = w->perm.as<int>();
+  int *perm = w->perm.as<int>(), *order = perm + k;
 
   // B = A or A^H (FP64 copy; A is preserved)
   if (tall) {
@@ -2486,7 +2507,7 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
   } else if (mode == QR_FP64 || k <= kMixedMinCols) {
     if (k > kPrecondMinCols) {
       svd_path(SP_QR_PRECOND_FP64);
-      QR_TRY(qr_precondition(s, w, B, rows0, k));
+      QR_TRY(qr_precondition(s, w, B, rows0, k, order));
       rows = k;
       pre = true;
     }
@@ -2519,8 +2540,8 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
     float tol32 = fmaxf(4e-6f, 2.0f * sqrtf((float)rows) * Eps<float>::v);
     // columns the polish rotates: all, or the leading keep + margin (see below)
     const int k0 = keep > 0 && keep < k ? std::min(k, keep + std::max(32, keep / 8)) : k;
-    // columns below `rel` of the largest, among the k0 leading ones by norm
-    auto small_cols = [&](double rel, int* count) -> int {
+    // columns below `rel` of the largest, among the `upto` leading ones by norm
+    auto small_cols = [&](double rel, int upto, int* count) -> int {
       col_norms_k<float2><<<ceil_div((long)k * 32, TPB), TPB, 0, s>>>(B32, rows, rows, k, nrm);
       QR_CHECK_LAUNCH("col_norms_k");
       double* hn = static_cast<double*>(host_scratch(sizeof(double) * k));
@@ -2530,7 +2551,7 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
       std::vector<double> sn(hn, hn + k);
       std::sort(sn.begin(), sn.end(), std::greater<double>());
       *count = 0;
-      for (int j = 0; j < k0; j++) *count += sn[j] < rel * sn[0];
+      for (int j = 0; j < upto; j++) *count += sn[j] < rel * sn[0];
       return QR_OK;
     };
     int conv32 = 0, small = 0;
@@ -2543,15 +2564,15 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
                            &frac32));
       ran = kMixedFirstSweeps;
       if (!conv32) {
-        QR_TRY(small_cols(kDecayCol, &small));
-        slow = small > kDecayFrac * k0;
+        QR_TRY(small_cols(kDecayCol, k, &small));
+        slow = small > kDecayFrac * k;
       }
     }
     if (!conv32 && !slow) {
       QR_TRY(jacobi<float>(s, w, B32, rows, rows, k, V32, k, kMixedProbeSweeps - ran, tol32, false, kPrecondTanStop,
                            &conv32, &frac32));
       if (!conv32) {
-        QR_TRY(small_cols(kSmallCol, &small));
+        QR_TRY(small_cols(kSmallCol, k0, &small));
         slow = small > kSmallColFrac * k0 || frac32 > kSlowFrac;
       }
     }
@@ -2568,7 +2589,7 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
     } else if (!conv32) {
       // slow convergence (widely spread spectrum): precondition in FP64 and start over on R^H
       svd_path(SP_QR_PRECOND_MIXED);
-      QR_TRY(qr_precondition(s, w, B, rows0, k));
+      QR_TRY(qr_precondition(s, w, B, rows0, k, order));
       rows = k;
       pre = true;
       tol32 = fmaxf(4e-6f, 2.0f * sqrtf((float)rows) * Eps<float>::v);
@@ -2605,8 +2626,8 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
   QR_TRY(w->E.ensure(sizeof(double2) * (size_t)k * k, s));
   double2* Rf = w->E.as<double2>();
   if (pre) {
-    // W = R^H = L Sigma Rf^H  =>  B0 = Q R = (Q Rf) Sigma L^H: the left factor of B0 is Q Rf
-    // (orthonormal: Householder Q times accumulated rotations) and its right factor is L
+    // W = R^H = L Sigma Rf^H  =>  B0 = Q R P^T = (Q Rf) Sigma (P L)^H: the left factor of B0 is Q Rf
+    // (orthonormal: Householder Q times accumulated rotations) and its right factor is P L
     QR_TRY(w->Rm.ensure(sizeof(double2) * (size_t)k * k, s));
     double2* L = w->Rm.as<double2>();
     gather_cols_k<double2><<<gs((long)k * k), TPB, 0, s>>>(B, k, k, k, perm, sorted, L, k);
@@ -2616,15 +2637,17 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
     gather_cols_k<double2><<<gs((long)k * k), TPB, 0, s>>>(V, k, k, k, perm, nullptr, Rf, k);
     QR_CHECK_LAUNCH("gather_cols_k");
     const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
-    if (tall) {  // A = B0: U = Q Rf (m x k), Vh = L^H
+    if (tall) {  // A = B0: U = Q Rf (m x k), Vh = (P L)^H
       QR_TRY(zgemm(s, OP_N, OP_N, rows0, k, k, one, w->Qp.as<double2>(), rows0, 0, Rf, k, 0, zero, U, ldu, 0, 1,
                    nullptr));
-      QR_TRY(ztranspose(s, L, k, k, k, Vh, ldvh, 1));
-    } else {  // A = B0^H = L Sigma (Q Rf)^H: U = L (m x m), Vh = (Q Rf)^H (m x n); B is free
+      scatter_rows_k<<<gs((long)k * k), TPB, 0, s>>>(L, k, order, V, k);
+      QR_CHECK_LAUNCH("scatter_rows_k");
+      QR_TRY(ztranspose(s, V, k, k, k, Vh, ldvh, 1));
+    } else {  // A = B0^H = P L Sigma (Q Rf)^H: U = P L (m x m), Vh = (Q Rf)^H (m x n); B is free
       QR_TRY(zgemm(s, OP_N, OP_N, rows0, k, k, one, w->Qp.as<double2>(), rows0, 0, Rf, k, 0, zero, B, rows0, 0, 1,
                    nullptr));
-      QR_CUDA(cudaMemcpy2DAsync(U, sizeof(double2) * ldu, L, sizeof(double2) * k, sizeof(double2) * k, k,
-                                cudaMemcpyDeviceToDevice, s));
+      scatter_rows_k<<<gs((long)k * k), TPB, 0, s>>>(L, k, order, U, ldu);
+      QR_CHECK_LAUNCH("scatter_rows_k");
       QR_TRY(ztranspose(s, B, rows0, rows0, k, Vh, ldvh, 1));
     }
     return QR_OK;
