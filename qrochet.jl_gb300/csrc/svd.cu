@@ -7,9 +7,11 @@
 // singular vectors X to ~1e-5 (svd_gram.cuh) and products at FP64 accuracy on the tensor cores finish
 // them (svd_refine.cuh); singular values, vectors and the truncation cutoff are FP64.
 //   QR_FP64: QR first, the sweeps on R^H; the finish to the FP64 sweeps' tolerance, one FP64 sweep to
-//            close it above 512 columns.  Up to 32 columns the whole Jacobi runs in FP64.
+//            close it above 512 columns.
 //   QR_MIXED: the sweeps on B itself (on R^H when the spectrum decays), the finish to a few times that
 //            tolerance and only for the leading triplets when the caller keeps no more.
+// Either way blocks of 17 to 32 columns run on one cluster in one launch (team_svd.cuh), and smaller ones take FP64
+// sweeps.
 //
 // Left singular vectors are the normalised columns B/sigma.  When the spectrum spans many
 // decades (or has exact zeros) those columns lose orthogonality in proportion to
@@ -1579,8 +1581,8 @@ inline unsigned gs(long n) {
   return (unsigned)(g < 1 ? 1 : g);
 }
 
-// Hestenes sweeps on B (rows x k) accumulating V (k x k).  Small problems (k <= 32) run the
-// whole iteration in one CTA; larger ones enqueue up to max_sweeps cooperative sweep launches
+// Hestenes sweeps on B (rows x k) accumulating V (k x k).  Small problems (k <= 128) run the
+// whole iteration in one cluster; larger ones enqueue up to max_sweeps cooperative sweep launches
 // whose convergence is decided on the device.  One host synchronisation per call.
 template <typename T>
 int jacobi(cudaStream_t s, SvdWork* w, cplx_t<T>* B, long ldb, int rows, int k, cplx_t<T>* V,
@@ -2382,12 +2384,14 @@ constexpr double kSmallColFrac = 0.1;
 // columns that part is 0 - 4% over 0.5 to 2 decades of Schmidt values (10 - 12 sweeps, 7 on R^H: not worth a QR at
 // large sizes) and 22 - 69% over 3 to 7 decades (11 - 19 sweeps).  768 columns over 7 decades: 45.2 ms when
 // deciding after 5 sweeps, without the order of qr_precondition, 32.3 now; 154 columns over 4 decades 5.8 and 4.7.
-// A last probe sweep that still rotates more than kSlowFrac of the pairs (1% at 2048 Gaussian columns,
-// 44% over 4 decades) restarts as well.
+// A last probe sweep that still rotates more than kSlowFrac of the pairs restarts as well: 1 - 5% over half a decade
+// (1024 and 2048 columns), 8 - 18% over 1 to 2.5 decades, 21 - 50% over 3 to 7.  Restarting from 5% on cost
+// 58 ms instead of 39 at 1024 columns over 1.5 decades, and 346 instead of 201 at 2048 over half a decade, where
+// that part lies at 4 - 6%.
 constexpr int kMixedFirstSweeps = 2;
 constexpr double kDecayCol = 3e-2;
 constexpr double kDecayFrac = 0.1;
-constexpr double kSlowFrac = 0.05;
+constexpr double kSlowFrac = 0.3;
 
 // B P = Q R (B rows x k, rows >= k) with Q in w->Qp (rows x k) and P, columns by falling norm, in `order`; B is
 // replaced by W = R^H (k x k, ld k).  The order gathers what the columns know of the spectrum, much like column
