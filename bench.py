@@ -139,10 +139,10 @@ class DevTimer:
 
 
 # DRAM bytes (read + write) per launch (one Jacobi sweep, or one GEMM) from one ncu capture of each
-# kernel on a 1024 x 1024 mixed SVD: jacobi_block_reg_k for jacobi_fp32, jacobi_block_df_k (the
-# full double-float sweeps) for jacobi_df, zgemm_df_k for zgemm_df.  A sweep's traffic is the first
-# touch of B and V and a GEMM's the first touch of its operands, so it scales with the operand
-# size: (k / 1024)^2 at k columns.
+# kernel on a 1024 x 1024 mixed SVD: jacobi_block_reg_k for jacobi_fp32 (the Gram sweeps touch the same
+# B and V; ncu does not launch them), jacobi_block_df_k (the full double-float sweeps) for jacobi_df,
+# zgemm_df_k for zgemm_df.  A sweep's traffic is the first touch of B and V and a GEMM's the first
+# touch of its operands, so it scales with the operand size: (k / 1024)^2 at k columns.
 NCU_TRAFFIC_1024 = {"jacobi_fp32": 16.937472e6 + 15.872e3, "jacobi_df": 34.0e6 + 5.3e6,
                     "zgemm_df": 16.850432e6}
 
@@ -649,10 +649,9 @@ def run_ours(args, chi):
             "executed_tflops": ex64 / (ms64 * 1e-3) / 1e12 if ms64 > 0 else 0.0,
             "executed_frac_of_dfma": ex64 / (ms64 * 1e-3) / (dfma * 1e12) if ms64 > 0 else 0.0,
             "time_share": {k: round(v["ms"] / max(1e-9, ms64), 4) for k, v in st64.items() if v["ms"] > 0},
-            "note": "executed = the FP64 operations the kernels count (Jacobi inner products and rotations, "
-                    "Householder QR, DMMA GEMMs) over their event time: one-sided Jacobi does ~4x the "
-                    "Golub-Van Loan R-SVD count, so the executed rate, not the algorithmic one, shows how "
-                    "busy the FP64 pipe is"}
+            "note": "executed = the operations the kernels count (Jacobi inner products and rotations, "
+                    "Householder QR, GEMMs) over their event time; the sweeps run in FP32 and the large "
+                    "products as exact 8-bit slices on the tensor cores, so it exceeds the FP64 pipe's rate"}
         del p64
 
     # ---- e2e through the C ABI with pinned host buffers --------------------------------------------
@@ -790,7 +789,7 @@ def run_ours(args, chi):
         line = {"metric": METRIC, "value": value, "unit": "gate-steps/s", "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": 1e3 * dt_max / args.steps, "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None,
-                "dtype": "complex64 Jacobi preconditioner + double-float (FP32-pair) theta GEMM, Newton-Schulz, B = A X and Jacobi polish; complex128 gate and results",
+                "dtype": "complex64 Jacobi sweeps; FP64-accurate products (exact 8-bit slices on tcgen05) for theta and the SVD's refinement; complex128 gate and results",
                 "data": "synthetic",
                 "config": {"workload": f"tebd_gate_step_chi{chi}", "chi": chi, "theta": f"{2 * chi}x{2 * chi}",
                            "maxdim": maxdim, "threshold": CUTOFF, "n_sites": N_SITES, "precision": "mixed",

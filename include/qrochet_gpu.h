@@ -53,12 +53,12 @@ typedef struct qr_mpo qr_mpo;     /* one open-boundary MPO resident in device me
 
 /* Precision of a chain's arithmetic (qr_chain_set_precision), a bit mask. */
 #define QR_FP64 0           /* plain: all ComplexF64 */
-#define QR_MIXED 1          /* two-site gates whose theta has more than 16 columns: theta formed by a
-                               double-float GEMM (FP32 pairs, ~2^-48, on the FP32 pipes; the gate is
-                               applied in FP64), then an SVD with an FP32 Jacobi preconditioner and
-                               double-float Newton-Schulz, B = A X and Jacobi polish; singular values
-                               and vectors and the truncation cutoff stay FP64.  Smaller SVDs run the
-                               FP64 Jacobi. */
+#define QR_MIXED 1          /* SVDs of more than 16 columns take their FP32 Jacobi sweeps straight on the
+                               matrix (QR_FP64 on the R^H of a QR above 32 columns), may finish by
+                               double-float sweeps (FP32 pairs, ~2^-48) where the refinement by products
+                               leaves pairs over, and accept couplings of 4 sqrt(m) eps sigma_max instead
+                               of sqrt(m) eps.  Products, singular values and vectors and the truncation
+                               cutoff are FP64-accurate in both modes. */
 #define QR_SPLIT_CONTRACT 2 /* environment contractions (expect, overlap, norm, MPO expectation) on
                                the BF16 tensor cores with 3-way BF16 splits, FP32 accumulation */
 
@@ -198,9 +198,9 @@ int qr_server_stats(qr_server* s, uint64_t* submitted, uint64_t* completed, int*
 typedef struct qr_batch qr_batch;
 int qr_batch_create(int device, qr_batch** out);
 int qr_batch_free(qr_batch* b);
-/* QR_FP64 (default): every gate's SVD in FP64.  QR_MIXED: SVDs of more than 32 columns run FP32
-   Jacobi sweeps first, one FP64 Newton-Schulz step on their rotations, then FP64 sweeps to the
-   FP64 tolerance; singular values, vectors and truncation decisions stay FP64.  Before run. */
+/* SVDs of more than 16 columns run FP32 Jacobi sweeps first and finish to the FP64 tolerance in FP64
+   (QR_FP64, the default) or, above 32 columns, in double-float (QR_MIXED); singular values, vectors and
+   truncation decisions stay FP64.  Before run. */
 int qr_batch_set_precision(qr_batch* b, int mode);
 int qr_batch_add(qr_batch* b, int n, int chi_max, double threshold, int ngates, const int* gate_site,
                  const double* gate_mats, int nobs, const int* obs_weight, const int* obs_sites,

@@ -14,7 +14,7 @@
 extern "C" {
 #endif
 
-/* per-kernel-class CUDA-event timing, for benchmarks: kinds 0 zgemm (FP64 DMMA), 1 Jacobi FP64,
+/* per-kernel-class CUDA-event timing, for benchmarks: kinds 0 zgemm (FP64), 1 Jacobi FP64,
    2 Jacobi FP32, 3 Householder QR, 4 environment mixing, 5 split-precision tensor-core zgemm,
    6 double-float Jacobi polish, 7 double-float zgemm.  `launches` counts kernel launches of the
    class (one per Jacobi sweep). */

@@ -10,12 +10,13 @@
 //   - bond dimensions, Lambda flags and Lambda vectors are device arrays that the kernels read
 //     and rewrite: the truncation decision (the first min(k, maxdim) singular values above the
 //     threshold) is taken on the device, so no layer waits for the host;
-//   - one CTA runs one whole gate step: theta = A_l diag(Lambda) A_r, the gate, a one-sided
-//     Jacobi SVD (theta of at most 128 x 128: chi_max <= 64; FP64, or with QR_MIXED FP32 sweeps
-//     first and a double-float finish on the FP32 pipes), the sort, the truncation,
-//     re-orthonormalisation of the kept vectors when their singular values fall below 1e-3
-//     sigma_max (classical Gram-Schmidt twice), and the write-back of U, Vh and Lambda.  A
-//     layer's gates sit on disjoint bonds, so the CTAs of one launch never touch the same site;
+//   - one cluster of 1, 4 or 8 CTAs runs one whole gate step: theta = A_l diag(Lambda) A_r, the
+//     gate, a Jacobi SVD (theta of at most 128 x 128: chi_max <= 64; FP32 sweeps first above 16
+//     columns, the finish in FP64 or, with QR_MIXED above 32 columns, in double-float on the FP32
+//     pipes), the sort, the truncation, re-orthonormalisation of the kept vectors when their
+//     singular values fall below 1e-3 sigma_max (classical Gram-Schmidt twice), and the write-back
+//     of U, Vh and Lambda.  A layer's gates sit on disjoint bonds, so the clusters of one launch
+//     never touch the same site;
 //   - the expectation values are one more launch: one cluster per Pauli string sweeps the chain's
 //     environment (FP64).
 // The layer kernel's CTA size comes from a small autotuner (timed on synthetic gate steps of the

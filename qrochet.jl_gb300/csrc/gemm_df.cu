@@ -2,9 +2,8 @@
 //
 // On this part FP64 runs at ~1.1 TFLOP/s (DMMA and DFMA alike) against ~75 TFLOP/s for FFMA, so a
 // product carried as hi + lo FP32 pairs with compensated (Dot2) accumulation reaches ~2^-48
-// relative accuracy at several times the FP64 rate.  The mixed SVD uses it for the
-// Newton-Schulz orthonormalisation of the FP32 Jacobi rotations and for B = A X, whose result
-// feeds the double-float Jacobi polish without an FP64 round trip.
+// relative accuracy at several times the FP64 rate.  The double-float Jacobi sweeps that stand behind the
+// SVD's refinement use it for their Gram tests and first-order rotations.
 //
 // Operands are column-major split arrays: the high parts (float2 complex) and the low parts
 // (float2 complex) of each matrix, with the same leading dimension.  Modes:
@@ -283,21 +282,6 @@ __global__ void to_df_scaled_k(const double2* __restrict__ src, long lds, int ro
   }
 }
 
-// hi/lo of src[:, j] * colscale[j] (the Lambda of a bond folded into a site's columns)
-__global__ void to_df_cols_k(const double2* __restrict__ src, long lds, int rows, int cols,
-                             const double* __restrict__ colscale, float2* __restrict__ hi, float2* __restrict__ lo,
-                             long ldd) {
-  const long total = (long)rows * cols;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
-    const long i = t % rows, j = t / rows;
-    const double f = colscale ? colscale[j] : 1.0;
-    const double2 v = src[i + j * lds];
-    const dfl re = df_from(v.x * f), im = df_from(v.y * f);
-    hi[i + j * ldd] = make_float2(re.h, im.h);
-    lo[i + j * ldd] = make_float2(re.l, im.l);
-  }
-}
-
 __global__ void from_df_scaled_k(const float2* __restrict__ hi, const float2* __restrict__ lo, long lds, int rows,
                                  int cols, const double* __restrict__ scale, double2* __restrict__ dst, long ldd) {
   const double f = scale ? scale[0] : 1.0;
@@ -352,14 +336,6 @@ int z2df(cudaStream_t s, const double2* src, long lds, int rows, int cols, const
   if (rows <= 0 || cols <= 0) return QR_OK;
   to_df_scaled_k<<<grid_for((long)rows * cols), TPB, 0, s>>>(src, lds, rows, cols, scale, hi, lo, ldd);
   QR_CHECK_LAUNCH("to_df_scaled_k");
-  return QR_OK;
-}
-
-int z2df_cols(cudaStream_t s, const double2* src, long lds, int rows, int cols, const double* colscale, float2* hi,
-              float2* lo, long ldd) {
-  if (rows <= 0 || cols <= 0) return QR_OK;
-  to_df_cols_k<<<grid_for((long)rows * cols), TPB, 0, s>>>(src, lds, rows, cols, colscale, hi, lo, ldd);
-  QR_CHECK_LAUNCH("to_df_cols_k");
   return QR_OK;
 }
 

@@ -208,9 +208,9 @@ __device__ __forceinline__ void gr_item(float2* __restrict__ B, long ldb, int m,
   }
   gr_item_sync<NT>();
   // Rotations on the Gram matrix, G <- J^H G J per round: the first warp forms the rotations and the
-  // pairs' own blocks, the next ones update the 2 x 2 blocks of pairs (a, b), a < b, a thread each.  G is kept by position and written to the positions after
-  // the shift, so a thread's addresses are the same in every round.  A round is one dependent chain (~500
-  // cycles): only the warps that take part synchronise in it.
+  // pairs' own blocks, the next ones update the 2 x 2 blocks of pairs (a, b), a < b, a thread each.  G is kept
+  // by position and written to the positions after the shift, so a thread's addresses are the same in every
+  // round.  A round is one dependent chain (~900 cycles): only the warps that take part synchronise in it.
   const int nr = full ? 2 * W - 1 : W;
   constexpr int NBL = W * (W - 1) / 2, GR_INNER = 32 + (NBL + 31) / 32 * 32, LG = C + 1;
   constexpr int PART = GR_INNER <= NT ? GR_INNER : NT, SLOTS = (NBL + PART - 33) / (PART - 32);
