@@ -53,8 +53,8 @@ typedef struct qr_mpo qr_mpo;     /* one open-boundary MPO resident in device me
 
 /* Precision of a chain's arithmetic (qr_chain_set_precision), a bit mask. */
 #define QR_FP64 0           /* plain: all ComplexF64 */
-#define QR_MIXED 1          /* SVDs of more than 16 columns take their FP32 Jacobi sweeps straight on the
-                               matrix (QR_FP64 on the R^H of a QR above 32 columns), may finish by
+#define QR_MIXED 1          /* SVDs of more than 32 columns take their FP32 Jacobi sweeps straight on the
+                               matrix (QR_FP64: on the R^H of a QR), may finish by
                                double-float sweeps (FP32 pairs, ~2^-48) where the refinement by products
                                leaves pairs over, and accept couplings of 4 sqrt(m) eps sigma_max instead
                                of sqrt(m) eps.  Products, singular values and vectors and the truncation
@@ -198,7 +198,7 @@ int qr_server_stats(qr_server* s, uint64_t* submitted, uint64_t* completed, int*
 typedef struct qr_batch qr_batch;
 int qr_batch_create(int device, qr_batch** out);
 int qr_batch_free(qr_batch* b);
-/* SVDs of more than 16 columns run FP32 Jacobi sweeps first and finish to the FP64 tolerance in FP64
+/* SVDs of more than 8 columns run FP32 Jacobi sweeps first and finish to the FP64 tolerance in FP64
    (QR_FP64, the default) or, above 32 columns, in double-float (QR_MIXED); singular values, vectors and
    truncation decisions stay FP64.  Before run. */
 int qr_batch_set_precision(qr_batch* b, int mode);

@@ -11,7 +11,7 @@
 //     and rewrite: the truncation decision (the first min(k, maxdim) singular values above the
 //     threshold) is taken on the device, so no layer waits for the host;
 //   - one cluster of 1, 4 or 8 CTAs runs one whole gate step: theta = A_l diag(Lambda) A_r, the
-//     gate, a Jacobi SVD (theta of at most 128 x 128: chi_max <= 64; FP32 sweeps first above 16
+//     gate, a Jacobi SVD (theta of at most 128 x 128: chi_max <= 64; FP32 sweeps first above 8
 //     columns, the finish in FP64 or, with QR_MIXED above 32 columns, in double-float on the FP32
 //     pipes), the sort, the truncation, re-orthonormalisation of the kept vectors when their
 //     singular values fall below 1e-3 sigma_max (classical Gram-Schmidt twice), and the write-back
@@ -43,7 +43,7 @@ constexpr int BT_MAX_SWEEPS = 60;
 // workspace of a gate step of theta up to side x side (double2): theta, B, V and the kept vectors, the SVD's
 // own, a column of coefficients and one of norms
 constexpr size_t slot_size(int side) { return 4 * (size_t)side * side + team_ws(side) + 2 * BT_MAXK; }
-constexpr int BT_PRE_MIN = 16;   // the SVD sweeps in FP32 first above this many columns
+constexpr int BT_PRE_MIN = 8;   // the SVD sweeps in FP32 first above this many columns
 constexpr int BT_TEAM_MAX = 32;  // and its FP64 refinement by products pays up to this many
 constexpr int BT_MAXTEAM = 8;    // CTAs per gate step
 

@@ -10,8 +10,7 @@
 //            close it above 512 columns.
 //   QR_MIXED: the sweeps on B itself (on R^H when the spectrum decays), the finish to a few times that
 //            tolerance and only for the leading triplets when the caller keeps no more.
-// Either way blocks of 17 to 32 columns run on one cluster in one launch (team_svd.cuh), and smaller ones take FP64
-// sweeps.
+// Either way blocks of up to 32 columns and 128 rows run on one cluster in one launch (team_svd.cuh).
 //
 // Left singular vectors are the normalised columns B/sigma.  When the spectrum spans many
 // decades (or has exact zeros) those columns lose orthogonality in proportion to
@@ -2286,11 +2285,12 @@ __global__ void __launch_bounds__(256) svd_team_k(double2* B, int rows, int k, d
   if (T.tid == 0) state[0] = ok ? 1u : 0u;
 }
 
-// One CTA per 8 rows or so of the products, as the FP64 rate of few SMs bounds the smallest ones.
+// As many CTAs as a cluster can have: the FP64 rate of its SMs bounds the products (8 CTAs: 1 - 4% slower gates).
 static int svd_team(cudaStream_t s, SvdWork* w, double2* B, int rows, int k, double2* V) {
   QR_TRY(w->T1.ensure(sizeof(double2) * (team_ws(rows) + TM_MAXK), s));
   QR_TRY(w->cnt.ensure(sizeof(unsigned) * 8, s));
-  const int team = 8;
+  const int team = 16;
+  QR_TRY(set_func_attr_once((const void*)svd_team_k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(team);
   cfg.blockDim = dim3(256);
@@ -2353,11 +2353,10 @@ static int polish_columns(cudaStream_t s, SvdWork* w, double2* L, long ldl, int 
 constexpr float kPrecondTanStop = 0.15f;
 // Smallest block (columns) that takes the mixed path; below it the FP64 cluster Jacobi is as fast.
 constexpr int kMixedMinCols = 16;
-// Blocks of up to TM_MAXK rows and a few dozen columns run on one cluster from norms to the last refinement step.
-// FP64 sweeps take 0.72 ms at 32 columns, the cluster 0.25 ms.  Below kTeamMinCols the sweeps' rounds are few; above
-// kTeamCols its FP64 products are bounded by the rate of 8 SMs, and the tensor-core refinement is faster (128
-// columns: 2.1 ms in one cluster even in double-float, 1.4 ms there).
-constexpr int kTeamMinCols = 16;
+// Blocks of up to TM_MAXK rows and a few dozen columns run on one cluster from norms to the last refinement step:
+// FP64 sweeps take 0.72 ms at 32 columns, the cluster 0.25 ms, and a whole gate 1.04 and 0.58 ms at 16, 0.69 and
+// 0.54 at 8, 0.55 and 0.51 at 4.  Above kTeamCols its FP64 products are bounded by the rate of its SMs, and the
+// tensor-core refinement is faster (128 columns: 2.1 ms in one cluster even in double-float, 1.4 ms there).
 constexpr int kTeamCols = 32;
 // QR preconditioning (Drmac and Veselic): B = Q R, then the one-sided Jacobi runs on W = R^H.
 // When B's singular values are spread over many decades and its right singular vectors are not
@@ -2502,12 +2501,10 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
     QR_TRY(ztranspose(s, A, lda, m, n, B, rows, 1));
   }
 
-  // The FP32-preconditioned path pays off above a few dozen columns; tiny blocks take the FP64
-  // Jacobi directly (same accuracy).
-  const bool team = rows0 <= TM_MAXK && k > kTeamMinCols && k <= kTeamCols;
+  const bool team = rows0 <= TM_MAXK && k > 1 && k <= kTeamCols;
   if (team) {
     QR_TRY(svd_team(s, w, B, rows, k, V));
-    refined = mode != QR_FP64;
+    refined = mode != QR_FP64 && k > kMixedMinCols;
   } else if (mode == QR_FP64 || k <= kMixedMinCols) {
     if (k > kPrecondMinCols) {
       svd_path(SP_QR_PRECOND_FP64);

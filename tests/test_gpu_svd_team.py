@@ -34,14 +34,14 @@ def check(mode, A, tol=1e-12):
 
 
 @pytest.mark.parametrize("mode", [0, 1])
-@pytest.mark.parametrize("m,n", [(16, 16), (17, 17), (23, 128), (24, 31), (32, 32), (128, 32), (129, 32), (33, 33),
+@pytest.mark.parametrize("m,n", [(2, 2), (128, 2), (3, 7), (8, 8), (9, 12), (16, 16), (17, 17), (23, 128), (24, 31), (32, 32), (128, 32), (129, 32), (33, 33),
                                  (40, 39), (64, 65), (65, 100), (127, 127), (128, 128), (17, 129)])
 def test_sizes(mode, m, n):
     check(mode, R.complex_gaussian(R.rng(m * 131 + n), (m, n)))
 
 
 @pytest.mark.parametrize("mode", [0, 1])
-@pytest.mark.parametrize("n", [20, 32, 100, 128])
+@pytest.mark.parametrize("n", [8, 20, 32, 100, 128])
 @pytest.mark.parametrize("kind", ["equal", "degenerate", "clusters", "decades", "steep", "rank"])
 def test_spectra(mode, n, kind):
     g = R.rng(n)
