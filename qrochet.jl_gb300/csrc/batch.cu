@@ -482,12 +482,12 @@ __global__ void __launch_bounds__(512, 1)
     }
     if (!converged && M.tid == 0) atomicExch(T.status, (int)QR_ENOCONV);
 
-    // ---- sigma, descending order (ties by index), truncation on the device
+    // ---- sigma, descending order (ranks_before), truncation on the device
     team_norms(M, B, rows, k, nrm, sig);
     for (int j = tid; j < k; j += blockDim.x) {
       int rank = 0;
       const double v = sig[j];
-      for (int i = 0; i < k; i++) rank += (sig[i] > v) || (sig[i] == v && i < j);
+      for (int i = 0; i < k; i++) rank += ranks_before(sig[i], i, v, j);
       perm[rank] = j;
       srt[rank] = v;
     }

@@ -33,6 +33,15 @@ template <typename C> __host__ __device__ inline C cmulc(C a, C b) {
 template <typename C> __host__ __device__ inline C cconj(C a) { C r; r.x = a.x; r.y = -a.y; return r; }
 template <typename C, typename T> __host__ __device__ inline C cscale(C a, T s) { C r; r.x = a.x * s; r.y = a.y * s; return r; }
 
+// Key a of index i comes before key b of index j: descending, ties by index, NaN before every number.  A total
+// order, so that ranks (the number of keys before a key) are a permutation whatever the keys hold: gathers go
+// through them, and a NaN stands first, where the caller's test of the largest value finds it.
+__host__ __device__ inline bool ranks_before(double a, int i, double b, int j) {
+  const bool na = a != a, nb = b != b;
+  if (na != nb) return na;
+  return a > b || ((na || a == b) && i < j);
+}
+
 // ---- error plumbing ----------------------------------------------------------------------------
 void set_error(const std::string& msg);
 int fail(int code, const std::string& msg);

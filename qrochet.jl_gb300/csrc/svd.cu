@@ -1525,16 +1525,13 @@ __global__ void col_norms_k(const C* __restrict__ B, long ldb, int m, int n, dou
   if (lane == 0) nrm[j] = sqrt(acc);
 }
 
-// perm[rank] = j, descending by key (ties by index), one thread per element
+// perm[rank] = j in the order of ranks_before, one thread per element
 __global__ void rank_sort_k(const double* __restrict__ key, int n, int* __restrict__ perm, double* __restrict__ sorted) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double ki = key[i];
   int rank = 0;
-  for (int j = 0; j < n; j++) {
-    double kj = key[j];
-    rank += (kj > ki) || (kj == ki && j < i);
-  }
+  for (int j = 0; j < n; j++) rank += ranks_before(key[j], j, ki, i);
   perm[rank] = i;
   if (sorted) sorted[rank] = ki;
 }
@@ -2549,6 +2546,8 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
       if (!hn) return fail(QR_ENOMEM, "page-locked host scratch");
       QR_CUDA(cudaMemcpyAsync(hn, nrm, sizeof(double) * k, cudaMemcpyDeviceToHost, s));
       QR_CUDA(cudaStreamSynchronize(s));
+      for (int j = 0; j < k; j++)  // (a NaN would break the order that std::sort needs)
+        if (!std::isfinite(hn[j])) return fail(QR_ENOCONV, "non-finite singular values");
       std::vector<double> sn(hn, hn + k);
       std::sort(sn.begin(), sn.end(), std::greater<double>());
       *count = 0;

@@ -242,6 +242,16 @@ int qr_test_qr(int m, int n, const double* A, double* Q, double* R, double* ms) 
   return QR_OK;
 } QR_ABI_CATCH
 
+int qr_test_rank_order(const double* keys, int n, int* perm) try {
+  if (n < 0 || (n > 0 && (!keys || !perm))) return fail(QR_EINVAL, "bad keys");
+  for (int i = 0; i < n; i++) {
+    int rank = 0;
+    for (int j = 0; j < n; j++) rank += ranks_before(keys[j], j, keys[i], i);
+    if (rank < n) perm[rank] = i;
+  }
+  return QR_OK;
+} QR_ABI_CATCH
+
 int qr_test_host_exception(int kind) try {
   struct NotStd {};
   if (kind == 0) throw std::bad_alloc();

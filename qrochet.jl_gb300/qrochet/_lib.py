@@ -122,6 +122,7 @@ SIGNATURES = {
     "qr_test_schedule_pairs": [C.c_void_p, C.c_void_p, _I, _I, C.c_void_p, C.c_void_p, C.POINTER(C.c_long),
                                C.POINTER(C.c_int)],
     "qr_test_qr": [_I, _I, _PD, _PD, _PD, _PD],
+    "qr_test_rank_order": [_PD, _I, C.POINTER(C.c_int)],
     "qr_test_host_exception": [_I],
 }
 
