@@ -249,6 +249,7 @@ int refine(cudaStream_t s, SvdWork* w, const double2* A, int rows, int k, double
   for (int step = 0; step < kRefineMaxSteps + 8; step++) {
     give_up = give_up || step >= kRefineMaxSteps;
     QR_TRY(zgemm_graded(s, rows, k, k, A, rows, X, k, B, rows));
+    const bool swept = pending;  // B and X have been through double-float: one more step before they are results
     if (pending) {
       long listed = 0;
       QR_TRY(df_listed(s, w, B, rows, k, X, width, nv, 32.0 * sqrt((double)rows) * Eps<double>::v, smax_d, k0, &listed));
@@ -274,7 +275,7 @@ int refine(cudaStream_t s, SvdWork* w, const double2* A, int rows, int k, double
       fprintf(stderr, "[qr] refine %dx%d step %d: %u pairs, largest tangent %.2e, column sum %.2e; |I - X^H X| %.2e\n", rows,
               k, step, fail_pairs, tmax, tsum, rmax);
     if (!(rmax < 0.5f) || !(tmax <= 1.f)) return fail(QR_ENOCONV, "SVD refinement: vectors far from unitary");
-    if (rmax < 1e-14f && (fail_pairs == 0 || give_up)) {
+    if (rmax < 1e-14f && !swept && (fail_pairs == 0 || give_up)) {
       *done = give_up ? 0 : 1;
       return QR_OK;
     }
