@@ -30,6 +30,7 @@
 // of one tile.  A tile grid that would leave SMs idle splits K over a cluster of up to 8 CTAs, which add
 // their integer sums through distributed shared memory.
 #include <cuda_bf16.h>
+#include <algorithm>
 #include <climits>
 #include <map>
 #include "kernels.cuh"
@@ -591,46 +592,70 @@ size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 // Largest K of the integer sums (hi stays below 2^51) and the largest plane rows TMA addresses.
 bool zgemm_oz_fits(int M, int N, int K) { return K <= (1 << 20) && M <= (1 << 28) && N <= (1 << 28); }
 
+// Workspace for slices at a time: a batch that needs more goes through in runs of whole entries.
+constexpr size_t OZ_ROOM = (size_t)1 << 30;
+constexpr int OZ_NO_ROOM = -1;  // oz_run: the slices found no memory, nothing was launched
+
 static int oz_run(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
                   const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk,
-                  int herm, int eq_a, int sub) {
+                  int herm, int eq_a, int sub, size_t room = OZ_ROOM) {
+  if (room == 0) return OZ_NO_ROOM;
   const bool bshared = sB == 0 || batch == 1;
-  const int bb = bshared ? 1 : batch;
   const int ntm = (M + 63) / 64, ntn = (N + OZ_BN - 1) / OZ_BN, Kh = (K + 15) / 16 * 16;
   const long Kp = 2L * Kh, arows = 128L * ntm, brows = (long)OZ_BN * ntn;
   const long apl = arows * Kp, bpl = brows * Kp;
-  const size_t ab = up256((size_t)batch * OZ_S * apl * 2), bbt = up256((size_t)bb * OZ_S * bpl * 2);
-  const size_t ea = up256(sizeof(int) * (size_t)batch * M), eb = up256(sizeof(int) * (size_t)bb * N);
-  const size_t gb = up256(sizeof(int) * (size_t)bb * K);
+  // bytes of one entry of A, and of B with its scales along K
+  const size_t abytes = (size_t)OZ_S * apl * 2 + sizeof(int) * (size_t)M;
+  const size_t bbytes = (size_t)OZ_S * bpl * 2 + sizeof(int) * ((size_t)N + K);
+  const size_t fixed = bshared ? bbytes : 0, each = abytes + (bshared ? 0 : bbytes);
+  int run_len = (int)std::min<size_t>(batch, std::max<size_t>(1, room > fixed ? (room - fixed) / each : 1));
   char* ws = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&ws, ab + bbt + ea + eb + gb, s);
-  if (e != cudaSuccess) return fail(QR_ENOMEM, std::string("GEMM slices: ") + cudaGetErrorString(e));
-  OzPlain pl;
-  pl.K = K;
-  const bool an = opA == OP_N || opA == OP_R, bn = opB == OP_N || opB == OP_R;
-  pl.a = {A, an ? 1 : lda, an ? lda : 1, sA, M, opA == OP_C || opA == OP_R, eq_a ? -1 : 1, dk, (__nv_bfloat16*)ws,
-          (int*)(ws + ab + bbt), apl};
-  pl.b = {B, bn ? ldb : 1, bn ? 1 : ldb, bshared ? 0 : sB, N, opB == OP_C || opB == OP_R, eq_a ? 1 : -1, nullptr,
-          (__nv_bfloat16*)(ws + ab), (int*)(ws + ab + bbt + ea), bpl};
+  int bb = 1;
+  size_t ab = 0, bbt = 0, ea = 0, eb = 0;
+  for (;;) {
+    bb = bshared ? 1 : run_len;
+    ab = up256((size_t)run_len * OZ_S * apl * 2);
+    bbt = up256((size_t)bb * OZ_S * bpl * 2);
+    ea = up256(sizeof(int) * (size_t)run_len * M);
+    eb = up256(sizeof(int) * (size_t)bb * N);
+    const cudaError_t e = cudaMallocAsync((void**)&ws, ab + bbt + ea + eb + sizeof(int) * (size_t)bb * K, s);
+    if (e == cudaSuccess) break;
+    if (e != cudaErrorMemoryAllocation) return cuda_fail(e, "GEMM slices");
+    (void)cudaGetLastError();  // not an error of the next launch
+    if (run_len == 1) return OZ_NO_ROOM;
+    run_len = (run_len + 1) / 2;
+  }
   int* g = (int*)(ws + ab + bbt + ea + eb);
-  auto run = [&]() -> int {
-    oz_kmax_k<<<dim3(ceil_div(K, KMAX_K), 1, bb), 256, 0, s>>>(eq_a ? pl.a : pl.b, K, g);
-    QR_CHECK_LAUNCH("oz_kmax_k");
+  const bool an = opA == OP_N || opA == OP_R, bn = opB == OP_N || opB == OP_R;
+  // entries z0 .. z0 + nz - 1
+  auto run = [&](int z0, int nz) -> int {
+    const int nb = bshared ? 1 : nz;
+    const bool slice_b = !bshared || z0 == 0;
+    OzPlain pl;
+    pl.K = K;
+    pl.a = {A + z0 * sA, an ? 1 : lda, an ? lda : 1, sA, M, opA == OP_C || opA == OP_R, eq_a ? -1 : 1, dk,
+            (__nv_bfloat16*)ws, (int*)(ws + ab + bbt), apl};
+    pl.b = {bshared ? B : B + z0 * sB, bn ? ldb : 1, bn ? 1 : ldb, bshared ? 0 : sB, N, opB == OP_C || opB == OP_R,
+            eq_a ? 1 : -1, nullptr, (__nv_bfloat16*)(ws + ab), (int*)(ws + ab + bbt + ea), bpl};
+    if (slice_b) {
+      oz_kmax_k<<<dim3(ceil_div(K, KMAX_K), 1, nb), 256, 0, s>>>(eq_a ? pl.a : pl.b, K, g);
+      QR_CHECK_LAUNCH("oz_kmax_k");
+    }
     // few rows: 4 per CTA so that the pass still covers the SMs; else 16
-    const long rows = (long)M * batch + (long)N * bb;
+    const long rows = (long)M * nz + (slice_b ? (long)N * nb : 0);
     const int rb = rows <= 2432 ? 4 : 16;
     const int nba = (M + rb - 1) / rb, nbb = (N + rb - 1) / rb;
-    const unsigned grid = (unsigned)((long)nba * batch + (long)nbb * bb);
+    const unsigned grid = (unsigned)((long)nba * nz + (slice_b ? (long)nbb * nb : 0));
     const long gs = bshared ? 0 : K;
-    if (rb == 4) oz_digits_k<4><<<grid, 256, 0, s>>>(pl.a, pl.b, K, Kh, g, gs, nba, nbb, batch);
-    else oz_digits_k<16><<<grid, 256, 0, s>>>(pl.a, pl.b, K, Kh, g, gs, nba, nbb, batch);
+    if (rb == 4) oz_digits_k<4><<<grid, 256, 0, s>>>(pl.a, pl.b, K, Kh, g, gs, nba, nbb, nz);
+    else oz_digits_k<16><<<grid, 256, 0, s>>>(pl.a, pl.b, K, Kh, g, gs, nba, nbb, nz);
     QR_CHECK_LAUNCH("oz_digits_k");
     CUtensorMap ma, mb;
-    QR_TRY(oz_map_make(&ma, ws, Kp, arows, (long)OZ_S * batch, OZ_BM));
-    QR_TRY(oz_map_make(&mb, ws + ab, Kp, brows, (long)OZ_S * bb, OZ_BN));
+    QR_TRY(oz_map_make(&ma, ws, Kp, arows, (long)OZ_S * nz, OZ_BM));
+    QR_TRY(oz_map_make(&mb, ws + ab, Kp, brows, (long)OZ_S * nb, OZ_BN));
     QR_TRY(set_func_attr_once((const void*)zgemm_oz_k, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
     const int nk = (int)(Kp / OZ_BK);
-    const long tiles = herm ? (long)ntm * (ntm + 1) / 2 : (long)ntm * ntn * batch;
+    const long tiles = herm ? (long)ntm * (ntm + 1) / 2 : (long)ntm * ntn * nz;
     // K split over a cluster: the split with the fewest (waves x stages per CTA), a CTA's fixed cost
     // counted as 5 stages and a split's as 2 more
     int cs = 1;
@@ -657,18 +682,28 @@ static int oz_run(cudaStream_t s, int opA, int opB, int M, int N, int K, const d
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    QR_CUDA(cudaLaunchKernelEx(&cfg, zgemm_oz_k, ma, mb, C, ldc, sC, M, N, nk, bshared ? 1 : 0, ntm, ntn, cs, herm, sub, pl));
+    QR_CUDA(cudaLaunchKernelEx(&cfg, zgemm_oz_k, ma, mb, C + z0 * sC, ldc, sC, M, N, nk, bshared ? 1 : 0, ntm, ntn, cs,
+                               herm, sub, pl));
     count_launch();
     return QR_OK;
   };
-  const int rc = run();
+  int rc = QR_OK;
+  for (int z0 = 0; z0 < batch && !rc; z0 += run_len) rc = run(z0, std::min(run_len, batch - z0));
   cudaFreeAsync(ws, s);
   return rc;
 }
 
+// (where the slices find no memory, the products run on the CUDA cores, which need none)
+int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
+             const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk, size_t room) {
+  const int rc = oz_run(s, opA, opB, M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, dk, 0, 0, 0, room);
+  if (rc != OZ_NO_ROOM) return rc;
+  return zgemm_spread(s, opA, opB, M, N, K, make_double2(1.0, 0.0), A, lda, sA, B, ldb, sB, make_double2(0.0, 0.0), C, ldc,
+                      sC, batch, dk);
+}
 int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
              const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk) {
-  return oz_run(s, opA, opB, M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, dk, 0, 0, 0);
+  return zgemm_oz(s, opA, opB, M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, dk, OZ_ROOM);
 }
 
 // C = A B (M x K, K x N) for an A whose columns spread over decades: the scaling along K equilibrates A's
@@ -680,7 +715,10 @@ int zgemm_graded(cudaStream_t s, int M, int N, int K, const double2* A, long lda
     return zgemm(s, OP_N, OP_N, M, N, K, make_double2(1.0, 0.0), A, lda, 0, B, ldb, 0, make_double2(0.0, 0.0), C, ldc, 0,
                  1, nullptr);
   const int pr = prof_begin(s, PK_ZGEMM, 8.0 * work, 16.0 * ((double)M * K + (double)K * N + (double)M * N));
-  const int rc = oz_run(s, OP_N, OP_N, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, nullptr, 0, 1, 0);
+  int rc = oz_run(s, OP_N, OP_N, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, nullptr, 0, 1, 0);
+  if (rc == OZ_NO_ROOM)
+    rc = zgemm_spread(s, OP_N, OP_N, M, N, K, make_double2(1.0, 0.0), A, lda, 0, B, ldb, 0, make_double2(0.0, 0.0), C, ldc,
+                      0, 1, nullptr);
   prof_end(s, pr);
   return rc;
 }
@@ -691,10 +729,12 @@ int zgemm_sub(cudaStream_t s, int M, int N, int K, const double2* A, long lda, c
   if (M <= 0 || N <= 0 || K <= 0) return QR_OK;
   const double work = (double)M * N * K;
   const int pr = prof_begin(s, PK_ZGEMM, 8.0 * work, 16.0 * ((double)M * K + (double)K * N + 2.0 * M * N));
-  const int rc = work >= OZ_MIN_WORK && zgemm_oz_fits(M, N, K)
-                     ? oz_run(s, OP_N, OP_N, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, nullptr, 0, 0, 1)
-                     : zgemm_spread(s, OP_N, OP_N, M, N, K, make_double2(-1.0, 0.0), A, lda, 0, B, ldb, 0,
-                                    make_double2(1.0, 0.0), C, ldc, 0, 1, nullptr);
+  int rc = OZ_NO_ROOM;
+  if (work >= OZ_MIN_WORK && zgemm_oz_fits(M, N, K))
+    rc = oz_run(s, OP_N, OP_N, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, nullptr, 0, 0, 1);
+  if (rc == OZ_NO_ROOM)
+    rc = zgemm_spread(s, OP_N, OP_N, M, N, K, make_double2(-1.0, 0.0), A, lda, 0, B, ldb, 0, make_double2(1.0, 0.0), C, ldc,
+                      0, 1, nullptr);
   prof_end(s, pr);
   return rc;
 }
@@ -705,9 +745,10 @@ int zherk(cudaStream_t s, int n, int K, const double2* A, long lda, double2* C, 
   if (n <= 0) return QR_OK;
   const double work = (double)n * n * K;
   const int pr = prof_begin(s, PK_ZGEMM, 4.0 * work, 16.0 * ((double)n * K + (double)n * n));
-  const int rc = work >= OZ_MIN_WORK && zgemm_oz_fits(n, n, K)
-                     ? oz_run(s, OP_C, OP_N, n, n, K, A, lda, 0, A, lda, 0, C, ldc, 0, 1, nullptr, 1, 0, 0)
-                     : zherk_spread(s, n, K, A, lda, C, ldc);
+  int rc = OZ_NO_ROOM;
+  if (work >= OZ_MIN_WORK && zgemm_oz_fits(n, n, K))
+    rc = oz_run(s, OP_C, OP_N, n, n, K, A, lda, 0, A, lda, 0, C, ldc, 0, 1, nullptr, 1, 0, 0);
+  if (rc == OZ_NO_ROOM) rc = zherk_spread(s, n, K, A, lda, C, ldc);
   prof_end(s, pr);
   return rc;
 }

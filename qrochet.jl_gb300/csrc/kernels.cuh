@@ -21,10 +21,14 @@ int zgemm_spread(cudaStream_t s, int opA, int opB, int M, int N, int K, double2 
                  const double* dk);
 
 // ---- gemm_oz.cu: C[b] = op(A[b]) diag(dk) op(B[b]) at FP64 accuracy on the tcgen05 tensor cores
-// (exact products of 8-bit slices); sB = 0 shares B.  Slices in a stream-ordered allocation.
+// (exact products of 8-bit slices); sB = 0 shares B.  Slices in a stream-ordered allocation: 56 bytes an entry
+// of A and 28 of B, a batch in runs of at most 1 GiB; zgemm_spread where there is no memory for them.  The second
+// form takes the bytes of a run (0: as if there were no memory).
 bool zgemm_oz_fits(int M, int N, int K);
 int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
              const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk);
+int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
+             const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk, size_t room);
 
 int zherk_spread(cudaStream_t s, int n, int K, const double2* A, long lda, double2* C, long ldc);
 // C = A B for an A whose columns spread over decades (see gemm_oz.cu)

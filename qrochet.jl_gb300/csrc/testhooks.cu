@@ -110,6 +110,39 @@ int qr_test_zgemm_tc(int opA, int opB, int M, int N, int K, int batch, const dou
   return QR_OK;
 } QR_ABI_CATCH
 
+// C[b] = op(A[b]) op(B[b]) on exact slices (gemm_oz.cu) with `room` bytes of workspace at a time; A and B hold
+// `batch` matrices at strides lda * columns (b_shared: one B), C at stride M * N.
+int qr_test_zgemm_oz(int opA, int opB, int M, int N, int K, int batch, int b_shared, const double* A, long lda,
+                     const double* B, long ldb, double* C, uint64_t room, double* ms) try {
+  if (M <= 0 || N <= 0 || K <= 0 || batch < 1 || !zgemm_oz_fits(M, N, K)) return fail(QR_EINVAL, "bad gemm shape");
+  const bool an = opA == OP_N || opA == OP_R, bn = opB == OP_N || opB == OP_R;
+  if (lda < (an ? M : K) || ldb < (bn ? K : N)) return fail(QR_EINVAL, "bad leading dimension");
+  const long sA = lda * (an ? K : M), sB = b_shared ? 0 : ldb * (bn ? N : K), sC = (long)M * N;
+  Dev dA, dB, dC;
+  QR_TRY(up(dA, A, (size_t)sA * batch));
+  QR_TRY(up(dB, B, (size_t)ldb * (bn ? N : K) * (b_shared ? 1 : batch)));
+  QR_TRY(up(dC, nullptr, (size_t)sC * batch));
+  cudaEvent_t e0, e1;
+  cudaEventCreate(&e0);
+  cudaEventCreate(&e1);
+  int rc = QR_OK;
+  float t = 0;
+  for (int it = 0; it < 2 && !rc; it++) {  // the second run is the timed one
+    cudaEventRecord(e0);
+    rc = zgemm_oz(0, opA, opB, M, N, K, (double2*)dA.p, lda, sA, (double2*)dB.p, ldb, sB, (double2*)dC.p, M, sC, batch,
+                  nullptr, (size_t)room);
+    cudaEventRecord(e1);
+    cudaEventSynchronize(e1);
+    cudaEventElapsedTime(&t, e0, e1);
+  }
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  QR_TRY(rc);
+  QR_CUDA(cudaMemcpy(C, dC.p, sizeof(double2) * sC * batch, cudaMemcpyDeviceToHost));
+  if (ms) *ms = t;
+  return QR_OK;
+} QR_ABI_CATCH
+
 // Double-float GEMM (gemm_df.cu) through FP64 host matrices: inputs are split into (hi, lo) FP32
 // pairs on the device, the result converted back (mode 1 returns the FP32 value I - op(A) B).
 int qr_test_zgemm_df(int mode, int opA, int M, int N, int K, const double* A, long lda, const double* B, long ldb,
