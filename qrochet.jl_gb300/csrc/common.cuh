@@ -35,11 +35,19 @@ template <typename C, typename T> __host__ __device__ inline C cscale(C a, T s) 
 
 // Key a of index i comes before key b of index j: descending, ties by index, NaN before every number.  A total
 // order, so that ranks (the number of keys before a key) are a permutation whatever the keys hold: gathers go
-// through them, and a NaN stands first, where the caller's test of the largest value finds it.
+// through them, and a NaN stands first, where the caller's test of the largest value finds it.  Integer
+// instructions only: a warp's FP64 comparison occupies the pipe for 16 cycles, and ranking 256 to 2048 keys with
+// them took 1 - 2% of a gate step.
+__host__ __device__ inline unsigned long long rank_key(double x) {
+  union { double d; unsigned long long u; } v = {x};
+  const unsigned long long sign = 1ull << 63, mag = v.u & ~sign;
+  if (mag > 0x7ff0000000000000ull) return ~0ull;
+  if (mag == 0) return sign;
+  return v.u & sign ? ~v.u : v.u | sign;
+}
 __host__ __device__ inline bool ranks_before(double a, int i, double b, int j) {
-  const bool na = a != a, nb = b != b;
-  if (na != nb) return na;
-  return a > b || ((na || a == b) && i < j);
+  const unsigned long long ka = rank_key(a), kb = rank_key(b);
+  return ka > kb || (ka == kb && i < j);
 }
 
 // ---- error plumbing ----------------------------------------------------------------------------

@@ -11,7 +11,7 @@ NAN, INF = float("nan"), float("inf")
 
 
 @pytest.mark.parametrize("keys", [[], [1.0], [NAN], [2.0, 2.0, 2.0], [NAN] * 5, [1.0, NAN, 3.0, NAN, 3.0, 0.0],
-                                  [INF, NAN, INF, 0.0, -0.0, 5.0], [0.0] * 7 + [NAN], [NAN] + [1.0] * 40])
+                                  [INF, NAN, INF, 0.0, -0.0, 5.0], [-1.0, 2.0, -INF, -3.0, NAN, 0.0], [0.0] * 7 + [NAN], [NAN] + [1.0] * 40])
 def test_ranks_are_a_permutation(keys):
     k = np.array(keys, dtype=np.float64)
     perm = np.full(k.size + 1, -1, dtype=np.int32)
