@@ -104,7 +104,7 @@ int zherk_spread(cudaStream_t s, int n, int K, const double2* A, long lda, doubl
 
 int zgemm(cudaStream_t s, int opA, int opB, int M, int N, int K, double2 alpha,
           const double2* A, long lda, long sA, const double2* B, long ldb, long sB,
-          double2 beta, double2* C, long ldc, long sC, int batch, const double* dk) {
+          double2 beta, double2* C, long ldc, long sC, int batch, const double* dk, bool normwise) {
   if (M <= 0 || N <= 0 || batch <= 0) return QR_OK;
   if (opA < 0 || opA > 3 || opB < 0 || opB > 3) return fail(QR_EINVAL, "zgemm: bad op");
   const double work = (double)M * N * K * batch;
@@ -112,7 +112,7 @@ int zgemm(cudaStream_t s, int opA, int opB, int M, int N, int K, double2 alpha,
   const int pr = prof_begin(s, PK_ZGEMM, 8.0 * work, by);
   const bool plain = alpha.x == 1.0 && alpha.y == 0.0 && beta.x == 0.0 && beta.y == 0.0;
   const int rc = plain && work >= OZ_MIN_WORK && zgemm_oz_fits(M, N, K)
-                     ? zgemm_oz(s, opA, opB, M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, dk)
+                     ? zgemm_oz(s, opA, opB, M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, dk, !normwise)
                      : zgemm_spread(s, opA, opB, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, dk);
   prof_end(s, pr);
   return rc;

@@ -23,6 +23,14 @@
 //     changes a bit of an exact sum.  The epilogue rounds hi + lo once to FP64.
 // The first neglected products (d = 7) lie at 2^-56 of the row and column maxima.  Rows or columns that
 // hold an infinity or NaN are recomputed by plain FP64 dot products in the epilogue.
+// So the error is relative to the maxima of a row and a column, and an element whose products are all far below
+// them (entries over many decades, the large ones of the row against the small ones of the column) would lose
+// digits that an FP64 product keeps.  With the guard an eighth accumulator sums the products of the leading
+// bytes' absolute values, sum |a||b| in units of 2^-14 of the two maxima, and elements where it is below
+// OZ_LEAST sqrt(K) are formed in FP64 instead, a warp each.  Above it the rounding of the slices, ~0.1 sqrt(2 K) 2^-55 of
+// the maxima, is at most ~2e-15 of sum |a||b|, about what an FP64 sum of 256 terms commits.  (Entries exp(6 x), x
+// normal: 2e-9 - 5e-8 of sum |a||b| without the guard.)  Products whose error the caller needs relative to norms only
+// (orthogonal factors, refinement, QR updates) do without: an identity's zeros would all be formed in FP64.
 //
 // Bound: the MMAs, 28 products x 2 per 32 k' (about 51 cycles each: at N = 64 shared memory feeds the
 // tensor core 6 KB per MMA in 48); loads alone take 60% of that.  2048^3: 1.77 ms (39 TFLOP/s
@@ -33,6 +41,7 @@
 #include <algorithm>
 #include <climits>
 #include <map>
+#include <tuple>
 #include "kernels.cuh"
 #include "prof.cuh"
 #include "tcgen05.cuh"
@@ -51,12 +60,18 @@ constexpr int OZ_DH = 4;                      // accumulators of H
 __device__ __forceinline__ bool oz_drain_h(int n, int last) { return n % 8 == 7 || n == last; }
 __device__ __forceinline__ bool oz_drain_l(int n, int last) { return n % 32 == 3 || n == last; }
 constexpr int OZ_AT = OZ_BM * OZ_BK * 2, OZ_BT = OZ_BN * OZ_BK * 2;  // bytes of one slice tile
-constexpr int OZ_STAGE = OZ_S * (OZ_AT + OZ_BT);
+// with the guard an eighth plane: the leading bytes' absolute values
+constexpr int oz_planes(bool guard) { return OZ_S + (guard ? 1 : 0); }
+constexpr int oz_stage(bool guard) { return oz_planes(guard) * (OZ_AT + OZ_BT); }
 constexpr int OZ_EPI_WARPS = 16;              // four per TMEM lane quarter, 16 columns each
 constexpr int OZ_THREADS = 32 * (2 + OZ_EPI_WARPS);  // warp 0 TMA, warp 1 MMA + TMEM, then the drain
-constexpr int OZ_SMEM = OZ_STAGES * OZ_STAGE + 1024 + 256;
+constexpr int oz_smem(bool guard) { return OZ_STAGES * oz_stage(guard) + 1024 + 256; }
 constexpr int OZ_TMEM_COLS = 512;
-static_assert(OZ_BM * OZ_BN * 16 <= OZ_STAGES * OZ_STAGE, "the integer sums reuse the stage memory");
+// after the products the stage memory holds the integer sums and, with the guard, its sums and a list of elements
+constexpr int OZ_SUMS = OZ_BM * OZ_BN * 16, OZ_GSUMS = OZ_BM * OZ_BN * 4, OZ_LIST = 16 + 64 * OZ_BN * 2;
+static_assert(OZ_SUMS <= OZ_STAGES * oz_stage(false), "the integer sums reuse the stage memory");
+static_assert(OZ_SUMS + OZ_GSUMS + OZ_LIST <= OZ_STAGES * oz_stage(true), "so do the guard's");
+static_assert(oz_smem(true) <= 227 * 1024, "two stages of eight planes");
 constexpr int OZ_BAD = INT_MIN;               // exponent of a row that holds an infinity or NaN
 constexpr int OZ_ZERO = INT_MIN / 2;          // of a row of zeros
 
@@ -147,7 +162,8 @@ __device__ __forceinline__ uint2 oz_slice4(const unsigned long long (&v)[4], int
 // RB rows of one operand per CTA: exponents, then digits through a shared tile of 1024 / RB k's.
 template <int RB>
 __global__ void __launch_bounds__(256) oz_digits_k(const OzOperand a, const OzOperand b, int K, int Kh,
-                                                   const int* __restrict__ g, long gstride, int nba, int nbb, int batch) {
+                                                   const int* __restrict__ g, long gstride, int nba, int nbb, int batch,
+                                                   int planes) {
   constexpr int KC = 1024 / RB, KL = 256 / RB;
   __shared__ double2 tile[RB][KC + 1];
   __shared__ int emax[RB];
@@ -179,7 +195,7 @@ __global__ void __launch_bounds__(256) oz_digits_k(const OzOperand a, const OzOp
   const int r = tid / (KC / 4), k4 = (tid % (KC / 4)) * 4;
   const int i = i0 + r, E = min(emax[r], 1 << 20);
   const long Kp = 2L * Kh;
-  __nv_bfloat16* out = o.out + (long)z * OZ_S * o.plane;
+  __nv_bfloat16* out = o.out + (long)z * planes * o.plane;
   for (int k0 = 0; k0 < Kh; k0 += KC) {
     __syncthreads();
 #pragma unroll
@@ -201,11 +217,16 @@ __global__ void __launch_bounds__(256) oz_digits_k(const OzOperand a, const OzOp
       vi[u] = oz_fixed(v.y, sh);
     }
 #pragma unroll
-    for (int s = 0; s < OZ_S; s++) {
-      const uint2 re = oz_slice4(vr, s), im = oz_slice4(vi, s);
+    for (int s = 0; s <= OZ_S; s++) {
+      if (s == OZ_S && planes == OZ_S) break;
+      uint2 re = oz_slice4(vr, s % OZ_S), im = oz_slice4(vi, s % OZ_S);
+      if (s == OZ_S) {  // the guard's plane
+        re = make_uint2(re.x & 0x7fff7fffu, re.y & 0x7fff7fffu);
+        im = make_uint2(im.x & 0x7fff7fffu, im.y & 0x7fff7fffu);
+      }
       __nv_bfloat16* pl = out + s * o.plane;
       if (is_a) {
-        const uint2 ng = make_uint2(im.x ^ 0x80008000u, im.y ^ 0x80008000u);
+        const uint2 ng = s == OZ_S ? im : make_uint2(im.x ^ 0x80008000u, im.y ^ 0x80008000u);
         const long rre = (long)(i / 64) * 128 + (i % 64), rim = rre + 64;
         *reinterpret_cast<uint2*>(pl + rre * Kp + k) = re;
         *reinterpret_cast<uint2*>(pl + rre * Kp + Kh + k) = ng;
@@ -284,6 +305,11 @@ __device__ __forceinline__ uint32_t oz_map(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
+__device__ __forceinline__ float oz_ldf_remote(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ longlong2 oz_ld_remote(uint32_t addr) {
   longlong2 v;
   asm volatile("ld.shared::cluster.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(addr) : "memory");
@@ -303,16 +329,21 @@ __device__ __forceinline__ double oz_double(long long hi, long long lo, int e) {
   return scalbn(scalbn(r, e / 2), e - e / 2);
 }
 
-// what the epilogue needs to recompute an element in plain FP64
+// The least sum of the guard's products per sqrt(K).  Gaussian entries give ~1000 K; rows with one entry that
+// counts (a diagonal environment) ~127 times the other operand's leading byte.
+constexpr float OZ_LEAST = 32.f;
+// what the epilogue needs to form an element in plain FP64
 struct OzPlain {
   OzOperand a, b;
   int K;
 };
 
+template <bool GUARD>
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     zgemm_oz_k(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, double2* __restrict__ C,
                long ldc, long sC, int M, int N, int nk, int bshared, int ntm, int ntn, int cs, int herm,
-               int sub, const OzPlain plain) {
+               int sub, float least, const OzPlain plain) {
+  constexpr int NP = oz_planes(GUARD), OZ_STAGE = oz_stage(GUARD);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OZ_STAGES * OZ_STAGE);
@@ -359,10 +390,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   longlong2* sums = reinterpret_cast<longlong2*>(smem);  // [column][row] (hi, lo), once the stages are free
+  float* gsums = reinterpret_cast<float*>(smem + OZ_SUMS);                       // [column][row], with the guard
+  unsigned* nlist = reinterpret_cast<unsigned*>(smem + OZ_SUMS + OZ_GSUMS);      // elements to form in FP64
+  uint16_t* list = reinterpret_cast<uint16_t*>(smem + OZ_SUMS + OZ_GSUMS + 16);
 
   if (warp == 0) {
     if (elect_one()) {
-      const int arow = tm * OZ_BM, brow = tn * OZ_BN, apl = OZ_S * z, bpl = bshared ? 0 : OZ_S * z;
+      const int arow = tm * OZ_BM, brow = tn * OZ_BN, apl = NP * z, bpl = bshared ? 0 : NP * z;
       int issued[OZ_STAGES] = {0, 0};
       bool ok = true;
       for (int kb = kb0; kb < kb1; kb++) {
@@ -373,9 +407,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         }
         uint8_t* st = smem + s * OZ_STAGE;
         mbar_expect_tx(full + s, OZ_STAGE);
-        for (int sl = 0; sl < OZ_S; sl++) {
+        for (int sl = 0; sl < NP; sl++) {
           tma_load_3d(st + sl * OZ_AT, &tmA, kb * OZ_BK, arow, apl + sl, full + s);
-          tma_load_3d(st + OZ_S * OZ_AT + sl * OZ_BT, &tmB, kb * OZ_BK, brow, bpl + sl, full + s);
+          tma_load_3d(st + NP * OZ_AT + sl * OZ_BT, &tmB, kb * OZ_BK, brow, bpl + sl, full + s);
         }
         issued[s]++;
       }
@@ -395,8 +429,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         const int s = n % OZ_STAGES;
         if (*abort_flag || !mbar_wait(full + s, (n / OZ_STAGES) & 1u, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint64_t da = oz_desc(smem_u32(smem + s * OZ_STAGE)), db = oz_desc(smem_u32(smem + s * OZ_STAGE) + OZ_S * OZ_AT);
+        const uint64_t da = oz_desc(smem_u32(smem + s * OZ_STAGE)), db = oz_desc(smem_u32(smem + s * OZ_STAGE) + NP * OZ_AT);
         const uint32_t dh = (uint32_t)(da >> 32);
+        if (GUARD) {  // into the columns behind the seven accumulators, drained once, with the last chunks
+#pragma unroll
+          for (int j = 0; j < OZ_BK / 16; j++)
+            oz_mma(tmem + OZ_S * OZ_BN, (uint32_t)da + (uint32_t)((OZ_S * OZ_AT + 32 * j) >> 4),
+                   (uint32_t)db + (uint32_t)((OZ_S * OZ_BT + 32 * j) >> 4), dh, n > 0 || j > 0 ? 1u : 0u);
+        }
         // the group that is being drained comes second
         for (int o = 0; o < 2; o++) {
           const bool low = first[1] ? o == 1 : o == 0;
@@ -479,6 +519,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       longlong2* o = sums + (long)(part * OZ_EC) * OZ_BM + 32 * q + lane;
 #pragma unroll
       for (int j = 0; j < OZ_EC; j++) o[j * OZ_BM] = make_longlong2(hi[j], lo[j]);
+      if (GUARD) {
+        float v[16];
+        oz_tmem_ld16(ta + OZ_S * OZ_BN, v);
+        float* p = gsums + (part * OZ_EC) * OZ_BM + 32 * q + lane;
+#pragma unroll
+        for (int j = 0; j < OZ_EC; j++) p[j * OZ_BM] = v[j];
+        if (warp == 2 && lane == 0) *nlist = 0;
+      }
     }
   }
   tc_fence_before();
@@ -488,7 +536,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   if (warp == 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(OZ_TMEM_COLS) : "memory");
   // this CTA rounds and stores 64 / cs of the tile's columns
-  const uint32_t sbase = smem_u32(sums), fbase = smem_u32(const_cast<const uint32_t*>(abort_flag));
+  const uint32_t sbase = smem_u32(sums), gbase = smem_u32(gsums), fbase = smem_u32(const_cast<const uint32_t*>(abort_flag));
   bool bad = false;
   for (int r = 0; r < cs; r++) {
     uint32_t f;
@@ -514,6 +562,17 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     } else if (xa == OZ_ZERO || xb == OZ_ZERO) {
       out.x = out.y = 0.0;
     } else {
+      if (GUARD) {
+        float p = 0.f;
+        for (int r = 0; r < cs; r++) {
+          const uint32_t at = oz_map(gbase + (uint32_t)(c * OZ_BM + i) * 4u, r);
+          p += oz_ldf_remote(at) + oz_ldf_remote(at + 64 * 4);
+        }
+        if (p < least) {
+          list[atomicAdd(nlist, 1u)] = (uint16_t)e;
+          continue;
+        }
+      }
       longlong2 re = make_longlong2(0, 0), im = re;
       for (int r0 = 0; r0 < cs; r0 += 2) {  // cs is 1 or even: two ranks' loads in flight
         longlong2 x[2], y[2];
@@ -540,7 +599,30 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     C[z * sC + gi + (long)gj * ldc] = out;
     if (herm && gi != gj) C[gj + (long)gi * ldc] = cconj(out);
   }
+  __syncwarp();
   if (cs > 1) oz_cluster_sync();  // the sums stay readable until every CTA of the cluster has them
+  else if (GUARD) __syncthreads();
+  if (GUARD && !bad) {  // a warp an element, lanes along K
+    const int n = (int)*nlist;
+    for (int f = warp; f < n; f += OZ_THREADS / 32) {
+      const int e = list[f], gi = tm * 64 + (e & 63), gj = tn * OZ_BN + rank * nc + (e >> 6);
+      const double2 *pa = plain.a.p + z * plain.a.sb, *pb = plain.b.p + (bshared ? 0 : z * plain.b.sb);
+      double2 out = make_double2(0.0, 0.0);
+      for (int k = lane; k < plain.K; k += 32) {
+        const double2 x = oz_entry(plain.a, pa, gi, k), y = oz_entry(plain.b, pb, gj, k);
+        out.x = fma(x.x, y.x, fma(-x.y, y.y, out.x));
+        out.y = fma(x.x, y.y, fma(x.y, y.x, out.y));
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        out.x += __shfl_xor_sync(0xffffffffu, out.x, o);
+        out.y += __shfl_xor_sync(0xffffffffu, out.y, o);
+      }
+      if (lane != 0) continue;
+      if (sub) out = csub(C[z * sC + gi + (long)gj * ldc], out);
+      C[z * sC + gi + (long)gj * ldc] = out;
+      if (herm && gi != gj) C[gj + (long)gi * ldc] = cconj(out);
+    }
+  }
 }
 
 int oz_map_make(CUtensorMap* map, const void* base, long Kp, long rows, long planes, int box_rows) {
@@ -558,18 +640,18 @@ int oz_map_make(CUtensorMap* map, const void* base, long Kp, long rows, long pla
 }
 
 // clusters of `cs` CTAs the device holds at once
-int oz_clusters(int cs, int* out) {
+int oz_clusters(bool guard, int cs, int* out) {
   static std::mutex mu;
-  static std::map<std::pair<int, int>, int> known;
+  static std::map<std::tuple<int, bool, int>, int> known;
   int dev = 0;
   QR_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(mu);
-  auto it = known.find({dev, cs});
+  auto it = known.find({dev, guard, cs});
   if (it == known.end()) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cs);
     cfg.blockDim = dim3(OZ_THREADS);
-    cfg.dynamicSmemBytes = OZ_SMEM;
+    cfg.dynamicSmemBytes = oz_smem(guard);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = cs;
@@ -578,8 +660,9 @@ int oz_clusters(int cs, int* out) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    QR_CUDA(cudaOccupancyMaxActiveClusters(&n, zgemm_oz_k, &cfg));
-    it = known.emplace(std::make_pair(dev, cs), n).first;
+    if (guard) QR_CUDA(cudaOccupancyMaxActiveClusters(&n, zgemm_oz_k<true>, &cfg));
+    else QR_CUDA(cudaOccupancyMaxActiveClusters(&n, zgemm_oz_k<false>, &cfg));
+    it = known.emplace(std::make_tuple(dev, guard, cs), n).first;
   }
   *out = it->second;
   return QR_OK;
@@ -598,15 +681,17 @@ constexpr int OZ_NO_ROOM = -1;  // oz_run: the slices found no memory, nothing w
 
 static int oz_run(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
                   const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk,
-                  int herm, int eq_a, int sub, size_t room = OZ_ROOM) {
+                  int herm, int eq_a, int sub, bool guard, size_t room = OZ_ROOM) {
   if (room == 0) return OZ_NO_ROOM;
+  const int planes = oz_planes(guard);
+  const float least = OZ_LEAST * sqrtf((float)K);
   const bool bshared = sB == 0 || batch == 1;
   const int ntm = (M + 63) / 64, ntn = (N + OZ_BN - 1) / OZ_BN, Kh = (K + 15) / 16 * 16;
   const long Kp = 2L * Kh, arows = 128L * ntm, brows = (long)OZ_BN * ntn;
   const long apl = arows * Kp, bpl = brows * Kp;
   // bytes of one entry of A, and of B with its scales along K
-  const size_t abytes = (size_t)OZ_S * apl * 2 + sizeof(int) * (size_t)M;
-  const size_t bbytes = (size_t)OZ_S * bpl * 2 + sizeof(int) * ((size_t)N + K);
+  const size_t abytes = (size_t)planes * apl * 2 + sizeof(int) * (size_t)M;
+  const size_t bbytes = (size_t)planes * bpl * 2 + sizeof(int) * ((size_t)N + K);
   const size_t fixed = bshared ? bbytes : 0, each = abytes + (bshared ? 0 : bbytes);
   int run_len = (int)std::min<size_t>(batch, std::max<size_t>(1, room > fixed ? (room - fixed) / each : 1));
   char* ws = nullptr;
@@ -614,8 +699,8 @@ static int oz_run(cudaStream_t s, int opA, int opB, int M, int N, int K, const d
   size_t ab = 0, bbt = 0, ea = 0, eb = 0;
   for (;;) {
     bb = bshared ? 1 : run_len;
-    ab = up256((size_t)run_len * OZ_S * apl * 2);
-    bbt = up256((size_t)bb * OZ_S * bpl * 2);
+    ab = up256((size_t)run_len * planes * apl * 2);
+    bbt = up256((size_t)bb * planes * bpl * 2);
     ea = up256(sizeof(int) * (size_t)run_len * M);
     eb = up256(sizeof(int) * (size_t)bb * N);
     const cudaError_t e = cudaMallocAsync((void**)&ws, ab + bbt + ea + eb + sizeof(int) * (size_t)bb * K, s);
@@ -647,13 +732,14 @@ static int oz_run(cudaStream_t s, int opA, int opB, int M, int N, int K, const d
     const int nba = (M + rb - 1) / rb, nbb = (N + rb - 1) / rb;
     const unsigned grid = (unsigned)((long)nba * nz + (slice_b ? (long)nbb * nb : 0));
     const long gs = bshared ? 0 : K;
-    if (rb == 4) oz_digits_k<4><<<grid, 256, 0, s>>>(pl.a, pl.b, K, Kh, g, gs, nba, nbb, nz);
-    else oz_digits_k<16><<<grid, 256, 0, s>>>(pl.a, pl.b, K, Kh, g, gs, nba, nbb, nz);
+    if (rb == 4) oz_digits_k<4><<<grid, 256, 0, s>>>(pl.a, pl.b, K, Kh, g, gs, nba, nbb, nz, planes);
+    else oz_digits_k<16><<<grid, 256, 0, s>>>(pl.a, pl.b, K, Kh, g, gs, nba, nbb, nz, planes);
     QR_CHECK_LAUNCH("oz_digits_k");
     CUtensorMap ma, mb;
-    QR_TRY(oz_map_make(&ma, ws, Kp, arows, (long)OZ_S * nz, OZ_BM));
-    QR_TRY(oz_map_make(&mb, ws + ab, Kp, brows, (long)OZ_S * nb, OZ_BN));
-    QR_TRY(set_func_attr_once((const void*)zgemm_oz_k, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
+    QR_TRY(oz_map_make(&ma, ws, Kp, arows, (long)planes * nz, OZ_BM));
+    QR_TRY(oz_map_make(&mb, ws + ab, Kp, brows, (long)planes * nb, OZ_BN));
+    auto kern = guard ? zgemm_oz_k<true> : zgemm_oz_k<false>;
+    QR_TRY(set_func_attr_once((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, oz_smem(guard)));
     const int nk = (int)(Kp / OZ_BK);
     const long tiles = herm ? (long)ntm * (ntm + 1) / 2 : (long)ntm * ntn * nz;
     // K split over a cluster: the split with the fewest (waves x stages per CTA), a CTA's fixed cost
@@ -662,7 +748,7 @@ static int oz_run(cudaStream_t s, int opA, int opB, int M, int N, int K, const d
     double best = 1e300;
     for (int c = 1; c <= 8 && c <= nk; c *= 2) {
       int resident = 0;
-      QR_TRY(oz_clusters(c, &resident));
+      QR_TRY(oz_clusters(guard, c, &resident));
       if (resident < 1) continue;
       const double cost = (double)ceil_div(tiles, resident) * (ceil_div(nk, c) + 5.0 + (c > 1 ? 2.0 : 0.0));
       if (cost < best) {
@@ -673,7 +759,7 @@ static int oz_run(cudaStream_t s, int opA, int opB, int M, int N, int K, const d
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(tiles * cs));
     cfg.blockDim = dim3(OZ_THREADS);
-    cfg.dynamicSmemBytes = OZ_SMEM;
+    cfg.dynamicSmemBytes = oz_smem(guard);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -682,8 +768,8 @@ static int oz_run(cudaStream_t s, int opA, int opB, int M, int N, int K, const d
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    QR_CUDA(cudaLaunchKernelEx(&cfg, zgemm_oz_k, ma, mb, C + z0 * sC, ldc, sC, M, N, nk, bshared ? 1 : 0, ntm, ntn, cs,
-                               herm, sub, pl));
+    QR_CUDA(cudaLaunchKernelEx(&cfg, kern, ma, mb, C + z0 * sC, ldc, sC, M, N, nk, bshared ? 1 : 0, ntm, ntn, cs, herm,
+                               sub, least, pl));
     count_launch();
     return QR_OK;
   };
@@ -695,15 +781,16 @@ static int oz_run(cudaStream_t s, int opA, int opB, int M, int N, int K, const d
 
 // (where the slices find no memory, the products run on the CUDA cores, which need none)
 int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
-             const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk, size_t room) {
-  const int rc = oz_run(s, opA, opB, M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, dk, 0, 0, 0, room);
+             const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk, bool guard,
+             size_t room) {
+  const int rc = oz_run(s, opA, opB, M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, dk, 0, 0, 0, guard, room);
   if (rc != OZ_NO_ROOM) return rc;
   return zgemm_spread(s, opA, opB, M, N, K, make_double2(1.0, 0.0), A, lda, sA, B, ldb, sB, make_double2(0.0, 0.0), C, ldc,
                       sC, batch, dk);
 }
 int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
-             const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk) {
-  return zgemm_oz(s, opA, opB, M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, dk, OZ_ROOM);
+             const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk, bool guard) {
+  return zgemm_oz(s, opA, opB, M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, dk, guard, OZ_ROOM);
 }
 
 // C = A B (M x K, K x N) for an A whose columns spread over decades: the scaling along K equilibrates A's
@@ -715,7 +802,7 @@ int zgemm_graded(cudaStream_t s, int M, int N, int K, const double2* A, long lda
     return zgemm(s, OP_N, OP_N, M, N, K, make_double2(1.0, 0.0), A, lda, 0, B, ldb, 0, make_double2(0.0, 0.0), C, ldc, 0,
                  1, nullptr);
   const int pr = prof_begin(s, PK_ZGEMM, 8.0 * work, 16.0 * ((double)M * K + (double)K * N + (double)M * N));
-  int rc = oz_run(s, OP_N, OP_N, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, nullptr, 0, 1, 0);
+  int rc = oz_run(s, OP_N, OP_N, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, nullptr, 0, 1, 0, false);
   if (rc == OZ_NO_ROOM)
     rc = zgemm_spread(s, OP_N, OP_N, M, N, K, make_double2(1.0, 0.0), A, lda, 0, B, ldb, 0, make_double2(0.0, 0.0), C, ldc,
                       0, 1, nullptr);
@@ -731,7 +818,7 @@ int zgemm_sub(cudaStream_t s, int M, int N, int K, const double2* A, long lda, c
   const int pr = prof_begin(s, PK_ZGEMM, 8.0 * work, 16.0 * ((double)M * K + (double)K * N + 2.0 * M * N));
   int rc = OZ_NO_ROOM;
   if (work >= OZ_MIN_WORK && zgemm_oz_fits(M, N, K))
-    rc = oz_run(s, OP_N, OP_N, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, nullptr, 0, 0, 1);
+    rc = oz_run(s, OP_N, OP_N, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, nullptr, 0, 0, 1, false);
   if (rc == OZ_NO_ROOM)
     rc = zgemm_spread(s, OP_N, OP_N, M, N, K, make_double2(-1.0, 0.0), A, lda, 0, B, ldb, 0, make_double2(1.0, 0.0), C, ldc,
                       0, 1, nullptr);
@@ -747,7 +834,7 @@ int zherk(cudaStream_t s, int n, int K, const double2* A, long lda, double2* C, 
   const int pr = prof_begin(s, PK_ZGEMM, 4.0 * work, 16.0 * ((double)n * K + (double)n * n));
   int rc = OZ_NO_ROOM;
   if (work >= OZ_MIN_WORK && zgemm_oz_fits(n, n, K))
-    rc = oz_run(s, OP_C, OP_N, n, n, K, A, lda, 0, A, lda, 0, C, ldc, 0, 1, nullptr, 1, 0, 0);
+    rc = oz_run(s, OP_C, OP_N, n, n, K, A, lda, 0, A, lda, 0, C, ldc, 0, 1, nullptr, 1, 0, 0, false);
   if (rc == OZ_NO_ROOM) rc = zherk_spread(s, n, K, A, lda, C, ldc);
   prof_end(s, pr);
   return rc;

@@ -7,9 +7,11 @@ namespace qr {
 enum { OP_N = 0, OP_T = 1, OP_C = 2, OP_R = 3 };
 
 // ---- gemm.cu -----------------------------------------------------------------------------------
+// normwise: the error may be relative to the maxima of op(A)'s rows and op(B)'s columns (see gemm_oz.cu); else
+// it is relative to the sum of the products' magnitudes, element by element, as FP64 arithmetic has it.
 int zgemm(cudaStream_t s, int opA, int opB, int M, int N, int K, double2 alpha,
           const double2* A, long lda, long sA, const double2* B, long ldb, long sB,
-          double2 beta, double2* C, long ldc, long sC, int batch, const double* dk);
+          double2 beta, double2* C, long ldc, long sC, int batch, const double* dk, bool normwise = false);
 // From this many complex multiply-adds on, the three launches of the sliced product cost less than the
 // spread kernel's FP64 time (4 DFMA each at 2 per SM and cycle): 96 x 128 x 96 takes 25 us sliced and 19
 // spread, 128 x 128 x 128 25 and 31, 256 x 512 x 256 34 and 372.  (The 64 x 64-tile DMMA kernel that ran all
@@ -22,13 +24,14 @@ int zgemm_spread(cudaStream_t s, int opA, int opB, int M, int N, int K, double2 
 
 // ---- gemm_oz.cu: C[b] = op(A[b]) diag(dk) op(B[b]) at FP64 accuracy on the tcgen05 tensor cores
 // (exact products of 8-bit slices); sB = 0 shares B.  Slices in a stream-ordered allocation: 56 bytes an entry
-// of A and 28 of B, a batch in runs of at most 1 GiB; zgemm_spread where there is no memory for them.  The second
+// of A and 28 of B (64 and 32 with the guard), a batch in runs of at most 1 GiB; zgemm_spread where there is no memory for them.  The second
 // form takes the bytes of a run (0: as if there were no memory).
 bool zgemm_oz_fits(int M, int N, int K);
 int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
-             const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk);
+             const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk, bool guard);
 int zgemm_oz(cudaStream_t s, int opA, int opB, int M, int N, int K, const double2* A, long lda, long sA,
-             const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk, size_t room);
+             const double2* B, long ldb, long sB, double2* C, long ldc, long sC, int batch, const double* dk, bool guard,
+             size_t room);
 
 int zherk_spread(cudaStream_t s, int n, int K, const double2* A, long lda, double2* C, long ldc);
 // C = A B for an A whose columns spread over decades (see gemm_oz.cu)

@@ -606,7 +606,8 @@ static int zqr_thin_blocked(cudaStream_t s, double2* A, int m, int n, long lda, 
     // the unit triangle apart: beside its ones the sliced product would round the long, small part of V
     // relative to 1 (2048 rows: 8x the error of an FP64 product)
     const int lo = mj - nb;
-    if (lo > 0) QR_TRY(zgemm(s, OP_C, OP_N, nb, nc, lo, one, Vp + nb, m, 0, C + nb, ldc, 0, zero, W, QB, 0, 1, nullptr));
+    if (lo > 0) QR_TRY(zgemm(s, OP_C, OP_N, nb, nc, lo, one, Vp + nb, m, 0, C + nb, ldc, 0, zero, W, QB, 0, 1, nullptr,
+                             true));
     QR_TRY(zgemm_spread(s, OP_C, OP_N, nb, nc, nb, one, Vp, m, 0, C, ldc, 0, lo > 0 ? one : zero, W, QB, 0, 1, nullptr));
     wy_solve_k<<<ceil_div(nc, 4), 128, 0, s>>>(S + (size_t)QB * QB * p, tau + p0, nb, W, nc, adjoint);
     QR_CHECK_LAUNCH("wy_solve_k");

@@ -2338,7 +2338,8 @@ static int polish_columns(cudaStream_t s, SvdWork* w, double2* L, long ldl, int 
   QR_CUDA(cudaMemsetAsync(T, 0, sizeof(double2) * (size_t)k * k, s));
   refine_m_k<<<gs((long)k * k), TPB, 0, s>>>(T, nullptr, S, k);  // (I - S) / 2
   QR_CHECK_LAUNCH("refine_m_k");
-  QR_TRY(zgemm(s, OP_N, OP_N, m, k, k, make_double2(1.0, 0.0), L, ldl, 0, T, k, 0, make_double2(0.0, 0.0), Y, m, 0, 1, nullptr));
+  QR_TRY(zgemm(s, OP_N, OP_N, m, k, k, make_double2(1.0, 0.0), L, ldl, 0, T, k, 0, make_double2(0.0, 0.0), Y, m, 0, 1, nullptr,
+               true));
   add_cols_k<<<gs((long)m * k), TPB, 0, s>>>(L, ldl, Y, m, k);
   QR_CHECK_LAUNCH("add_cols_k");
   return QR_OK;
@@ -2639,13 +2640,13 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
     const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
     if (tall) {  // A = B0: U = Q Rf (m x k), Vh = (P L)^H
       QR_TRY(zgemm(s, OP_N, OP_N, rows0, k, k, one, w->Qp.as<double2>(), rows0, 0, Rf, k, 0, zero, U, ldu, 0, 1,
-                   nullptr));
+                   nullptr, true));
       scatter_rows_k<<<gs((long)k * k), TPB, 0, s>>>(L, k, order, V, k);
       QR_CHECK_LAUNCH("scatter_rows_k");
       QR_TRY(ztranspose(s, V, k, k, k, Vh, ldvh, 1));
     } else {  // A = B0^H = P L Sigma (Q Rf)^H: U = P L (m x m), Vh = (Q Rf)^H (m x n); B is free
       QR_TRY(zgemm(s, OP_N, OP_N, rows0, k, k, one, w->Qp.as<double2>(), rows0, 0, Rf, k, 0, zero, B, rows0, 0, 1,
-                   nullptr));
+                   nullptr, true));
       scatter_rows_k<<<gs((long)k * k), TPB, 0, s>>>(L, k, order, U, ldu);
       QR_CHECK_LAUNCH("scatter_rows_k");
       QR_TRY(ztranspose(s, B, rows0, rows0, k, Vh, ldvh, 1));

@@ -237,7 +237,7 @@ int refine(cudaStream_t s, SvdWork* w, const double2* A, int rows, int k, double
   }
   auto product = [&](const double2* P, const double2* Q2, double2* C) {
     return tc ? zgemm_tc(s, OP_N, OP_N, k, k, k, P, k, 0, Q2, k, 0, C, k, 0, 1, tcw, err)
-              : zgemm(s, OP_N, OP_N, k, k, k, one, P, k, 0, Q2, k, 0, zero, C, k, 0, 1, nullptr);
+              : zgemm(s, OP_N, OP_N, k, k, k, one, P, k, 0, Q2, k, 0, zero, C, k, 0, 1, nullptr, true);
   };
   unsigned* hs = static_cast<unsigned*>(host_scratch(sizeof(unsigned) * 8));
   if (!hs) return fail(QR_ENOMEM, "page-locked host scratch");

@@ -130,7 +130,7 @@ int qr_test_zgemm_oz(int opA, int opB, int M, int N, int K, int batch, int b_sha
   for (int it = 0; it < 2 && !rc; it++) {  // the second run is the timed one
     cudaEventRecord(e0);
     rc = zgemm_oz(0, opA, opB, M, N, K, (double2*)dA.p, lda, sA, (double2*)dB.p, ldb, sB, (double2*)dC.p, M, sC, batch,
-                  nullptr, (size_t)room);
+                  nullptr, true, (size_t)room);
     cudaEventRecord(e1);
     cudaEventSynchronize(e1);
     cudaEventElapsedTime(&t, e0, e1);
