@@ -32,10 +32,10 @@ int qr_test_zgemm(int opA, int opB, int M, int N, int K, const double* alpha, co
    accumulators); `batch` matrices at strides sA / sB (sB = 0: B shared), C[b] at b * ldc * N. */
 int qr_test_zgemm_tc(int opA, int opB, int M, int N, int K, int batch, const double* A, long lda, long sA,
                      const double* B, long ldb, long sB, double* C, long ldc, int iters, double* ms_per_iter);
-/* C[b] = op(A[b]) op(B[b]) as exact 8-bit slices on the tensor cores with `room` bytes of workspace at a time
-   (0: as if there were no memory); `batch` matrices one after another (b_shared: one B), C[b] at b * M * N. */
+/* C[b] = op(A[b]) op(B[b]) as 8-bit slices on the tensor cores, accurate element by element (guard) or relative to
+   the rows' and columns' maxima, with `room` bytes of workspace at a time (0: as if there were no memory); `batch` matrices one after another (b_shared: one B), C[b] at b * M * N. */
 int qr_test_zgemm_oz(int opA, int opB, int M, int N, int K, int batch, int b_shared, const double* A, long lda,
-                     const double* B, long ldb, double* C, uint64_t room, double* ms);
+                     const double* B, long ldb, double* C, int guard, uint64_t room, double* ms);
 /* Double-float GEMM on the FP32 pipes.  mode 0: C = op(A) B; 1: C = I - op(A) B; 2: C = D + 0.5
    op(A) B with FP32 products (A, B rounded to FP32); 3: C = I - A^H A from the upper tiles (op C,
    B ignored).  op(A) in {0 N, 1 T, 2 C}; D used by mode 2. */

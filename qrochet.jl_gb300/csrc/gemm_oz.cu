@@ -21,14 +21,18 @@
 //     every 256 k', those of d >= 4 every 1024, into two 64-bit integers per element, while the other
 //     group's products keep the tensor core busy.  Neither the K order nor the split of K over a cluster
 //     changes a bit of an exact sum.  The epilogue rounds hi + lo once to FP64.
-// The first neglected products (d = 7) lie at 2^-56 of the row and column maxima.  Rows or columns that
-// hold an infinity or NaN are recomputed by plain FP64 dot products in the epilogue.
+// The first neglected products (d = 7) lie at 2^-56 of the row and column maxima (with the guard, below, 2^-64).
+// Rows or columns that hold an infinity or NaN are recomputed by plain FP64 dot products in the epilogue.
 // So the error is relative to the maxima of a row and a column, and an element whose products are all far below
 // them (entries over many decades, the large ones of the row against the small ones of the column) would lose
 // digits that an FP64 product keeps.  With the guard an eighth accumulator sums the products of the leading
 // bytes' absolute values, sum |a||b| in units of 2^-14 of the two maxima, and elements where it is below
-// OZ_LEAST sqrt(K) are formed in FP64 instead, a warp each.  Above it the rounding of the slices, ~0.1 sqrt(2 K) 2^-55 of
-// the maxima, is at most ~2e-15 of sum |a||b|, about what an FP64 sum of 256 terms commits.  (Entries exp(6 x), x
+// OZ_LEAST sqrt(K) are formed in FP64 instead, a warp each.  The guard also adds the products of d = 7, whose absence is
+// the larger part of the error where a row's maximum stands out (R's diagonal: R diag(Lambda) B at 256 columns is
+// 1.0e-15 off without and 2.0e-16 with them, an FP64 product 7e-16): with slice s weighed 2^(-8 s), which bf16 holds
+// exactly, they go into the accumulator of d = 6, whose sums then round at 2^-24 of themselves, 2^-66 of the maxima.
+// What is left, the rounding of the entries, ~0.1 sqrt(2 K) 2^-55 of the maxima, is at most ~2e-15 of sum |a||b| for
+// elements above the line, about what an FP64 sum of 256 terms commits.  (Entries exp(6 x), x
 // normal: 2e-9 - 5e-8 of sum |a||b| without the guard.)  Products whose error the caller needs relative to norms only
 // (orthogonal factors, refinement, QR updates) do without: an identity's zeros would all be formed in FP64.
 //
@@ -149,15 +153,19 @@ __device__ __forceinline__ unsigned long long oz_fixed(double x, int shift) {
   else v = (m + (1ull << (sh - 1))) >> sh;
   return bits < 0 ? kBias - v : kBias + v;
 }
-// slice s of four biased values as four bf16
-__device__ __forceinline__ uint2 oz_slice4(const unsigned long long (&v)[4], int s) {
+// slice s of four biased values as four bf16, times `scale` (a power of two)
+__device__ __forceinline__ uint2 oz_slice4(const unsigned long long (&v)[4], int s, float scale) {
   float f[4];
 #pragma unroll
   for (int u = 0; u < 4; u++)
-    f[u] = __uint_as_float(0x4B000000u | (unsigned)((v[u] >> (8 * (OZ_S - 1 - s))) & 0xff)) - 8388736.f;
+    f[u] = (__uint_as_float(0x4B000000u | (unsigned)((v[u] >> (8 * (OZ_S - 1 - s))) & 0xff)) - 8388736.f) * scale;
   const __nv_bfloat162 a = __floats2bfloat162_rn(f[0], f[1]), b = __floats2bfloat162_rn(f[2], f[3]);
   return make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
 }
+
+// the weight of slice s (accumulator d) with the guard, 2^(-8 s), and its inverse
+__device__ __forceinline__ float oz_down(int s) { return __uint_as_float((unsigned)(127 - 8 * s) << 23); }
+__device__ __forceinline__ float oz_up(int d) { return __uint_as_float((unsigned)(127 + 8 * d) << 23); }
 
 // RB rows of one operand per CTA: exponents, then digits through a shared tile of 1024 / RB k's.
 template <int RB>
@@ -219,7 +227,8 @@ __global__ void __launch_bounds__(256) oz_digits_k(const OzOperand a, const OzOp
 #pragma unroll
     for (int s = 0; s <= OZ_S; s++) {
       if (s == OZ_S && planes == OZ_S) break;
-      uint2 re = oz_slice4(vr, s % OZ_S), im = oz_slice4(vi, s % OZ_S);
+      const float scale = planes == OZ_S ? 1.f : oz_down(s % OZ_S);
+      uint2 re = oz_slice4(vr, s % OZ_S, scale), im = oz_slice4(vi, s % OZ_S, scale);
       if (s == OZ_S) {  // the guard's plane
         re = make_uint2(re.x & 0x7fff7fffu, re.y & 0x7fff7fffu);
         im = make_uint2(im.x & 0x7fff7fffu, im.y & 0x7fff7fffu);
@@ -258,8 +267,8 @@ __device__ __forceinline__ void oz_mma(uint32_t d, uint32_t alo, uint32_t blo, u
       "r"(alo), "r"(blo), "r"(hi), "r"(kOzIdesc), "r"(accumulate)
       : "memory");
 }
-// the products of accumulators D0 <= d < D1 of one stage
-template <int D0, int D1>
+// the products of accumulators D0 <= d < D1 of one stage; with the guard those of d = 7 go into the last one
+template <int D0, int D1, bool GUARD>
 __device__ __forceinline__ void oz_products(uint32_t tmem, uint32_t alo, uint32_t blo, uint32_t hi, bool first) {
 #pragma unroll
   for (int d = D0; d < D1; d++)
@@ -269,6 +278,14 @@ __device__ __forceinline__ void oz_products(uint32_t tmem, uint32_t alo, uint32_
       for (int j = 0; j < OZ_BK / 16; j++)
         oz_mma(tmem + (uint32_t)(d * OZ_BN), alo + (uint32_t)((i * OZ_AT + 32 * j) >> 4),
                blo + (uint32_t)(((d - i) * OZ_BT + 32 * j) >> 4), hi, (first && i == 0 && j == 0) ? 0u : 1u);
+  if (GUARD && D1 == OZ_S) {
+#pragma unroll
+    for (int i = 1; i < OZ_S; i++)
+#pragma unroll
+      for (int j = 0; j < OZ_BK / 16; j++)
+        oz_mma(tmem + (uint32_t)((OZ_S - 1) * OZ_BN), alo + (uint32_t)((i * OZ_AT + 32 * j) >> 4),
+               blo + (uint32_t)(((OZ_S - i) * OZ_BT + 32 * j) >> 4), hi, 1u);
+  }
 }
 __device__ __forceinline__ void oz_tmem_ld16(uint32_t taddr, float (&v)[16]) {
   uint32_t r[16];
@@ -281,11 +298,16 @@ __device__ __forceinline__ void oz_tmem_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
   for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
-// acc += w * (16 accumulator columns as integers).  Sums below 2^22 (nearly always) turn into integers
+// acc += w * (16 accumulator columns, times `up`, as integers).  Sums below 2^22 (nearly always) turn into integers
 // by adding 1.5 2^23 and reading the bits; the conversion instruction runs at an eighth of that rate.
-__device__ __forceinline__ void oz_drain(uint32_t ta, int w, long long (&acc)[16]) {
+template <bool GUARD>
+__device__ __forceinline__ void oz_drain(uint32_t ta, int w, float up, long long (&acc)[16]) {
   float v[16];
   oz_tmem_ld16(ta, v);
+  if (GUARD) {
+#pragma unroll
+    for (int j = 0; j < 16; j++) v[j] *= up;
+  }
   float top = 0.f;
 #pragma unroll
   for (int j = 0; j < 16; j++) top = fmaxf(top, fabsf(v[j]));
@@ -447,8 +469,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           }
           const bool f = first[grp];
           first[grp] = false;
-          if (low) oz_products<OZ_DH, OZ_S>(tmem, (uint32_t)da, (uint32_t)db, dh, f);
-          else oz_products<0, OZ_DH>(tmem, (uint32_t)da, (uint32_t)db, dh, f);
+          if (low) oz_products<OZ_DH, OZ_S, GUARD>(tmem, (uint32_t)da, (uint32_t)db, dh, f);
+          else oz_products<0, OZ_DH, GUARD>(tmem, (uint32_t)da, (uint32_t)db, dh, f);
         }
         if (!ok) break;
         tc_commit(empty + s);
@@ -500,15 +522,15 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         if (!(ok = wait_group(0))) break;
         int w = 1 << 16;
 #pragma unroll 1
-        for (int d = 0; d < 3; d++, w >>= 8) oz_drain(ta + d * OZ_BN, w, hi);
-        oz_drain(ta + 3 * OZ_BN, 1 << 24, lo);
+        for (int d = 0; d < 3; d++, w >>= 8) oz_drain<GUARD>(ta + d * OZ_BN, w, oz_up(d), hi);
+        oz_drain<GUARD>(ta + 3 * OZ_BN, 1 << 24, oz_up(3), lo);
         release(0);
       }
       if (oz_drain_l(n, last)) {
         if (!(ok = wait_group(1))) break;
         int w = 1 << 16;
 #pragma unroll 1
-        for (int d = OZ_DH; d < OZ_S; d++, w >>= 8) oz_drain(ta + d * OZ_BN, w, lo);
+        for (int d = OZ_DH; d < OZ_S; d++, w >>= 8) oz_drain<GUARD>(ta + d * OZ_BN, w, oz_up(d), lo);
         release(1);
       }
       if (n == last) break;

@@ -110,10 +110,10 @@ int qr_test_zgemm_tc(int opA, int opB, int M, int N, int K, int batch, const dou
   return QR_OK;
 } QR_ABI_CATCH
 
-// C[b] = op(A[b]) op(B[b]) on exact slices (gemm_oz.cu) with `room` bytes of workspace at a time; A and B hold
+// C[b] = op(A[b]) op(B[b]) on slices (gemm_oz.cu), guarded or not, with `room` bytes of workspace at a time; A and B hold
 // `batch` matrices at strides lda * columns (b_shared: one B), C at stride M * N.
 int qr_test_zgemm_oz(int opA, int opB, int M, int N, int K, int batch, int b_shared, const double* A, long lda,
-                     const double* B, long ldb, double* C, uint64_t room, double* ms) try {
+                     const double* B, long ldb, double* C, int guard, uint64_t room, double* ms) try {
   if (M <= 0 || N <= 0 || K <= 0 || batch < 1 || !zgemm_oz_fits(M, N, K)) return fail(QR_EINVAL, "bad gemm shape");
   const bool an = opA == OP_N || opA == OP_R, bn = opB == OP_N || opB == OP_R;
   if (lda < (an ? M : K) || ldb < (bn ? K : N)) return fail(QR_EINVAL, "bad leading dimension");
@@ -130,7 +130,7 @@ int qr_test_zgemm_oz(int opA, int opB, int M, int N, int K, int batch, int b_sha
   for (int it = 0; it < 2 && !rc; it++) {  // the second run is the timed one
     cudaEventRecord(e0);
     rc = zgemm_oz(0, opA, opB, M, N, K, (double2*)dA.p, lda, sA, (double2*)dB.p, ldb, sB, (double2*)dC.p, M, sC, batch,
-                  nullptr, true, (size_t)room);
+                  nullptr, guard != 0, (size_t)room);
     cudaEventRecord(e1);
     cudaEventSynchronize(e1);
     cudaEventElapsedTime(&t, e0, e1);

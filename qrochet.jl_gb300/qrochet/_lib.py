@@ -116,7 +116,7 @@ SIGNATURES = {
     "qr_test_zgemm": [_I, _I, _I, _I, _I, _PD, _PD, C.c_long, _PD, C.c_long, _PD, _PD, C.c_long, _PD, _I, _PD],
     "qr_test_zgemm_tc": [_I, _I, _I, _I, _I, _I, _PD, C.c_long, C.c_long, _PD, C.c_long, C.c_long, _PD, C.c_long,
                          _I, _PD],
-    "qr_test_zgemm_oz": [_I, _I, _I, _I, _I, _I, _I, _PD, C.c_long, _PD, C.c_long, _PD, C.c_uint64, _PD],
+    "qr_test_zgemm_oz": [_I, _I, _I, _I, _I, _I, _I, _PD, C.c_long, _PD, C.c_long, _PD, _I, C.c_uint64, _PD],
     "qr_test_zgemm_df": [_I, _I, _I, _I, _I, _PD, C.c_long, _PD, C.c_long, _PD, _PD, C.c_long, _I, _PD],
     "qr_test_svd": [_I, _I, _I, _PD, _PD, _PD, _PD, _PD],
     "qr_test_svd_paths": [C.POINTER(C.c_uint64), _I, C.POINTER(C.c_int)],

@@ -1,5 +1,6 @@
 """Batched FP64 products on exact slices whose workspace holds a part of the batch only, or none of it: runs of
-entries give the bits of one run over the whole batch; without memory the CUDA cores give the product."""
+entries give the bits of one run over the whole batch (the guarded product, whose last accumulator rounds, the same
+values); without memory the CUDA cores give the product."""
 import ctypes as C
 
 import numpy as np
@@ -14,14 +15,14 @@ pytestmark = pytest.mark.gpu
 ROOM = 1 << 30
 
 
-def batched(A, B, room, opA=0):
+def batched(A, B, room, opA=0, guard=0):
     batch, N, M = A.shape[0], B.shape[-1], A.shape[1] if opA == 0 else A.shape[2]
     K = B.shape[-2]
     fa = np.ascontiguousarray(np.swapaxes(A, 1, 2))  # column-major matrices, one after another
     fb = np.ascontiguousarray(np.swapaxes(B, -1, -2))
     out, ms = np.empty((batch, N, M), dtype=np.complex128), C.c_double()
     _lib.check(_lib.lib().qr_test_zgemm_oz(opA, 0, M, N, K, batch, int(B.ndim == 2), _lib.dptr(fa), A.shape[1],
-                                           _lib.dptr(fb), K, _lib.dptr(out), room, C.byref(ms)))
+                                           _lib.dptr(fb), K, _lib.dptr(out), guard, room, C.byref(ms)))
     return np.swapaxes(out, 1, 2)
 
 
@@ -40,7 +41,8 @@ def test_runs_of_a_batch(shared, batch, M, N, K):
     ref = A @ B
     bound = K * 2.0 ** -50 * np.max(np.abs(A)) * np.max(np.abs(B))
     assert np.max(np.abs(whole - ref)) <= bound
-    assert np.max(np.abs(batched(A, B, 0) - ref)) <= bound
+    for room in (0, 1, 3 * entry + (b if shared else 3 * b), ROOM):
+        assert np.max(np.abs(batched(A, B, room, guard=1) - ref)) <= bound
 
 
 def test_transposed_operand_in_runs():
