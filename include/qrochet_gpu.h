@@ -168,8 +168,9 @@ int qr_mpo_random(int n, int d, int chi, uint64_t seed, int complex_entries, qr_
    |0...0> (evolve! with `threshold` and maxdim = chi_max; gate g acts on sites gate_site[g] and
    gate_site[g]+1 with the 4x4 row-major complex matrix at gate_mats + 32 g) followed by Pauli
    strings (string j: obs_weight[j] entries of (site, code 0 I / 1 X / 2 Y / 3 Z), packed).  Requests
-   are admitted FIFO when their device-memory footprint (qr_server_footprint) fits the budget;
-   each of `workers` threads runs one admitted request on its own chain and stream, so admitted
+   are accepted when their device-memory footprint (qr_server_footprint) fits the budget and admitted
+   FIFO when their gate steps' peak (up to 2.6 footprints) fits what running requests leave of it, or
+   nothing runs; each of `workers` threads runs one admitted request on its own chain and stream, so admitted
    requests overlap on the GPU.  Results are the unnormalised <psi|P|psi> per string (re, im). */
 typedef struct qr_server qr_server;
 int qr_server_create(int device, int workers, uint64_t hbm_budget_bytes, int precision, qr_server** out);

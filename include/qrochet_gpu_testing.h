@@ -61,6 +61,9 @@ int qr_test_qr(int m, int n, const double* A, double* Q, double* R, double* ms);
 /* The order in which the SVD ranks column norms (ranks_before), on the host: perm[rank] = index for n keys.
    No GPU needed. */
 int qr_test_rank_order(const double* keys, int n, int* perm);
+/* The share of a server's budget that a running request takes: its gate steps' peak, at most the budget (a
+   request whose footprint fits but whose peak does not runs alone).  No GPU needed. */
+int qr_test_server_admission(int n, int chi_max, uint64_t budget, uint64_t* bytes);
 /* Throws a C++ exception inside an exported function (kind 0: std::bad_alloc, 1: a standard
    std::runtime_error, 2: an object of no standard type) so that a test sees the ABI guard turn it
    into a status (QR_ENOMEM, QR_EHOST, QR_EHOST) and a message; any other kind returns QR_OK.

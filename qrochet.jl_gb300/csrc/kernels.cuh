@@ -113,6 +113,9 @@ int zqr_thin(cudaStream_t s, double2* A, int m, int n, long lda, double2* Q, lon
 int zqr_thin_steps(cudaStream_t s, double2* A, int m, int n, long lda, double2* Q, long ldq,
                    double2* R, long ldr, double2* tau);
 
+// ---- serve.cu: the share of the budget that a request takes while it runs
+uint64_t admission_bytes(int n, int chi_max, uint64_t budget);
+
 // ---- svd.cu ------------------------------------------------------------------------------------
 struct SvdWork;  // opaque, grows on demand
 SvdWork* svd_work_create();

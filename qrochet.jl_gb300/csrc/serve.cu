@@ -7,7 +7,9 @@
 // device-memory footprint fits the remaining budget, so work that arrives while other requests
 // run starts as soon as a worker slot and memory free up.  Each worker thread owns its request's
 // chain and CUDA stream, so admitted requests overlap on the GPU.  Requests whose footprint
-// exceeds the whole budget are rejected at submission (QR_ENOMEM).
+// exceeds the whole budget are rejected at submission (QR_ENOMEM).  What admitted requests hold
+// together is counted at the gate step's peak (admission_bytes), which lies above the footprint: a
+// request between the two is accepted and runs alone.
 #include <vector>
 #include <deque>
 #include <thread>
@@ -32,7 +34,7 @@ struct Request {
   std::vector<int> gate_site;
   std::vector<double> gate_mats;  // 32 doubles (4x4 complex) per gate
   std::vector<int> obs_weight, obs_sites, obs_paulis;
-  uint64_t footprint = 0;
+  uint64_t resident = 0;  // its share of the budget while it runs
   Clock::time_point t_submit, t_start, t_end;
   int status = QR_OK;
   std::string error;
@@ -40,9 +42,8 @@ struct Request {
   bool done = false;
 };
 
-uint64_t footprint_bytes(int n, int chi_max) {
-  // sites at their largest (chi = min(chi_max, 2^i, 2^(n-i))) plus the SVD/theta workspaces of the
-  // largest two-site block (about a dozen (2 chi) x (2 chi) complex buffers)
+// sites at their largest (chi = min(chi_max, 2^i, 2^(n-i)))
+uint64_t sites_bytes(int n, int chi_max) {
   uint64_t sites = 0;
   for (int i = 0; i < n; i++) {
     auto bond = [&](int b) -> uint64_t {  // bond b joins sites b and b+1
@@ -53,11 +54,26 @@ uint64_t footprint_bytes(int n, int chi_max) {
     };
     sites += 16ull * 2 * bond(i - 1) * bond(i);
   }
-  const uint64_t t = 2ull * chi_max;
-  return sites + 12ull * t * t * 16ull + (64ull << 20);
+  return sites;
 }
-
+// the sites plus `buffers` complex (2 chi) x (2 chi) matrices of SVD and theta workspace
+uint64_t request_bytes(int n, int chi_max, uint64_t buffers) {
+  const uint64_t t = 2ull * chi_max;
+  return sites_bytes(n, chi_max) + buffers * t * t * 16ull + (64ull << 20);
+}
+// Device memory that a gate step takes at its peak, in buffers of (2 chi)^2 complex numbers (mem_get_info after one
+// gate at chi 384 to 1024, less the sites): FP64 and decaying spectra 28.6 - 30.4, mixed 25.0 - 26.1.  Two thirds are
+// the SVD's workspace, which stays with the chain; the slices of its products take five more while they run.
+constexpr uint64_t kGateBuffers = 31;
+// what a request must find in the budget to be accepted
+uint64_t footprint_bytes(int n, int chi_max) { return request_bytes(n, chi_max, 12); }
 }  // namespace
+
+namespace qr {
+uint64_t admission_bytes(int n, int chi_max, uint64_t budget) {
+  return std::min(request_bytes(n, chi_max, kGateBuffers), budget);
+}
+}  // namespace qr
 
 struct qr_server {
   int device = 0, precision = 0;
@@ -138,16 +154,16 @@ void worker_loop(qr_server* sv) {
     {
       std::unique_lock<std::mutex> lk(sv->mu);
       sv->cv_work.wait(lk, [&] {
-        return sv->stop || (!sv->pending.empty() && sv->in_use + sv->pending.front()->footprint <= sv->budget);
+        return sv->stop || (!sv->pending.empty() && sv->in_use + sv->pending.front()->resident <= sv->budget);
       });
       if (sv->stop && sv->pending.empty()) return;
-      if (sv->pending.empty() || sv->in_use + sv->pending.front()->footprint > sv->budget) {
+      if (sv->pending.empty() || sv->in_use + sv->pending.front()->resident > sv->budget) {
         if (sv->stop) return;
         continue;
       }
       r = sv->pending.front();
       sv->pending.pop_front();
-      sv->in_use += r->footprint;
+      sv->in_use += r->resident;
       sv->in_flight++;
       r->t_start = Clock::now();
     }
@@ -156,7 +172,7 @@ void worker_loop(qr_server* sv) {
       std::lock_guard<std::mutex> lk(sv->mu);
       r->t_end = Clock::now();
       r->done = true;
-      sv->in_use -= r->footprint;
+      sv->in_use -= r->resident;
       sv->in_flight--;
       sv->completed++;
     }
@@ -234,8 +250,8 @@ int qr_server_submit(qr_server* sv, int n, int chi_max, double threshold, int ng
     if (obs_sites[q] < 0 || obs_sites[q] >= n) return qr::fail(QR_EINVAL, "Pauli string site outside the chain");
     if (obs_paulis[q] < 0 || obs_paulis[q] > 3) return qr::fail(QR_EINVAL, "Pauli code must be 0..3 (I, X, Y, Z)");
   }
-  r->footprint = footprint_bytes(n, chi_max);
-  if (r->footprint > sv->budget) return qr::fail(QR_ENOMEM, "request footprint exceeds the server's HBM budget");
+  r->resident = qr::admission_bytes(n, chi_max, sv->budget);
+  if (footprint_bytes(n, chi_max) > sv->budget) return qr::fail(QR_ENOMEM, "request footprint exceeds the server's HBM budget");
   {
     std::lock_guard<std::mutex> lk(sv->mu);
     r->ticket = sv->next_ticket++;

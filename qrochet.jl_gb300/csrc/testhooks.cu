@@ -285,6 +285,12 @@ int qr_test_rank_order(const double* keys, int n, int* perm) try {
   return QR_OK;
 } QR_ABI_CATCH
 
+int qr_test_server_admission(int n, int chi_max, uint64_t budget, uint64_t* bytes) try {
+  if (!bytes || n < 2 || chi_max < 1) return fail(QR_EINVAL, "bad request shape");
+  *bytes = admission_bytes(n, chi_max, budget);
+  return QR_OK;
+} QR_ABI_CATCH
+
 int qr_test_host_exception(int kind) try {
   struct NotStd {};
   if (kind == 0) throw std::bad_alloc();

@@ -124,6 +124,7 @@ SIGNATURES = {
                                C.POINTER(C.c_int)],
     "qr_test_qr": [_I, _I, _PD, _PD, _PD, _PD],
     "qr_test_rank_order": [_PD, _I, C.POINTER(C.c_int)],
+    "qr_test_server_admission": [_I, _I, C.c_uint64, C.POINTER(C.c_uint64)],
     "qr_test_host_exception": [_I],
 }
 
