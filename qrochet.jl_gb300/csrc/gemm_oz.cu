@@ -14,13 +14,13 @@
 //     real-ified, [[Ar, -Ai], [Ai, Ar]], in 128-row tiles of 64 complex rows.  Integer and FP32
 //     instructions only.
 //  3. zgemm_oz_k: the 28 slice products with i + j = d <= 6 as tcgen05.mma (M 128, N 64, K 16) into
-//     seven TMEM accumulators, one per d (448 of 512 columns, which is why the tile is 64 columns wide).
-//     Each |q q'| <= 2^14, so a sum of 256 k' stays below 2^24 for d <= 3 and every FP32 addition there
+//     seven TMEM accumulators, one per d (448 of 512 columns, which is why the tile is 64 columns wide; the
+//     guard below takes the rest).  Each |q q'| <= 2^14, so a sum of 256 k' stays below 2^24 for d <= 3 and every FP32 addition there
 //     is exact; d >= 4 weighs at most 2^-32 of the leading sum and stays exact while its sums, random in
 //     sign, are below 2^24 (2^19 after 1024 k' of random bytes).  The accumulators of d <= 3 are drained
 //     every 256 k', those of d >= 4 every 1024, into two 64-bit integers per element, while the other
 //     group's products keep the tensor core busy.  Neither the K order nor the split of K over a cluster
-//     changes a bit of an exact sum.  The epilogue rounds hi + lo once to FP64.
+//     changes a bit of an exact sum (with the guard d = 6 rounds, see there).  The epilogue rounds hi + lo once to FP64.
 // The first neglected products (d = 7) lie at 2^-56 of the row and column maxima (with the guard, below, 2^-64).
 // Rows or columns that hold an infinity or NaN are recomputed by plain FP64 dot products in the epilogue.
 // So the error is relative to the maxima of a row and a column, and an element whose products are all far below
@@ -31,15 +31,18 @@
 // the larger part of the error where a row's maximum stands out (R's diagonal: R diag(Lambda) B at 256 columns is
 // 1.0e-15 off without and 2.0e-16 with them, an FP64 product 7e-16): with slice s weighed 2^(-8 s), which bf16 holds
 // exactly, they go into the accumulator of d = 6, whose sums then round at 2^-24 of themselves, 2^-66 of the maxima.
-// What is left, the rounding of the entries, ~0.1 sqrt(2 K) 2^-55 of the maxima, is at most ~2e-15 of sum |a||b| for
-// elements above the line, about what an FP64 sum of 256 terms commits.  (Entries exp(6 x), x
-// normal: 2e-9 - 5e-8 of sum |a||b| without the guard.)  Products whose error the caller needs relative to norms only
-// (orthogonal factors, refinement, QR updates) do without: an identity's zeros would all be formed in FP64.
+// What is left is the rounding of the entries.  Measured over entries exp(2 x) and exp(6 x) (x normal), 12 decades,
+// 2% nonzeros and K of 64 to 4096, relative to sum |a||b|: rms 0.2 - 9e-16, largest 0.4 - 9e-15 (without the guard up
+// to 7e-7 and 1e-4; an FP64 product 1 - 8e-15 at the largest).  A line four times lower doubles that, and a line twice
+// as high takes 1.8 ms instead of 1.1 where every other element is one term (an orthogonal 1024 x 1024 factor with noise
+// for zeros, times 1024 x 2048; 0.75 for ordinary entries).  Products whose error the caller needs relative to norms
+// only (orthogonal factors, refinement, QR updates) do without.
 //
 // Bound: the MMAs, 28 products x 2 per 32 k' (about 51 cycles each: at N = 64 shared memory feeds the
-// tensor core 6 KB per MMA in 48); loads alone take 60% of that.  2048^3: 1.77 ms (39 TFLOP/s
-// complex-equivalent, FP64 DMMA 1.06), 512^3: 45 us, 256 x 512 x 256: 22 us, of which ~15 is the latency
-// of one tile.  A tile grid that would leave SMs idle splits K over a cluster of up to 8 CTAs, which add
+// tensor core 6 KB per MMA in 48; with the guard 35 x 2); loads alone take 60% of that.  The kernel alone at 2048^3:
+// 1.80 ms (38 TFLOP/s complex-equivalent, FP64 DMMA 1.06), 2.06 with the guard, tensor pipe 46 and 50% busy, its
+// operand ports in shared memory 69 and 75%.  All three launches: 2.09 and 2.36 ms; at 512^3 77 and 84 us, at
+// 256 x 512 x 256 47 and 49, most of it launches and the latency of one tile.  A tile grid that would leave SMs idle splits K over a cluster of up to 8 CTAs, which add
 // their integer sums through distributed shared memory.
 #include <cuda_bf16.h>
 #include <algorithm>
@@ -100,6 +103,10 @@ __device__ __forceinline__ double2 oz_entry(const OzOperand& o, const double2* p
   }
   if (o.conj) v.y = -v.y;
   return v;
+}
+
+__device__ __forceinline__ bool oz_zero(double2 v) {  // without the FP64 pipe
+  return !(((__double2hiint(v.x) | __double2hiint(v.y)) & 0x7fffffff) | __double2loint(v.x) | __double2loint(v.y));
 }
 
 // Biased exponent of x (subnormals: 1), OZ_ZERO for 0; 0x7ff for infinities and NaN.  One more when
@@ -353,7 +360,7 @@ __device__ __forceinline__ double oz_double(long long hi, long long lo, int e) {
 
 // The least sum of the guard's products per sqrt(K).  Gaussian entries give ~1000 K; rows with one entry that
 // counts (a diagonal environment) ~127 times the other operand's leading byte.
-constexpr float OZ_LEAST = 32.f;
+constexpr float OZ_LEAST = 16.f;
 // what the epilogue needs to form an element in plain FP64
 struct OzPlain {
   OzOperand a, b;
@@ -584,26 +591,22 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     } else if (xa == OZ_ZERO || xb == OZ_ZERO) {
       out.x = out.y = 0.0;
     } else {
-      if (GUARD) {
-        float p = 0.f;
-        for (int r = 0; r < cs; r++) {
-          const uint32_t at = oz_map(gbase + (uint32_t)(c * OZ_BM + i) * 4u, r);
-          p += oz_ldf_remote(at) + oz_ldf_remote(at + 64 * 4);
-        }
-        if (p < least) {
-          list[atomicAdd(nlist, 1u)] = (uint16_t)e;
-          continue;
-        }
-      }
       longlong2 re = make_longlong2(0, 0), im = re;
+      float p = 0.f;
       for (int r0 = 0; r0 < cs; r0 += 2) {  // cs is 1 or even: two ranks' loads in flight
         longlong2 x[2], y[2];
+        float px[2] = {0.f, 0.f}, py[2] = {0.f, 0.f};
 #pragma unroll
         for (int u = 0; u < 2; u++)
           if (r0 + u < cs) {
             const uint32_t at = oz_map(sbase + (uint32_t)(c * OZ_BM + i) * 16u, r0 + u);
             x[u] = oz_ld_remote(at);
             y[u] = oz_ld_remote(at + 64 * 16);
+            if (GUARD) {
+              const uint32_t gat = oz_map(gbase + (uint32_t)(c * OZ_BM + i) * 4u, r0 + u);
+              px[u] = oz_ldf_remote(gat);
+              py[u] = oz_ldf_remote(gat + 64 * 4);
+            }
           } else {
             x[u] = y[u] = make_longlong2(0, 0);
           }
@@ -611,6 +614,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         re.y += x[0].y + x[1].y;
         im.x += y[0].x + y[1].x;
         im.y += y[0].y + y[1].y;
+        if (GUARD) p += (px[0] + py[0]) + (px[1] + py[1]);
+      }
+      if (GUARD && p < least) {
+        list[atomicAdd(nlist, 1u)] = (uint16_t)e;
+        continue;
       }
       // units: q q' of slices 6 is 2^(E_i - 1077 + E_j - 1077); the sums carry 2^48 and hi 2^32 of it
       const int sc = xa + xb - 2154 + 48 + 32;
@@ -631,10 +639,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       const double2 *pa = plain.a.p + z * plain.a.sb, *pb = plain.b.p + (bshared ? 0 : z * plain.b.sb);
       double2 out = make_double2(0.0, 0.0);
       for (int k = lane; k < plain.K; k += 32) {
+        // (zeros, of which such operands are often full, cost the FP64 pipe nothing; the other factor is finite here)
+        if (oz_zero(pa[gi * plain.a.si + k * plain.a.sk]) || oz_zero(pb[gj * plain.b.si + k * plain.b.sk])) continue;
         const double2 x = oz_entry(plain.a, pa, gi, k), y = oz_entry(plain.b, pb, gj, k);
         out.x = fma(x.x, y.x, fma(-x.y, y.y, out.x));
         out.y = fma(x.x, y.y, fma(x.y, y.x, out.y));
       }
+      __syncwarp();
       for (int o = 16; o > 0; o >>= 1) {
         out.x += __shfl_xor_sync(0xffffffffu, out.x, o);
         out.y += __shfl_xor_sync(0xffffffffu, out.y, o);
@@ -748,7 +759,7 @@ static int oz_run(cudaStream_t s, int opA, int opB, int M, int N, int K, const d
       oz_kmax_k<<<dim3(ceil_div(K, KMAX_K), 1, nb), 256, 0, s>>>(eq_a ? pl.a : pl.b, K, g);
       QR_CHECK_LAUNCH("oz_kmax_k");
     }
-    // few rows: 4 per CTA so that the pass still covers the SMs; else 16
+    // up to 16 rows for each of the 152 SMs: 4 per CTA so that the pass still covers them; else 16
     const long rows = (long)M * nz + (slice_b ? (long)N * nb : 0);
     const int rb = rows <= 2432 ? 4 : 16;
     const int nba = (M + rb - 1) / rb, nbb = (N + rb - 1) / rb;

@@ -1,11 +1,10 @@
 """FP64 products of entries over many decades, element by element: the error is relative to sum |a||b|, not to the
 largest entries of the row and the column.
 
-Bound.  An element comes from slices when the sum of its leading bytes' products is at least 32 sqrt(K); a byte
+Bound.  An element comes from slices when the sum of its leading bytes' products is at least 16 sqrt(K); a byte
 may round a magnitude up to twofold, so the product X of the two maxima's powers of two is at most 2^16 2 /
-(32 sqrt(K)) = 2^12 / sqrt(K) times sum |a||b|.  A term's rounding and neglected slices have an rms of
-2^-54.2 X; eight sigma over K independent terms: 2^-51.2 sqrt(K) X <= 2^-39 of sum |a||b|.  NumPy's reference adds
-K 2^-52."""
+(16 sqrt(K)) = 2^13 / sqrt(K) times sum |a||b|.  The two roundings of a term have an rms of 2^-56.3 X each; eight
+sigma over K independent terms: 2^-52.8 sqrt(K) X < 2^-39 of sum |a||b|.  NumPy's reference adds K 2^-52."""
 import ctypes as C
 
 import numpy as np
