@@ -138,13 +138,11 @@ class DevTimer:
         return self.e0.elapsed_time(self.e1) * 1e-3
 
 
-# DRAM bytes (read + write) per launch (one Jacobi sweep, or one GEMM) from one ncu capture of each
-# kernel on a 1024 x 1024 mixed SVD: jacobi_block_reg_k for jacobi_fp32 (the Gram sweeps touch the same
-# B and V; ncu does not launch them), jacobi_block_df_k (the full double-float sweeps) for jacobi_df,
-# zgemm_df_k for zgemm_df.  A sweep's traffic is the first touch of B and V and a GEMM's the first
-# touch of its operands, so it scales with the operand size: (k / 1024)^2 at k columns.
-NCU_TRAFFIC_1024 = {"jacobi_fp32": 16.937472e6 + 15.872e3, "jacobi_df": 34.0e6 + 5.3e6,
-                    "zgemm_df": 16.850432e6}
+def sweep_bytes(kind, k):
+    """Bytes that one Jacobi sweep over k x k reads and writes at least (B and V once each way); computed, as ncu
+    does not launch the Gram-matrix sweeps (cooperative clusters).  None for classes that are not sweeps."""
+    entry = {"jacobi_fp32": 8, "jacobi_df": 16, "jacobi_fp64": 16}.get(kind)
+    return 4 * entry * k * k if entry else None
 
 
 def workload(chi):
@@ -712,10 +710,9 @@ def run_ours(args, chi):
     ms_step = 1e3 * dt_max / args.steps
     alg = gate_flops(chi)
     achieved = alg / (ms_step * 1e-3) / 1e12
-    # DRAM traffic per gate step: ncu bytes per launch (per sweep for the Jacobi kernels) times the
-    # launches (sweeps) per step of each profiled class
-    traffic = sum(NCU_TRAFFIC_1024[k] * (2 * chi / 1024) ** 2 * stats[k]["launches"] / nprof
-                  for k in NCU_TRAFFIC_1024)
+    # bytes per gate step, computed: B and V of every Jacobi sweep, operands and results of every product
+    traffic = sum((sweep_bytes(k, 2 * chi) * v["launches"] if sweep_bytes(k, 2 * chi) else v["bytes"]) / nprof
+                  for k, v in stats.items())
     roofline = {"bound": "fp32", "kernel": "gate step (all kernels of one evolve!)", "achieved": achieved,
                 "peak": ffma, "unit": "TFLOP/s", "frac": achieved / ffma if ffma else None,
                 "traffic": traffic, "launches": launches / max(1, args.steps), "avg_launch_ms": ms_step,
@@ -723,14 +720,13 @@ def run_ours(args, chi):
                                    f"Golub-Van Loan R-SVD count of a {2 * chi}x{2 * chi} complex SVD) / ms_per_step",
                 "peak_source": "FP32 FFMA rate measured in-process (loop kernel, best of 3): the mixed path runs "
                                "on the FP32 pipes; MEASURED_PEAKS.json holds only HBM and cuBLAS BF16",
-                "traffic_source": "DRAM bytes per gate step: ncu dram__bytes_read.sum + dram__bytes_write.sum per "
-                                  "launch (one Jacobi sweep, one GEMM) at k = 1024 scaled by (k / 1024)^2, times "
-                                  "the launches per step of jacobi_fp32, jacobi_df and zgemm_df",
+                "traffic_source": "computed, not measured: bytes that the step's sweeps (B and V read and written "
+                                  "once) and products (operands and results) move at least; most of it stays in L2",
                 "units": "launches and traffic per gate step; avg_launch_ms = ms per gate step",
                 "pipe_busy": {"kernel": dom, "executed_tflops": executed, "frac_of_ffma": executed / ffma if ffma else None,
                               "sweeps_per_step": st["launches"] / nprof,
                               "avg_sweep_ms": st["ms"] / max(1, st["launches"]),
-                              "traffic_per_sweep": (NCU_TRAFFIC_1024.get(dom, 0.0) * (2 * chi / 1024) ** 2) or None,
+                              "traffic_per_sweep": sweep_bytes(dom, 2 * chi),
                               "note": "FP32 instructions the kernel class executes (compensated inner products and "
                                       "rotations) per second, not algorithmic work"},
                 "time_share": shares}

@@ -52,9 +52,13 @@ typedef struct qr_mpo qr_mpo;     /* one open-boundary MPO resident in device me
 #define QR_EHOST 9        /* other host-side failure (a worker thread that could not start) */
 
 /* Precision of a chain's arithmetic (qr_chain_set_precision), a bit mask. */
-#define QR_FP64 0           /* plain: all ComplexF64 */
-#define QR_MIXED 1          /* SVDs of more than 32 columns take their FP32 Jacobi sweeps straight on the
-                               matrix (QR_FP64: on the R^H of a QR), may finish by
+#define QR_FP64 0           /* plain: results of FP64 accuracy from ComplexF64 data.  Large products run as exact
+                               8-bit slices on the tensor cores (error relative to sum |a||b|, as in FP64
+                               arithmetic), and SVDs start from FP32 sweeps that FP64-accurate steps finish
+                               to sqrt(m) eps sigma_max. */
+#define QR_MIXED 1          /* SVDs of more than 16 columns (unless at most 32 columns and 128 rows) take their
+                               FP32 Jacobi sweeps straight on the
+                               matrix (QR_FP64: above 32 columns on the R^H of a QR), may finish by
                                double-float sweeps (FP32 pairs, ~2^-48) where the refinement by products
                                leaves pairs over, and accept couplings of 4 sqrt(m) eps sigma_max instead
                                of sqrt(m) eps.  Products, singular values and vectors and the truncation

@@ -286,10 +286,10 @@ __device__ void team_orthonormalise(const Team& T, double2* W, int rows, int kee
 // One cluster per task (strided over the layer's tasks).  ws: slot_size(side) double2 per cluster.  dry = 1 runs
 // the arithmetic without writing the chain (the autotuner's timing runs).
 //
-// Above BT_PRE_MIN columns the SVD first runs FP32 sweeps on a copy of theta (64x the FP64 rate on
-// this part): two Newton-Schulz steps X <- X + X (I - X^H X) / 2 make their rotations unitary to rounding,
-// B = theta X is formed, and full-precision sweeps finish from couplings of ~1e-6 in two or three sweeps:
-// in FP64, or with MIXED in double-float on the FP32 pipes.
+// The SVD: FP64 sweeps up to BT_PRE_MIN columns, team_svd (FP32 sweeps refined by FP64 products) up to
+// BT_TEAM_MAX.  Above that FP32 sweeps on a copy of theta (64x the FP64 rate on this part), two Newton-Schulz
+// steps X <- X + X (I - X^H X) / 2 that make their rotations unitary to rounding, B = theta X, and full-precision
+// sweeps that finish from couplings of ~1e-6 in two or three: in FP64, or with MIXED in double-float on the FP32 pipes.
 //
 // What bounds a step is its chain of rounds: 127 of them in a sweep of 128 columns.  On one CTA a
 // double-float sweep of theta 128 x 128 needs 1.4 ms of its SM's FP32 rate and an FP64 sweep ~10, so a layer of

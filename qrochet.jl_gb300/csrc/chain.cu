@@ -579,10 +579,10 @@ bool build_mix_table(const double2* W, int wl, int d, int wr, MixTable* t) {
 // mix_k over the nonzeros only: Y[b,o,w',a'] = sum over the table's (w, i) of W X[w,b,i,a'].
 //
 // A block takes nb values of b at one a'; with STAGED it copies their X (contiguous for every i) to shared
-// memory first, from which the terms' strided reads are conflict-free for odd wl.  Bound by memory: the
-// coefficients of Pauli sums are mostly 1, -1, i and -i, which cost no multiplication, and real ones half of a
-// complex one.  (Reading global memory once per term, with complex multiply-adds throughout, was bound by both
-// FP64 and latency: 91 us for 704 x 704 pairs and 5 channels, 53 now.)  A sum that is not finite
+// memory first, from which the terms' strided reads are conflict-free for odd wl.  The coefficients of Pauli sums
+// are mostly 1, -1, i and -i, which cost no multiplication, and real ones half of a complex one.  Bound: the FP64
+// additions that are left (the pipe is 70% active; DRAM 24%).  Reading global memory once per term, with complex
+// multiply-adds throughout, took 91 us for 704 x 704 pairs and 5 channels; now 53.  A sum that is not finite
 // is formed again with all operations, as 0 * inf belongs to it.
 __device__ __forceinline__ double flip(double x) {  // -x without the FP64 pipe
   return __hiloint2double(__double2hiint(x) ^ 0x80000000, __double2loint(x));

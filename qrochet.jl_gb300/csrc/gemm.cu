@@ -1,8 +1,8 @@
 // Complex FP64 GEMM, C[b] = alpha op(A[b]) diag(dk) op(B[b]) + beta C[b]:
 //   op: N (as stored, column-major), T (transpose), C (conjugate transpose), R (conjugate).
 //
-// Two kernels.  Products from OZ_MIN_WORK multiply-adds on (alpha = 1, beta = 0: every call of the
-// library) run on the tensor cores as exact integer slices (gemm_oz.cu).  The rest run here, in FP64:
+// Two kernels.  Products from OZ_MIN_WORK multiply-adds on (alpha = 1, beta = 0: every large product of the
+// library) run on the tensor cores as integer slices (gemm_oz.cu).  The rest run here, in FP64:
 // an SM does 7 GFLOP/s in FP64 whatever instruction issues it (DMMA or DFMA), so a small product is fast
 // only when all SMs share it.  zgemm_spread_k gives a CTA 32 elements of C and a warp a slice of K.
 #include "kernels.cuh"
@@ -78,7 +78,7 @@ int zgemm_spread(cudaStream_t s, int opA, int opB, int M, int N, int K, double2 
   const bool an = opA == OP_N || opA == OP_R, bn = opB == OP_N || opB == OP_R;
   const Strided a = {A, an ? 1 : lda, an ? lda : 1, sA, opA == OP_C || opA == OP_R};
   const Strided b = {B, bn ? ldb : 1, bn ? 1 : ldb, sB, opB == OP_C || opB == OP_R};
-  const bool few = (long)M * N * batch < 32 * 76;  // fewer than half of the SMs with 32 elements a CTA
+  const bool few = (long)M * N * batch < 32 * 76;  // 32 elements a CTA would reach less than half of the 152 SMs
   const int slices = few ? 4 : 1, warps = K >= 32 * slices ? 8 : K >= 8 * slices ? 4 : 1;
   const dim3 grid(ceil_div((long)M * N, few ? 8 : 32), 1, batch);
   if (few) zgemm_spread_k<8><<<grid, 32 * warps, 0, s>>>(a, b, M, N, K, alpha, beta, C, ldc, sC, dk, 0);
@@ -93,7 +93,7 @@ int zherk_spread(cudaStream_t s, int n, int K, const double2* A, long lda, doubl
   if (K <= 0) return zscale_matrix(s, n, n, zero, C, ldc, 0, 1);
   const Strided a = {A, lda, 1, 0, 1}, b = {A, lda, 1, 0, 0};
   const long total = (long)n * (n + 1) / 2;
-  const bool few = total < 32 * 76;
+  const bool few = total < 32 * 76;  // as in zgemm_spread
   const int slices = few ? 4 : 1, warps = K >= 32 * slices ? 8 : K >= 8 * slices ? 4 : 1;
   const unsigned grid = ceil_div(total, few ? 8 : 32);
   if (few) zgemm_spread_k<8><<<grid, 32 * warps, 0, s>>>(a, b, n, n, K, one, zero, C, ldc, 0, nullptr, 1);

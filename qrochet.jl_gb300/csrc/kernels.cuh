@@ -12,10 +12,11 @@ enum { OP_N = 0, OP_T = 1, OP_C = 2, OP_R = 3 };
 int zgemm(cudaStream_t s, int opA, int opB, int M, int N, int K, double2 alpha,
           const double2* A, long lda, long sA, const double2* B, long ldb, long sB,
           double2 beta, double2* C, long ldc, long sC, int batch, const double* dk, bool normwise = false);
-// From this many complex multiply-adds on, the three launches of the sliced product cost less than the
-// spread kernel's FP64 time (4 DFMA each at 2 per SM and cycle): 96 x 128 x 96 takes 25 us sliced and 19
-// spread, 128 x 128 x 128 25 and 31, 256 x 512 x 256 34 and 372.  (The 64 x 64-tile DMMA kernel that ran all
-// sizes before took 592 us at 128^3, 1176 at 256 x 512 x 256 and 64.9 ms at 2048^3; sliced: 2.07 ms.)
+// From this many complex multiply-adds on, the three launches of the sliced product cost no more than the
+// spread kernel's FP64 time (4 DFMA each at 2 per SM and cycle).  Events around one product on an idle stream, us:
+// 96 x 128 x 96 37 sliced and 23 spread, 128 x 128 x 128 36 and 35, 256 x 512 x 256 49 and 378, 512^3 84 and 1474.
+// (The 64 x 64-tile DMMA kernel that ran all sizes before took 592 us at 128^3, 1176 at 256 x 512 x 256 and 64.9 ms
+// at 2048^3; sliced: 2.36 ms with the guard, 2.09 without.)
 constexpr double OZ_MIN_WORK = 1.5 * (1 << 20);
 // the same product in FP64 on the CUDA cores, spread over all SMs; allocates nothing
 int zgemm_spread(cudaStream_t s, int opA, int opB, int M, int N, int K, double2 alpha, const double2* A, long lda,
@@ -59,7 +60,8 @@ int zgemm_tc(cudaStream_t s, int opA, int opB, int M, int N, int K, const float2
 enum { DF_STORE = 0, DF_I_MINUS = 1, DF_F32_AXPY = 2, DF_GRAM = 3 };
 // DF_STORE: (Ch, Cl) = op(A) B; DF_I_MINUS: Ch = I - op(A) B (FP32); DF_F32_AXPY: (Ch, Cl) = D +
 // alpha op(A_hi) B_hi with FP32 products; DF_GRAM: Ch = I - A^H A from the tiles on or above the
-// diagonal (op C, B = A).  op(A) in {N, T, C}; B is not transformed.
+// diagonal (op C, B = A).  op(A) in {N, T, C}; B is not transformed.  The SVD's fallback sweeps use DF_GRAM and
+// DF_F32_AXPY with op N; the other forms are reached by the kernel tests only.
 int zgemm_df(cudaStream_t s, int mode, int opA, int M, int N, int K, const float2* Ah, const float2* Al, long lda,
              const float2* Bh, const float2* Bl, long ldb, float2* Ch, float2* Cl, long ldc,
              const float2* Dh = nullptr, const float2* Dl = nullptr, long ldd = 0, float alpha = 1.f);
@@ -133,12 +135,12 @@ long schedule_pairs_host(const unsigned* mask, const unsigned* flag, int nv, int
 // check which ordering and which kernel a size reached.
 enum SvdPath {
   SP_CLUSTER = 0,        // whole Jacobi in one thread-block cluster (k <= 128)
-  SP_BLOCK_CLUSTER,      // FP32 block Jacobi in one cluster
-  SP_BLOCK_BARRIER,      // FP32 block sweep, grid barrier between rounds
-  SP_BLOCK_DATAFLOW,     // FP32 block sweep, per-block flags (more block pairs than CTAs)
+  SP_BLOCK_CLUSTER,      // FP32 Gram-matrix sweeps in one cluster
+  SP_BLOCK_BARRIER,      // (no sweep counts this any more; it keeps its place in the order that the hook documents)
+  SP_BLOCK_DATAFLOW,     // FP32 Gram-matrix sweep, per-block flags
   SP_F64_BARRIER,        // FP64 scalar sweep, grid barrier
   SP_F64_DATAFLOW,       // FP64 scalar sweep, per-column flags
-  SP_F32_BARRIER,        // FP32 scalar sweep (rows > 2048), grid barrier
+  SP_F32_BARRIER,        // FP32 scalar sweep (rows > 4096), grid barrier
   SP_F32_DATAFLOW,       // FP32 scalar sweep, per-column flags
   SP_DF_CLUSTER,         // double-float polish in one cluster
   SP_DF_BARRIER,         // double-float polish sweep, grid barrier

@@ -7,7 +7,7 @@
 // like the R that Julia's qr returns.
 //
 // Three schedules of the same factorisation:
-//  - zqr_thin, up to 6400 rows: panels of 32 columns in one thread-block cluster each (house_panel_k), the
+//  - zqr_thin, up to 6144 rows: panels of 32 columns in one thread-block cluster each (house_panel_k), the
 //    trailing columns and Q by products (zqr_thin_blocked).
 //  - zqr_thin, more rows: the whole factorisation in one cooperative launch.  CTA b owns the columns
 //    c = b (mod grid).  At step j every CTA reads column j (final after step j - 1), forms the
@@ -326,7 +326,8 @@ __device__ __forceinline__ double inv_root(double s, double* root) {
 // than 16 (8) are left a warp takes 2 (4) rows at a time.  On exit R's rows are in A, the unit lower
 // trapezoid (zeros above the diagonal) in V (m x nb), and tau.
 // Bound: at 16 rows a CTA the latency of a step (~5 us: a 16-CTA exchange 1.1, sums 0.9, the reflector's serial
-// FP64 chain 2); at 100 rows and more the FP64 pipe (8 FMAs per element and step, 2 per cycle and SM).
+// FP64 chain 2); at 64 rows and more the FP64 pipe (8 FMAs per element and step, 2 per cycle and SM): a panel of
+// 1024 rows takes 247 us with that pipe 57% active.
 __global__ void __launch_bounds__(QB_NT) house_panel_k(double2* __restrict__ A, long lda, int m, int nb,
                                                        double2* __restrict__ V, long ldv, double2* __restrict__ tau, int L,
                                                        int cs) {

@@ -1552,7 +1552,6 @@ __global__ void gather_cols_k(const CS* __restrict__ src, long lds, int rows, in
 }
 
 
-// Q[:, j] *= phase(R_jj) (R_jj == 0 -> 1): keeps Q as close to the input columns as possible
 // row i of src to row perm[i] of dst
 __global__ void scatter_rows_k(const double2* __restrict__ src, int k, const int* __restrict__ perm, double2* __restrict__ dst,
                                long ldd) {
@@ -1560,6 +1559,7 @@ __global__ void scatter_rows_k(const double2* __restrict__ src, int k, const int
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x)
     dst[perm[t % k] + t / k * ldd] = src[t];
 }
+// Q[:, j] *= phase(R_jj) (R_jj == 0 -> 1): keeps Q as close to the input columns as possible
 __global__ void phase_fix_k(double2* Q, long ldq, int m, int k, const double2* R, long ldr) {
   long total = (long)m * k;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
@@ -1615,7 +1615,7 @@ int jacobi(cudaStream_t s, SvdWork* w, cplx_t<T>* B, long ldb, int rows, int k, 
   if (small) {
     // one cluster of up to 16 CTAs with one warp per pair of a round: as many CTAs as pairs (up
     // to 16), then 2-4 warps per CTA
-    // FP32 with at most 128 rows: the block form (one CTA per block pair of 4-column blocks)
+    // FP32 with at most 128 rows: the Gram-matrix form (one CTA per pair of 8-column blocks)
     const bool blk = sizeof(T) == 4 && rows <= JC_NT && k > 2 * JR_W;
     constexpr int bw = 8;
     const int nbk = (k + bw - 1) / bw;

@@ -8,8 +8,10 @@
 // squared from step to step (second-order terms of both corrections remain), so FP32 vectors
 // (t ~ 1e-2) take three corrections and a final test.  A Jacobi sweep over 2048 columns is 1023
 // dependent rounds, 72 ms in double-float; a step here is one and two half products of 2048^3, ~5 ms.
-// The largest tangents (near-degenerate clusters) go through a listed double-float Jacobi sweep instead.  (Ogita and Aishima, "Iterative refinement for symmetric eigenvalue
-// decomposition", 2018, give the first-order form of the correction.)
+// The largest tangents (near-degenerate clusters) go through a listed double-float Jacobi sweep instead, which is
+// never the last word: the next step forms B = A X again and corrects X, so results carry FP64 and not 48 bits.
+// (Ogita and Aishima, "Iterative refinement for symmetric eigenvalue decomposition", 2018, give the first-order form
+// of the correction.)
 
 // The pairs of the first step within this factor of its largest tangent, and at any step those at or
 // above kRefineListTan, are left out of T and rotated by a listed sweep: the second-order terms of the rest

@@ -281,7 +281,7 @@ __device__ void team_correct(const Team& T, double2* Xt, const float2* Xf, const
   }
 }
 
-// Squares of side^2 double2 that team_svd works in, and three columns (norms, sweep counters).
+// Squares of side^2 double2 that team_svd works in, and one column (norms, sweep counters).
 constexpr int TM_SQUARES = 7;
 constexpr size_t team_ws(int side) { return TM_SQUARES * (size_t)side * side + TM_MAXK; }
 
