@@ -2327,17 +2327,17 @@ static int reorthonormalize(cudaStream_t s, SvdWork* w, double2* L, long ldl, in
   return QR_OK;
 }
 
-// One Newton-Schulz step on nearly orthonormal columns, L <- L (3 I - L^H L) / 2 (m x k, ld ldl; columns of
-// singular values far below sigma_max are noise and must stay out of it).  The
-// columns B / sigma are orthogonal to ~eps sigma_max / sigma_j; the step brings that to rounding and moves
-// the represented matrix by eps sigma_max, for two products instead of a Householder QR.
-static int polish_columns(cudaStream_t s, SvdWork* w, double2* L, long ldl, int m, int k) {
+// One orthonormalisation step on nearly orthonormal columns of singular values sigma (device; m x k, ld ldl;
+// columns of singular values far below sigma_max are noise and must stay out of it).  The columns B / sigma are
+// orthogonal to ~eps sigma_max / sigma_j, the rounding of B's short columns; the short column of a pair gives up
+// most of the overlap, which moves the represented matrix by eps sigma_j and not, as equal shares would, by eps
+// sigma_max.  Two products instead of a Householder QR.
+static int polish_columns(cudaStream_t s, SvdWork* w, double2* L, long ldl, int m, int k, const double* sigma) {
   QR_TRY(w->rfG.ensure(sizeof(double2) * (2 * (size_t)k * k + (size_t)m * k), s));
   double2 *S = w->rfG.as<double2>(), *T = S + (size_t)k * k, *Y = T + (size_t)k * k;
   QR_TRY(zherk(s, k, m, L, ldl, S, k));
-  QR_CUDA(cudaMemsetAsync(T, 0, sizeof(double2) * (size_t)k * k, s));
-  refine_m_k<<<gs((long)k * k), TPB, 0, s>>>(T, nullptr, S, k);  // (I - S) / 2
-  QR_CHECK_LAUNCH("refine_m_k");
+  orthonormal_m_k<<<gs((long)k * k), TPB, 0, s>>>(T, S, sigma, k);
+  QR_CHECK_LAUNCH("orthonormal_m_k");
   QR_TRY(zgemm(s, OP_N, OP_N, m, k, k, make_double2(1.0, 0.0), L, ldl, 0, T, k, 0, make_double2(0.0, 0.0), Y, m, 0, 1, nullptr,
                true));
   add_cols_k<<<gs((long)m * k), TPB, 0, s>>>(L, ldl, Y, m, k);
@@ -2501,8 +2501,7 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
 
   const bool team = rows0 <= TM_MAXK && k > 1 && k <= kTeamCols;
   if (team) {
-    QR_TRY(svd_team(s, w, B, rows, k, V));
-    refined = mode != QR_FP64 && k > kMixedMinCols;
+    QR_TRY(svd_team(s, w, B, rows, k, V));  // (its columns are tidied up already)
   } else if (mode == QR_FP64 || k <= kMixedMinCols) {
     if (k > kPrecondMinCols) {
       svd_path(SP_QR_PRECOND_FP64);
@@ -2634,7 +2633,7 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
     gather_cols_k<double2><<<gs((long)k * k), TPB, 0, s>>>(B, k, k, k, perm, sorted, L, k);
     QR_CHECK_LAUNCH("gather_cols_k");
     if (reorth) QR_TRY(reorthonormalize(s, w, L, k, k, kk));
-    else QR_TRY(polish_columns(s, w, L, k, k, kk));
+    else QR_TRY(polish_columns(s, w, L, k, k, kk, sorted));
     gather_cols_k<double2><<<gs((long)k * k), TPB, 0, s>>>(V, k, k, k, perm, nullptr, Rf, k);
     QR_CHECK_LAUNCH("gather_cols_k");
     const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
@@ -2657,7 +2656,7 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
     gather_cols_k<double2><<<gs((long)rows * k), TPB, 0, s>>>(B, rows, rows, k, perm, sorted, U, ldu);
     QR_CHECK_LAUNCH("gather_cols_k");
     if (reorth) QR_TRY(reorthonormalize(s, w, U, ldu, m, kk));
-    else if (refined) QR_TRY(polish_columns(s, w, U, ldu, m, kk));
+    else if (refined) QR_TRY(polish_columns(s, w, U, ldu, m, kk, sorted));
     gather_cols_k<double2><<<gs((long)k * k), TPB, 0, s>>>(V, k, k, k, perm, nullptr, Rf, k);
     QR_CHECK_LAUNCH("gather_cols_k");
     QR_TRY(ztranspose(s, Rf, k, k, k, Vh, ldvh, 1));  // Vh = Rf^H (k x n)
@@ -2668,7 +2667,7 @@ int zsvd_thin(cudaStream_t s, SvdWork* w, int mode, const double2* A, int m, int
     gather_cols_k<double2><<<gs((long)rows * k), TPB, 0, s>>>(B, rows, rows, k, perm, sorted, L, rows);
     QR_CHECK_LAUNCH("gather_cols_k");
     if (reorth) QR_TRY(reorthonormalize(s, w, L, rows, rows, kk));
-    else if (refined) QR_TRY(polish_columns(s, w, L, rows, rows, kk));
+    else if (refined) QR_TRY(polish_columns(s, w, L, rows, rows, kk, sorted));
     gather_cols_k<double2><<<gs((long)k * k), TPB, 0, s>>>(V, k, k, k, perm, nullptr, U, ldu);
     QR_CHECK_LAUNCH("gather_cols_k");
     QR_TRY(ztranspose(s, L, rows, rows, k, Vh, ldvh, 1));

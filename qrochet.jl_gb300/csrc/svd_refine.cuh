@@ -25,14 +25,19 @@ constexpr float kRefineCrowd = 4.f;
 // are below this part of the tolerance needs no further test.
 constexpr float kRefineLast = 0.03f;
 constexpr int kRefineMaxSteps = 12;
+// Couplings that meet the tolerance are turned along with the others, down to a sixteenth of it, where that takes a
+// tangent of at most this.  Left alone they add up: |U S V^H - A| of 512 x 512 in FP64 is 18 - 23 eps sigma_max over
+// flat, linear and twofold to fourfold degenerate spectra instead of 106 - 227.  Their second-order terms are this part of
+// couplings below the tolerance, so no test waits for them; larger tangents would show the products' 2^-23.
+constexpr float kRefineTidyTan = 1e-7f;
 
 // Column q of T per block: the rotation test of the pairs (p, q) and T_pq (diagonal 0).  out[0] += pairs
-// (p < q) that fail the test, out[1] = largest tangent, out[2] = largest |R|, out[3] = largest sum of
-// tangents in a column, a bound of |T|_2 (float bits).
+// (p < q) that fail the test, out[1] = their largest tangent, out[2] = largest |R|, out[3] = largest sum of
+// their tangents in a column, out[5] = of all tangents in a column, a bound of |T|_2 (float bits).
 __global__ void __launch_bounds__(256) refine_pairs_k(const double2* __restrict__ G, const double2* __restrict__ S, int k,
                                                       int k0, double tol, const double* __restrict__ smax_p,
                                                       double2* __restrict__ T, unsigned* __restrict__ out) {
-  __shared__ float red[8][3];
+  __shared__ float red[8][4];
   __shared__ unsigned redc[8];
   const double smax = smax_p[0] / smax_p[1];
   const float fl = (float)(4.0 * Eps<double>::v * smax);
@@ -40,7 +45,7 @@ __global__ void __launch_bounds__(256) refine_pairs_k(const double2* __restrict_
   const int q = blockIdx.x;
   const double lq = G[(long)q * (k + 1)].x;
   unsigned cnt = 0;
-  float tmax = 0.f, rmax = 0.f, sum = 0.f;
+  float tmax = 0.f, rmax = 0.f, sum = 0.f, all = 0.f;
   for (int p = threadIdx.x; p < k; p += 256) {
     const long e = p + (long)q * k;
     const double2 s = S[e];
@@ -58,16 +63,23 @@ __global__ void __launch_bounds__(256) refine_pairs_k(const double2* __restrict_
         // scaled magnitude: squares of tiny couplings would underflow
         const float inv = big > 0.f ? 1.f / big : 0.f;
         const float ux = gx * inv, uy = gy * inv, un = sqrtf(ux * ux + uy * uy), g = big * un;
-        if (lp > 0.0 && lq > 0.0 && g > tols * sqrtf((float)fmin(lp, lq)) + fl * fl) {
+        const float lim = tols * sqrtf((float)fmin(lp, lq)) + fl * fl;
+        if (lp > 0.0 && lq > 0.0 && g > 0.0625f * lim) {
           const float d = (float)(lq - lp);
           const float az = fabsf(d) / (2.f * g);
           const float tt = az > 1e18f ? 0.5f / az : 1.f / (az + sqrtf(1.f + az * az));
           // equal norms: the sign of a zero difference must differ between T_pq and T_qp
           const float sg = ((d < 0.f || (d == 0.f && p > q)) ? -tt : tt) / un;
-          t = make_double2((double)(sg * ux), (double)(sg * uy));
-          if (p < q) cnt++;
-          tmax = fmaxf(tmax, tt);
-          sum += tt;
+          const bool fails = g > lim;
+          if (fails || tt <= kRefineTidyTan) {
+            t = make_double2((double)(sg * ux), (double)(sg * uy));
+            all += tt;
+          }
+          if (fails) {
+            if (p < q) cnt++;
+            tmax = fmaxf(tmax, tt);
+            sum += tt;
+          }
         }
       }
     }
@@ -77,6 +89,7 @@ __global__ void __launch_bounds__(256) refine_pairs_k(const double2* __restrict_
     tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
     rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
     sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    all += __shfl_xor_sync(0xffffffffu, all, o);
   }
   cnt = __reduce_add_sync(0xffffffffu, cnt);
   const int w = threadIdx.x >> 5;
@@ -84,6 +97,7 @@ __global__ void __launch_bounds__(256) refine_pairs_k(const double2* __restrict_
     red[w][0] = tmax;
     red[w][1] = rmax;
     red[w][2] = sum;
+    red[w][3] = all;
     redc[w] = cnt;
   }
   __syncthreads();
@@ -92,12 +106,14 @@ __global__ void __launch_bounds__(256) refine_pairs_k(const double2* __restrict_
       tmax = fmaxf(tmax, red[i][0]);
       rmax = fmaxf(rmax, red[i][1]);
       sum += red[i][2];
+      all += red[i][3];
       cnt += redc[i];
     }
     if (cnt) atomicAdd(out, cnt);
     atomicMax(out + 1, __float_as_uint(tmax));
     atomicMax(out + 2, __float_as_uint(rmax));
     atomicMax(out + 3, __float_as_uint(sum));
+    atomicMax(out + 5, __float_as_uint(all));
   }
 }
 
@@ -132,6 +148,19 @@ __global__ void refine_m_k(double2* __restrict__ T, const double2* __restrict__ 
     m.x += 0.5 * ((e % k == e / k ? 1.0 : 0.0) - s.x);
     m.y -= 0.5 * s.y;
     T[e] = m;
+  }
+}
+// T <- the first-order correction that makes unit columns with Gram matrix S orthonormal: a pair's overlap is taken
+// from its columns in the shares sigma_p^2 and sigma_q^2 that move U diag(sigma) least
+__global__ void orthonormal_m_k(double2* __restrict__ T, const double2* __restrict__ S, const double* __restrict__ sigma,
+                                int k) {
+  const long tot = (long)k * k;
+  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < tot; e += (long)gridDim.x * blockDim.x) {
+    const long p = e % k, q = e / k;
+    const double2 s = S[e];
+    const float r = sigma[p] > 0.0 ? (float)(sigma[q] / sigma[p]) : 1e18f;
+    const float w = -1.f / (1.f + r * r);  // column p's share in column q
+    T[e] = p == q ? make_double2(0.5 * (1.0 - s.x), 0.0) : make_double2(w * s.x, w * s.y);
   }
 }
 // L (m x k, ld ldl) += Y (ld m)
@@ -261,6 +290,7 @@ int refine(cudaStream_t s, SvdWork* w, const double2* A, int rows, int k, double
     QR_TRY(zherk(s, k, rows, B, rows, G, k));
     QR_TRY(zherk(s, k, k, X, k, S, k));
     QR_CUDA(cudaMemsetAsync(out, 0, 16, s));
+    QR_CUDA(cudaMemsetAsync(out + 5, 0, 4, s));
     refine_pairs_k<<<k, 256, 0, s>>>(G, S, k, k0, tol, smax_d, T, out);
     QR_CHECK_LAUNCH("refine_pairs_k");
     hs = static_cast<unsigned*>(host_scratch(sizeof(unsigned) * 8));
@@ -269,10 +299,11 @@ int refine(cudaStream_t s, SvdWork* w, const double2* A, int rows, int k, double
     QR_CUDA(cudaStreamSynchronize(s));
     if (hs[4]) return fail(QR_ECUDA, "tcgen05 product: a bounded wait gave up");
     const unsigned fail_pairs = hs[0];
-    float tmax, rmax, tsum;
+    float tmax, rmax, tsum, tall;
     memcpy(&tmax, &hs[1], sizeof(float));
     memcpy(&rmax, &hs[2], sizeof(float));
     memcpy(&tsum, &hs[3], sizeof(float));
+    memcpy(&tall, &hs[5], sizeof(float));
     if (debug_on())
       fprintf(stderr, "[qr] refine %dx%d step %d: %u pairs, largest tangent %.2e, column sum %.2e; |I - X^H X| %.2e\n", rows,
               k, step, fail_pairs, tmax, tsum, rmax);
@@ -309,7 +340,7 @@ int refine(cudaStream_t s, SvdWork* w, const double2* A, int rows, int k, double
       }
       last = tmax;
     }
-    const bool second = rotate && tsum > 1e-8f;
+    const bool second = rotate && tall > 1e-8f;
     if (rotate) svd_path(SP_DF_LINEAR);
     else QR_CUDA(cudaMemsetAsync(T, 0, sizeof(double2) * kk, s));
     if (second) QR_TRY(product(T, T, G));

@@ -211,11 +211,14 @@ __device__ void team_grams(const Team& T, double2* Bt, int rows, double2* Xt, in
 
 constexpr float TM_BIGTAN = 0.03f;   // tangents above this are not rotated at once
 constexpr float TM_LASTTAN = 1e-8f;  // a correction this small leaves nothing above rounding
+// Couplings that meet the tolerance are turned too, down to a sixteenth of it, where that takes a rotation this
+// small: a step forms them anyway, and left alone they add up in the factors.
+constexpr float TM_TIDYTAN = 1e-9f;
 constexpr int TM_STEPS = 10;
 
 // The correction E of X <- X + X E, Et[i + k j] = E[j, i]: -S / 2, and for a pair that fails the rotation test
-// of rotation_params its tangent times the phase of its coupling, as orthonormal columns would have it.
-// count[1] <- largest |E|, count[0] += tangents above TM_BIGTAN (left out).
+// of rotation_params (or may be tidied up) its tangent times the phase of its coupling, as orthonormal columns would
+// have it.  count[1] <- largest |E| of the former, count[0] += tangents above TM_BIGTAN (left out).
 __device__ inline void team_correction(const Team& T, const float4* gs, const double* dg, int k, double tol, double smax,
                                        bool rotate, float2* Et, unsigned* count) {
   const double fl = 4.0 * Eps<double>::v * smax, t2 = tol * tol * smax * smax, fl4 = fl * fl * fl * fl;
@@ -234,17 +237,19 @@ __device__ inline void team_correction(const Team& T, const float4* gs, const do
     const double a = dg[i], b = dg[j], h = 0.5 * (a + b);
     const double gx = v.x - h * v.z, gy = v.y - h * v.w, g2 = gx * gx + gy * gy;
     float sx = 0.f, sy = 0.f;
-    if (rotate && a > 0.0 && b > 0.0 && g2 > t2 * fmin(a, b) + fl4) {
+    const double lim = t2 * fmin(a, b) + fl4;
+    if (rotate && a > 0.0 && b > 0.0 && g2 > lim * (1.0 / 256.0)) {
       // (the coupling may lie below FP32's range)
       const float big_g = (float)fmax(fabs(gx), fabs(gy));
       const float inv = 1.f / big_g, ux = (float)gx * inv, uy = (float)gy * inv, ru = rsqrtf(ux * ux + uy * uy);
       const float z = (float)(0.5 * (b - a)) * inv * ru, tt = (z >= 0.f ? 1.f : -1.f) / (fabsf(z) + sqrtf(1.f + z * z));
-      if (fabsf(tt) > TM_BIGTAN) {
+      const bool fails = g2 > lim;
+      if (fails && fabsf(tt) > TM_BIGTAN) {
         big++;
-      } else {
+      } else if (fails || fabsf(tt) <= TM_TIDYTAN) {
         sx = tt * ux * ru;
         sy = tt * uy * ru;
-        emax = fmaxf(emax, fabsf(tt));
+        if (fails) emax = fmaxf(emax, fabsf(tt));
       }
     }
     Et[j + k * i] = make_float2(rx + sx, ry + sy);   // E[i, j] = s
@@ -278,6 +283,46 @@ __device__ void team_correct(const Team& T, double2* Xt, const float2* Xf, const
       im += __shfl_xor_sync(0xffffffffu, im, o);
     }
     if (t < total && part == 0) Yt[e] = make_double2(Xt[e].x + re, Xt[e].y + im);
+  }
+}
+
+// B (rows x k, ld rows) = the columns of Bt (by rows) made orthogonal: b_q -= b_p g / (d_p + d_q) and b_p -= b_q
+// conj(g) / (d_p + d_q) with g = b_p^H b_q, d the squared norms (dg), the least change of B that does it.  B = A X
+// rounds every column at eps smax, which is eps smax / sigma of a short one: a product's columns over 3 decades are
+// 100 to 1000 eps from orthogonal, after this 10.
+__device__ void team_tidy(const Team& T, double2* Bt, int rows, int k, const double* dg, double2* G, double2* B) {
+  const int sums = k * (k - 1) / 2, parts = team_parts(T, sums), total = sums * parts;
+  for (int t0 = T.tid - T.lane; t0 < total; t0 += T.nt) {
+    const int t = t0 + T.lane, part = t % parts, e = t / parts;
+    int q = (int)((sqrtf(8.f * e + 1.f) + 1.f) * 0.5f);  // e = q (q - 1) / 2 + p, p < q
+    while (q * (q - 1) / 2 > e) q--;
+    while ((q + 1) * q / 2 <= e) q++;
+    const int p = e - q * (q - 1) / 2;
+    double2 s = make_double2(0.0, 0.0);
+    if (t < total) {
+#pragma unroll 2
+      for (int r = part; r < rows; r += parts) macc(s, Bt[p + k * r], Bt[q + k * r]);
+    }
+    s = parts_sum(s, parts);
+    if (t < total && part == 0) {
+      const float d = (float)dg[p] + (float)dg[q], inv = d > 1e-30f ? 1.f / d : 0.f;
+      const double2 c = make_double2(s.x * inv, s.y * inv);
+      G[p + k * q] = c;
+      G[q + k * p] = cconj(c);
+    }
+  }
+  T.sync();
+  const int nb = rows * k, pb = team_parts(T, nb), tb = nb * pb;
+  for (int t0 = T.tid - T.lane; t0 < tb; t0 += T.nt) {
+    const int t = t0 + T.lane, part = t % pb, e = t / pb, j = e % k, r = e / k;
+    double2 s = make_double2(0.0, 0.0);
+    if (t < tb) {
+#pragma unroll 2
+      for (int i = part; i < k; i += pb)
+        if (i != j) mac(s, Bt[i + k * r], G[i + k * j]);
+    }
+    s = parts_sum(s, pb);
+    if (t < tb && part == 0) B[r + rows * j] = csub(Bt[j + k * r], s);
   }
 }
 
@@ -360,8 +405,9 @@ __device__ bool team_svd(const Team& T, double2* A, double2* B, double2* V, int 
   if (done) {
     team_product(T, Am, rows, X, k, Bt);
     T.sync();
-    for (int t = T.tid; t < rows * k; t += T.nt) B[t] = Bt[t % rows * k + t / rows];
     for (int t = T.tid; t < k * k; t += T.nt) V[t] = X[t % k * k + t / k];
+    if (rotate) team_tidy(T, Bt, rows, k, dg, reinterpret_cast<double2*>(S5), B);
+    else for (int t = T.tid; t < rows * k; t += T.nt) B[t] = Bt[t % rows * k + t / rows];
   } else {
     for (int t = T.tid; t < rows * k; t += T.nt) B[t] = A[t];
     for (int t = T.tid; t < k * k; t += T.nt) V[t] = make_double2(t % k == t / k ? 1.0 : 0.0, 0.0);
